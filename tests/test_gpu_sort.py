@@ -147,3 +147,29 @@ def test_gather_rejects_out_of_range_records(ctx):
     tile.meta["rec"][5] = len(bam) - 10  # span past the chunk end
     with pytest.raises(MojoAlignError, match="outside their chunks"):
         gather_sorted(ctx, [bam], tile, res)
+
+
+@pytest.mark.parametrize("n", [1, 5, 33, 1000, 40_000, 200_000, 700_001])
+def test_gather_copies_records_of_every_size_and_phase(ctx, n):
+    """Record sizes around the copy's words and rounds (0 .. 24, 255 .. 273,
+    512 .. 520 and a few kilobytes) at random byte offsets of two chunks, for
+    tiles that give a warp 4, 8, 16 and 32 records."""
+    rng = np.random.default_rng(n)
+    sizes = np.concatenate([np.arange(25), np.arange(255, 274), np.arange(512, 521), [3000, 4097]])
+    length = rng.choice(sizes[:44] if n > 100_000 else sizes, n).astype(np.uint32)
+    chunks = [rng.integers(0, 256, 1 << 20, dtype=np.uint8) for _ in range(2)]
+    off = rng.integers(0, (1 << 20) - 4097, n).astype(np.uint64)
+    off[0] = (1 << 20) - int(length[0])  # up to the chunk's last byte
+    rec = (rng.integers(0, 2, n).astype(np.uint64) << np.uint64(32)) | off
+    perm = rng.permutation(n).astype(np.uint32)
+    dup = rng.integers(0, 2, n).astype(np.uint32)
+    tile = BamTile(meta_cap=n, n_reads=n)
+    tile.meta["rec"][:], tile.meta["len"][:] = rec, length
+    want = []
+    for o in perm:
+        r = chunks[int(rec[o]) >> 32][int(off[o]):int(off[o]) + int(length[o])].copy()
+        if dup[o] and r.size > 19:
+            r[19] |= 4
+        want.append(r)
+    got = gather_sorted(ctx, chunks, tile, SortResult(dup, perm, None, 0))
+    np.testing.assert_array_equal(got, np.concatenate(want))
