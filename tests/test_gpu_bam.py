@@ -145,3 +145,34 @@ def test_errors_leave_the_tile_unchanged(ctx):
                             10 ** 6)
     empty = emit_bam_from_batch(ctx, hits, 0, True, arena, RID_TO_TID, RG, BamTile(meta_cap=0), 0)
     assert empty.size == 0
+
+
+@pytest.mark.parametrize("paired", [False, True])
+@pytest.mark.parametrize("rg", [b"g", b"r" * 119, b"r" * 120, b"r" * 200])
+def test_read_lengths_at_the_edges_of_the_lanes_and_the_stage(ctx, rg, paired):
+    """Bases and qualities around one lane's eight and a warp's 256, records
+    around the warp's 3072-byte output stage, names around 32 bytes, bases and
+    qualities of any byte value, both strands."""
+    from mojoalign_b200.bam import BatchArena
+
+    rng = np.random.default_rng(len(rg))
+    lens = [0, 1, 2, 7, 8, 9, 15, 16, 17, 31, 32, 33, 149, 150, 151, 255, 256, 257, 263, 264, 265] * 3
+    lens += list(range(1930, 2030, 7)) + [511, 512, 513] + [100] * 41
+    n1 = len(lens)
+    n_seq = n1 * (2 if paired else 1)
+
+    def record(n):
+        seq = rng.choice(np.frombuffer(b"ACGTacgtNn\xc1\x81", np.uint8), n, p=[.2, .2, .2, .2] + [.025] * 8)
+        qual = rng.integers(0, 256, n).astype(np.uint8) if rng.random() < 0.3 else rng.integers(33, 74, n).astype(np.uint8)
+        return bytes(rng.integers(65, 90, int(rng.integers(0, 70))).astype(np.uint8)), seq.tobytes(), qual.tobytes()
+
+    arena = BatchArena.from_records([record(int(n)) for n in rng.permutation(lens)] +
+                                    ([record(int(n)) for n in rng.permutation(lens)] if paired else []))
+    rid = rng.integers(-1, len(RID_TO_TID), n_seq).astype(np.int32)
+    u32 = lambda hi: rng.integers(0, hi, n_seq).astype(np.uint32)  # noqa: E731
+    hits = {"rid": rid, "pos": u32(1 << 20), "mapq": u32(61), "flag": np.where(rid < 0, 4, 16 * (u32(2) == 1)).astype(np.int32),
+            "sl": u32(3) * u32(20), "sr": u32(3) * u32(20), "nm": u32(300)}
+    cap = bam_cap_for(arena, len(rg))
+    want, _, _ = oracle.emit_bam(hits, vars(arena), n1, paired, RID_TO_TID, rg, meta_cap=n_seq, cap=cap)
+    got = emit_bam_from_batch(ctx, hits, n1, paired, arena, RID_TO_TID, rg, BamTile(meta_cap=n_seq), cap)
+    assert got.tobytes() == want
