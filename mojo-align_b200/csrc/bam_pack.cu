@@ -25,9 +25,15 @@
 
 #include "bam_pack.h"
 #include "ma_internal.h"
+#include "span.cuh"
 
 namespace ma {
 namespace {
+
+using span::put_bytes;
+using span::Span8;
+using span::span8_bytes;
+using span::span8_load;
 
 constexpr int LAYOUT_THREADS = 256;
 constexpr int REC_WARPS = 4;
@@ -291,34 +297,6 @@ __device__ __forceinline__ void plan_record(RecPlan& q, const BamDev& b, const B
     q.nm = static_cast<uint32_t>(clamp255(r.nm));
 }
 
-// Bytes 8i .. 8i+7 of a span of n bytes, in order or (rev) of the span read
-// backwards: the aligned words that cover them, loaded where they hold a byte
-// of the span, and then the bytes as two words (what lies outside the span is
-// undefined).
-struct Span8 {
-    uint32_t w0, w1, w2;
-};
-
-__device__ __forceinline__ Span8 span8_load(const uint8_t* src, uint32_t n, uint32_t i, bool rev) {
-    const uintptr_t a = reinterpret_cast<uintptr_t>(src);
-    const uint32_t* w = reinterpret_cast<const uint32_t*>(a & ~uintptr_t(3));
-    const uint32_t lead = static_cast<uint32_t>(a & 3), nw = (lead + n + 3) >> 2;
-    const uint32_t k = rev ? ((lead + n) >> 2) - 2 - 2 * i : 2 * i;  // first word; wraps below the span's start
-    w += static_cast<int32_t>(k);
-    Span8 s;
-    s.w0 = k < nw ? __ldg(w) : 0;
-    s.w1 = k + 1 < nw ? __ldg(w + 1) : 0;
-    s.w2 = k + 2 < nw ? __ldg(w + 2) : 0;
-    return s;
-}
-
-__device__ __forceinline__ uint2 span8_bytes(const Span8& s, const uint8_t* src, uint32_t n, bool rev) {
-    const uint32_t lead = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(src));
-    const uint32_t sh = ((rev ? lead + n : lead) & 3) * 8;
-    const uint32_t lo = __funnelshift_r(s.w0, s.w1, sh), hi = __funnelshift_r(s.w1, s.w2, sh);
-    return rev ? make_uint2(__byte_perm(hi, 0, 0x0123), __byte_perm(lo, 0, 0x0123)) : make_uint2(lo, hi);
-}
-
 // _nt16 (L455-464) of four bases at once: A/C/G/T in either case -> 1/2/4/8,
 // anything else 15; comp: _nt16_comp (L467-476) of that, A<->T, C<->G.
 // Bits 1-2 of a letter tell A, C, T and G apart; the letter they stand for
@@ -351,13 +329,6 @@ __device__ __forceinline__ uint8_t tag_byte(const BamDev& b, uint32_t i) {
     return i == 0 ? 0 : (i == 1 ? 78 : (i == 2 ? 77 : 67));
 }
 
-__device__ __forceinline__ void put_bytes(uint8_t* p, uint32_t v, uint32_t n) {
-    p[0] = static_cast<uint8_t>(v);
-    if (n > 1) p[1] = static_cast<uint8_t>(v >> 8);
-    if (n > 2) p[2] = static_cast<uint8_t>(v >> 16);
-    if (n > 3) p[3] = static_cast<uint8_t>(v >> 24);
-}
-
 // A lane's share of a record's source bytes: two name bytes, eight bases,
 // eight qualities; for records of up to 63 name bytes and 256 bases that is
 // all of them.
@@ -365,7 +336,7 @@ struct RecRaw {
     uint32_t n0, n1;
     Span8 seq, qual;
 };
-constexpr uint32_t RAW_NAME = 64, RAW_BASES = 256;  // l_qname and bases one RecRaw per lane covers
+constexpr uint32_t RAW_NAME = 64;  // l_qname that one RecRaw per lane covers
 
 __device__ __forceinline__ void load_raw(RecRaw& x, const RecPlan& q, uint32_t lane) {
     const uint8_t* name = q.name;
@@ -419,23 +390,6 @@ __device__ __forceinline__ void write_record(uint8_t* dst, const BamDev& b, cons
     if (n_tags > 32)
         for (uint32_t i = 32 + lane; i < n_tags; i += 32)
             dst[o_tag + i] = i + 1 == n_tags ? static_cast<uint8_t>(q.nm) : tag_byte(b, i);
-}
-
-// Stores stage[from, to) (stage[0] stands for the 16-byte aligned address
-// g): 16-byte stores, byte stores where a block is not whole.
-__device__ __forceinline__ void store_stage(uint8_t* g, const uint8_t* stage, uint32_t from, uint32_t to,
-                                            uint32_t lane) {
-    const uint32_t a = (from + 15) & ~15u, e = to & ~15u;
-    for (uint32_t i = a + 16 * lane; i < e; i += 512)
-        *reinterpret_cast<uint4*>(g + i) = *reinterpret_cast<const uint4*>(stage + i);
-    if (a > from) {  // the first block is not whole
-        const uint32_t i = from + lane;
-        if (i < min(a, to)) g[i] = stage[i];
-    }
-    if (to > e && e >= a) {  // the last one
-        const uint32_t i = e + lane;
-        if (i < to) g[i] = stage[i];
-    }
 }
 
 // A warp takes `per` consecutive records (whole pairs).  One lane per record
@@ -495,48 +449,14 @@ __global__ void __launch_bounds__(REC_WARPS * 32) bam_records_kernel(BamDev b, c
         if (mine) plan_record(plan[lane], b, r);
         __syncwarp();
         const uint32_t count = static_cast<uint32_t>(n_rec - base < per ? n_rec - base : per);
-        uint8_t* g = b.bam + __shfl_sync(FULL, start, 0);
-        uint32_t from = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(g) & 15);  // first byte of the stage that is ours
-        uint32_t fill = from;
-        g -= from;
         RecRaw next;
         load_raw(next, plan[0], lane);
-        for (uint32_t k = 0; k < count; ++k) {
-            const uint32_t n = __shfl_sync(FULL, bytes, k);
-            const RecRaw x = next;  // the next record's bytes are on their way while this one is written
-            if (k + 1 < count) load_raw(next, plan[k + 1], lane);
-            if (fill + n > REC_STAGE) {
-                if (fill > from) {
-                    // the whole blocks; the rest (from a block's start on, unless
-                    // the stage holds less than a block) moves to the front
-                    __syncwarp();
-                    const uint32_t e = fill & ~15u;
-                    if (e > from) {
-                        store_stage(g, stage, from, e, lane);
-                        const uint8_t v = lane < fill - e ? stage[e + lane] : 0;
-                        __syncwarp();
-                        if (lane < fill - e) stage[lane] = v;
-                        __syncwarp();
-                        g += e;
-                        fill -= e;
-                        from = 0;
-                    }
-                }
-                if (fill + n > REC_STAGE) {  // longer than the stage: in place
-                    store_stage(g, stage, from, fill, lane);
-                    write_record(g + fill, b, plan[k], x, tag, n_tags, lane);
-                    __syncwarp();
-                    g += (fill + n) & ~15u;
-                    from = fill = (fill + n) & 15u;
-                    continue;
-                }
-            }
-            write_record(stage + fill, b, plan[k], x, tag, n_tags, lane);
-            fill += n;
-        }
-        __syncwarp();
-        if (fill > from) store_stage(g, stage, from, fill, lane);
-        __syncwarp();
+        span::staged_run<REC_STAGE>(b.bam + __shfl_sync(FULL, start, 0), stage, bytes, count, lane,
+                                    [&](uint8_t* dst, uint32_t k) {
+                                        const RecRaw x = next;  // the next record's bytes are on their way
+                                        if (k + 1 < count) load_raw(next, plan[k + 1], lane);
+                                        write_record(dst, b, plan[k], x, tag, n_tags, lane);
+                                    });
     }
 }
 

@@ -7,32 +7,33 @@
 // hit_to_sam_line (L297-320) + the RG tag (_sam_with_rg_fm, L80-81) and
 // writes it.  Here the lines of a whole batch are built in HBM in three
 // passes:
-//   1. sam_layout_kernel (one thread per pair): both hits and the pair
-//      fields, each line's byte length and a compact record of its fields,
+//   1. sam_layout_kernel (one thread per line): its hit and the pair
+//      fields, the line's byte length and a compact record of its fields,
 //      names' bytes >= 0x80 counted (each becomes U+FFFD), SEQ / QUAL
 //      checked for strict UTF-8, mapped records and error bits;
 //   2. a device scan of the lengths (line end offsets);
-//   3. sam_write_kernel (one warp per line): the line assembled in a
-//      shared-memory stage at its destination's 16-byte phase (lanes copy the name, the
-//      contig names, SEQ reverse-complemented on flag 16, QUAL and the RG
-//      tag from aligned word loads; lane 0 writes the integer fields), then
-//      stored with 16-byte stores; lines longer than the stage are built in
-//      place.
+//   3. sam_write_kernel (a warp per run of lines): one lane formats a line's
+//      fields FLAG .. TLEN, then the warp assembles the lines in a
+//      shared-memory stage at the destination's 16-byte phase (name, the
+//      formatted fields, SEQ reverse-complemented on flag 16, QUAL and the RG
+//      tag from aligned word loads) and stores it in 16-byte blocks; lines
+//      longer than the stage are built in place.
 #include <cub/device/device_scan.cuh>
 
 #include <string>
 
 #include "ma_internal.h"
 #include "sam_emit.h"
+#include "span.cuh"
 
 namespace ma {
 namespace {
 
 constexpr int THREADS = 256;
-constexpr int WARPS = THREADS / 32;
 constexpr unsigned FULL = 0xffffffffu;
-constexpr uint32_t STAGE = 2048;  // bytes of a warp's line stage in shared memory
-constexpr int SPAN_UNROLL = 2;    // words a lane loads per round of a span copy
+constexpr int WRITE_WARPS = 4;
+constexpr uint32_t STAGE = 2048;  // bytes of output a warp gathers before it stores them
+constexpr uint32_t SLOT = 100;    // formatted fields of a line; an odd number of words, so lanes' slots spread over the banks
 
 enum : unsigned { E_OVER = 1, E_UTF8 = 2, E_RID = 4, E_SPAN = 8 };
 enum : uint8_t { K_NAME = 0, K_STAR = 1, K_EQ = 2 };
@@ -99,36 +100,32 @@ __device__ Hit hit_of(const SamDev& d, uint64_t r, unsigned& err) {
     return h;
 }
 
-// pair_hits (linear_extend.mojo:263-294); len2 = len(SEQ of R2).
-__device__ void pair_up(Hit& a, Hit& b, uint32_t len2) {
-    a.flag |= 1 | 64;
-    b.flag |= 1 | 128;
-    if (!a.star && !b.star && a.canon == b.canon) {
-        a.flag |= 2;
-        b.flag |= 2;
-        a.rnext_kind = b.rnext_kind = K_EQ;
-        a.pnext = b.pos1;
-        b.pnext = a.pos1;
-        int64_t t = b.pos1 - a.pos1;
+// pair_hits (linear_extend.mojo:263-294) from the side of one mate: R1 sits
+// in lane 2i, R2 in lane 2i + 1; seq_len = len(SEQ) of this lane's read.
+__device__ __forceinline__ void pair_up(Hit& h, uint32_t seq_len, bool second) {
+    const bool mstar = __shfl_xor_sync(FULL, static_cast<int>(h.star), 1) != 0;
+    const uint32_t mcanon = __shfl_xor_sync(FULL, h.canon, 1), mlen = __shfl_xor_sync(FULL, h.contig_len, 1);
+    const uint32_t mseq = __shfl_xor_sync(FULL, seq_len, 1);
+    const int64_t mpos1 = __shfl_xor_sync(FULL, h.pos1, 1);
+    const uint64_t moff = __shfl_xor_sync(FULL, h.contig_off, 1);
+    h.flag |= second ? 1 | 128 : 1 | 64;
+    if (!h.star && !mstar && h.canon == mcanon) {
+        h.flag |= 2;
+        h.rnext_kind = K_EQ;
+        h.pnext = mpos1;
+        int64_t t = mpos1 - h.pos1;
         if (t < 0) t = -t;
-        t += len2;
-        a.tlen = t;
-        b.tlen = -t;
+        t += second ? seq_len : mseq;  // len(SEQ of R2)
+        h.tlen = second ? -t : t;
         return;
     }
-    if (a.star) b.flag |= 8;
-    if (b.star) a.flag |= 8;
-    if (!a.star) {
-        b.rnext_kind = K_NAME;
-        b.rnext_off = a.contig_off;
-        b.rnext_len = a.contig_len;
-        b.pnext = a.pos1;
-    }
-    if (!b.star) {
-        a.rnext_kind = K_NAME;
-        a.rnext_off = b.contig_off;
-        a.rnext_len = b.contig_len;
-        a.pnext = b.pos1;
+    if (mstar) {
+        h.flag |= 8;
+    } else {
+        h.rnext_kind = K_NAME;
+        h.rnext_off = moff;
+        h.rnext_len = mlen;
+        h.pnext = mpos1;
     }
 }
 
@@ -154,18 +151,6 @@ __device__ __forceinline__ uint64_t mag(int64_t v) {
 }
 
 __device__ __forceinline__ uint32_t sdig(int64_t v) { return (v < 0) + ndig(mag(v)); }
-
-__device__ __forceinline__ uint32_t cigar_len(const Hit& h) {
-    if (!h.mapped) return 1;
-    return (h.sl > 0 ? sdig(h.sl) + 1 : 0) + sdig(h.m) + 1 + (h.sr > 0 ? sdig(h.sr) + 1 : 0);
-}
-
-// Bytes from the line's start to SEQ: the name (width name_w) and the
-// tab-separated fields FLAG .. TLEN.
-__device__ __forceinline__ uint64_t head_len(const Hit& h, uint64_t name_w) {
-    return name_w + 1 + sdig(h.flag) + 1 + h.contig_len + 1 + sdig(h.pos1) + 1 + sdig(h.mapq) + 1 + cigar_len(h) +
-           1 + h.rnext_len + 1 + sdig(h.pnext) + 1 + sdig(h.tlen) + 1;
-}
 
 // Strict UTF-8 (RFC 3629): no overlong forms, surrogates or code points
 // above U+10FFFF.
@@ -219,6 +204,16 @@ struct LineRec {
 };
 static_assert(sizeof(LineRec) == 80, "line record layout");
 
+__device__ __forceinline__ uint32_t clip_dig(uint32_t n) { return n ? ndig(n) + 1 : 0; }
+
+// Length of a line's formatted fields, from the tab after the name to the
+// one before SEQ.
+__device__ __forceinline__ uint64_t fields_len(const LineRec& h) {
+    const uint32_t cig = h.mapped ? clip_dig(h.sl) + ndig(h.m) + 1 + clip_dig(h.sr) : 1;
+    return 9ull + sdig(h.flag) + h.contig_len + sdig(h.pos1) + ndig(h.mapq) + cig + h.rnext_len + sdig(h.pnext) +
+           sdig(h.tlen);
+}
+
 // Bytes >= 0x80 in p[0, n), from the aligned 16-byte blocks that cover the
 // span (their bytes outside the span lie in the same block as one inside).
 __device__ __forceinline__ uint32_t count_high(const uint8_t* p, uint32_t n) {
@@ -244,11 +239,28 @@ __device__ __forceinline__ uint32_t count_high(const uint8_t* p, uint32_t n) {
     return c;
 }
 
-// One thread per pair (one per read single-end): both hits, the pairing,
-// each line's length and record; the SEQ / QUAL UTF-8 check; mapped records
-// and error bits gathered per block.
-__global__ void __launch_bounds__(THREADS) sam_layout_kernel(SamDev d, uint64_t n_units, uint32_t* line_len,
-                                                             LineRec* recs) {
+// This lane's part of the 16-byte blocks that cover [lo, hi) (at most 1009
+// bytes), ORed: the bit 0x80 of some byte tells a byte >= 0x80.
+__device__ __forceinline__ uint32_t covered_or(const uint8_t* lo, const uint8_t* hi, uint32_t lane) {
+    const uintptr_t e = reinterpret_cast<uintptr_t>(hi), q = (reinterpret_cast<uintptr_t>(lo) & ~uintptr_t(15)) + 16 * lane;
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+    const uint4 v = q < e ? __ldg(reinterpret_cast<const uint4*>(q)) : zero;
+    const uint4 w = q + 512 < e ? __ldg(reinterpret_cast<const uint4*>(q + 512)) : zero;
+    return (v.x | v.y | v.z | v.w | w.x | w.y | w.z | w.w) & 0x80808080u;
+}
+
+// One thread per line: its hit, the pairing (by shuffle), its length and
+// record; the SEQ / QUAL UTF-8 check; mapped records and error bits gathered
+// per block.  The warp looks through each record's bytes together (the stretch
+// from its first span to the end of its last one, up to HIGH_SPAN bytes):
+// without a byte >= 0x80 there no name widens and SEQ and QUAL are valid,
+// otherwise the record's own thread checks its spans.  1 M records of 356
+// bytes: 137 us; with a thread per pair that walked the pair's bytes 222.
+constexpr uint64_t HIGH_SPAN = 1008;
+constexpr int HIGH_UNROLL = 4;  // records whose bytes are on their way at once
+
+__global__ void __launch_bounds__(THREADS, 4) sam_layout_kernel(SamDev d, uint64_t n_lines, uint32_t* line_len,
+                                                                LineRec* recs) {
     __shared__ unsigned long long blk_mapped;
     __shared__ unsigned blk_err;
     if (threadIdx.x == 0) {
@@ -259,53 +271,73 @@ __global__ void __launch_bounds__(THREADS) sam_layout_kernel(SamDev d, uint64_t 
     unsigned err = 0;
     uint32_t mapped = 0;
     const uint64_t stride = static_cast<uint64_t>(gridDim.x) * THREADS;
-    for (uint64_t u = static_cast<uint64_t>(blockIdx.x) * THREADS + threadIdx.x; u < n_units; u += stride) {
-        Hit hs[2];
-        hs[0] = hit_of(d, u, err);
-        const int k = d.paired ? 2 : 1;
-        if (d.paired) {
-            hs[1] = hit_of(d, u + d.n1, err);
-            pair_up(hs[0], hs[1], d.seq_len[u + d.n1]);
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint64_t base = static_cast<uint64_t>(blockIdx.x) * THREADS + (threadIdx.x & ~31u); base < n_lines;
+         base += stride) {
+        const uint64_t L = base + lane;
+        const uint64_t r = d.paired ? (L >> 1) + (L & 1) * d.n1 : L;
+        const bool mine = L < n_lines;
+        const bool spans = mine && spans_ok(d, r);
+        uint64_t lo = 0, hi = 0;
+        if (spans) {
+            const uint64_t a = d.name_off[r], b = d.seq_off[r], c = d.qual_off[r];
+            lo = min(a, min(b, c));
+            hi = max(a + d.name_len[r], max(b + d.seq_len[r], c + d.qual_len[r]));
+            if (hi - lo > HIGH_SPAN) hi = lo;
         }
-        for (int m = 0; m < k; ++m) {
-            const Hit& h = hs[m];
-            const uint64_t r = u + static_cast<uint64_t>(m) * d.n1;
-            const uint64_t L = d.paired ? 2 * u + m : u;
-            if (!spans_ok(d, r)) {
-                err |= E_SPAN;
-                line_len[L] = 0;
-                continue;
-            }
+        uint32_t seen = 0;  // bit k: lane k's record holds a byte >= 0x80
+        for (int k = 0; k < 32; k += HIGH_UNROLL) {
+            uint32_t v[HIGH_UNROLL];
+#pragma unroll
+            for (int j = 0; j < HIGH_UNROLL; ++j)
+                v[j] = covered_or(d.arena + __shfl_sync(FULL, lo, k + j), d.arena + __shfl_sync(FULL, hi, k + j), lane);
+#pragma unroll
+            for (int j = 0; j < HIGH_UNROLL; ++j) seen |= (__any_sync(FULL, v[j] != 0) ? 1u : 0u) << (k + j);
+        }
+        const bool clean = hi > lo && !((seen >> lane) & 1u);
+        Hit h{};
+        h.star = true;
+        const uint32_t n_sq = mine ? d.seq_len[r] : 0;
+        if (mine) h = hit_of(d, r, err);
+        if (d.paired) pair_up(h, n_sq, L & 1);
+        if (!mine) continue;
+        if (!spans) {
+            err |= E_SPAN;
+            line_len[L] = 0;
+            continue;
+        }
+        const uint32_t n_nm = d.name_len[r], n_ql = d.qual_len[r];
+        uint32_t high = 0;
+        if (!clean) {
             const uint8_t* sq = d.arena + d.seq_off[r];
             const uint8_t* ql = d.arena + d.qual_off[r];
-            const uint32_t n_nm = d.name_len[r], n_sq = d.seq_len[r], n_ql = d.qual_len[r];
-            const uint32_t high = count_high(d.arena + d.name_off[r], n_nm);
+            high = count_high(d.arena + d.name_off[r], n_nm);
             if ((count_high(sq, n_sq) || count_high(ql, n_ql)) && !(utf8_ok(sq, n_sq) && utf8_ok(ql, n_ql)))
                 err |= E_UTF8;
-            const uint64_t len = head_len(h, n_nm + 2ull * high) + n_sq + 1 + n_ql + 6 + d.rg_n + 1;
-            if (len > 0xffffffffull) err |= E_OVER;
-            line_len[L] = static_cast<uint32_t>(len);
-            mapped += !h.star;
-            LineRec rc;
-            rc.flag = h.flag;
-            rc.pos1 = h.pos1;
-            rc.pnext = h.pnext;
-            rc.tlen = h.tlen;
-            rc.contig_off = h.contig_off;
-            rc.rnext_off = h.rnext_off;
-            rc.mapq = static_cast<uint32_t>(h.mapq);
-            rc.sl = static_cast<uint32_t>(h.sl);
-            rc.sr = static_cast<uint32_t>(h.sr);
-            rc.m = static_cast<uint32_t>(h.mapped ? h.m : 0);
-            rc.contig_len = h.contig_len;
-            rc.rnext_len = h.rnext_len;
-            rc.contig_kind = h.contig_kind;
-            rc.rnext_kind = h.rnext_kind;
-            rc.mapped = h.mapped;
-            rc.widen = high != 0;
-            rc.pad = 0;
-            recs[L] = rc;
         }
+        LineRec rc;
+        rc.flag = h.flag;
+        rc.pos1 = h.pos1;
+        rc.pnext = h.pnext;
+        rc.tlen = h.tlen;
+        rc.contig_off = h.contig_off;
+        rc.rnext_off = h.rnext_off;
+        rc.mapq = static_cast<uint32_t>(h.mapq);
+        rc.sl = static_cast<uint32_t>(h.sl);
+        rc.sr = static_cast<uint32_t>(h.sr);
+        rc.m = static_cast<uint32_t>(h.mapped ? h.m : 0);
+        rc.contig_len = h.contig_len;
+        rc.rnext_len = h.rnext_len;
+        rc.contig_kind = h.contig_kind;
+        rc.rnext_kind = h.rnext_kind;
+        rc.mapped = h.mapped;
+        rc.widen = high != 0;
+        rc.pad = 0;
+        const uint64_t len = n_nm + 2ull * high + fields_len(rc) + n_sq + 1 + n_ql + 6 + d.rg_n + 1;
+        if (len > 0xffffffffull) err |= E_OVER;
+        line_len[L] = static_cast<uint32_t>(len);
+        mapped += !h.star;
+        recs[L] = rc;
     }
     for (int o = 16; o > 0; o >>= 1) {
         err |= __shfl_xor_sync(FULL, err, o);
@@ -319,59 +351,6 @@ __global__ void __launch_bounds__(THREADS) sam_layout_kernel(SamDev d, uint64_t 
     if (threadIdx.x == 0) {
         if (blk_mapped) atomicAdd(&d.status[1], blk_mapped);
         if (blk_err) atomicOr(&d.status[2], static_cast<unsigned long long>(blk_err));
-    }
-}
-
-// The aligned 4-byte words covering a span, up to 32 * SPAN_UNROLL of them
-// (256 bytes) loaded at once: one round of loads for a span that fits.
-struct SpanWords {
-    uint32_t v[SPAN_UNROLL];
-    uint32_t lead, nw;
-};
-
-__device__ __forceinline__ bool span_fits(const uint8_t* src, uint32_t n) {
-    return ((reinterpret_cast<uintptr_t>(src) & 3) + n + 3) / 4 <= 32u * SPAN_UNROLL;
-}
-
-__device__ __forceinline__ void span_load(SpanWords& s, const uint8_t* src, uint32_t n, int lane) {
-    const uintptr_t a = reinterpret_cast<uintptr_t>(src);
-    const uint32_t* w0 = reinterpret_cast<const uint32_t*>(a & ~uintptr_t(3));
-    s.lead = static_cast<uint32_t>(a & 3);
-    s.nw = n ? (s.lead + n + 3) >> 2 : 0;
-#pragma unroll
-    for (int t = 0; t < SPAN_UNROLL; ++t) {
-        const uint32_t i = 32 * t + lane;
-        s.v[t] = i < s.nw ? w0[i] : 0u;
-    }
-}
-
-template <typename F>
-__device__ __forceinline__ void span_scatter(const SpanWords& s, uint32_t n, int lane, F&& f) {
-#pragma unroll
-    for (int t = 0; t < SPAN_UNROLL; ++t) {
-        const uint32_t i = 32 * t + lane;
-        if (i < s.nw) {
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const uint32_t j = 4 * i + k - s.lead;  // wraps below the span's start
-                if (j < n) f(j, static_cast<uint8_t>(s.v[t] >> (8 * k)));
-            }
-        }
-    }
-}
-
-// Calls f(j, byte) for every byte j of src[0, n), any length, 32 *
-// SPAN_UNROLL words per round.
-template <typename F>
-__device__ __forceinline__ void for_span_bytes(const uint8_t* src, uint32_t n, int lane, F&& f) {
-    for (uint32_t b = 0; b < n;) {
-        const uint8_t* p = src + b;
-        const uint32_t lead = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(p) & 3);
-        const uint32_t take = min(n - b, 32u * SPAN_UNROLL * 4 - lead);
-        SpanWords s;
-        span_load(s, p, take, lane);
-        span_scatter(s, take, lane, [&](uint32_t j, uint8_t c) { f(b + j, c); });
-        b += take;
     }
 }
 
@@ -392,147 +371,155 @@ __device__ __forceinline__ void put_int(uint8_t* o, int64_t v, uint32_t k) {
     if (v < 0) o[0] = '-';
 }
 
-// Lanes copy a contig field: a name span, "*" or "=".
-__device__ __forceinline__ void put_field(uint8_t* o, const SamDev& d, uint8_t kind, uint64_t off, uint32_t len,
-                                          int lane) {
+// A contig field at o: a name span, "*" or "=" (one lane).
+__device__ __forceinline__ void put_field(uint8_t* o, const SamDev& d, uint8_t kind, uint64_t off, uint32_t len) {
     if (kind == K_NAME) {
-        for (uint32_t j = lane; j < len; j += 32) o[j] = d.names[off + j];
-    } else if (lane == 0) {
+        for (uint32_t j = 0; j < len; ++j) o[j] = __ldg(d.names + off + j);
+    } else {
         o[0] = kind == K_EQ ? '=' : '*';
     }
 }
 
-__device__ __forceinline__ uint8_t complement(uint8_t c) {
-    return c == 'A' ? 'T' : c == 'T' ? 'A' : c == 'C' ? 'G' : c == 'G' ? 'C' : 'N';
+// \t FLAG \t RNAME \t POS \t MAPQ \t CIGAR \t RNEXT \t PNEXT \t TLEN \t at o (one
+// lane); fields_len(h) bytes.
+__device__ __forceinline__ void put_fields(uint8_t* o, const SamDev& d, const LineRec& h) {
+    auto num = [&](int64_t v, uint8_t after) {
+        const uint32_t k = sdig(v);
+        put_int(o, v, k);
+        o[k] = after;
+        o += k + 1;
+    };
+    *o++ = '\t';
+    num(h.flag, '\t');
+    put_field(o, d, h.contig_kind, h.contig_off, h.contig_len);
+    o += h.contig_len;
+    *o++ = '\t';
+    num(h.pos1, '\t');
+    num(h.mapq, '\t');
+    if (h.mapped) {
+        if (h.sl) num(h.sl, 'S');
+        num(h.m, 'M');
+        if (h.sr) num(h.sr, 'S');
+    } else {
+        *o++ = '*';
+    }
+    *o++ = '\t';
+    put_field(o, d, h.rnext_kind, h.rnext_off, h.rnext_len);
+    o += h.rnext_len;
+    *o++ = '\t';
+    num(h.pnext, '\t');
+    num(h.tlen, '\t');
 }
 
-// One line at o (shared-memory stage or the output itself) by the warp.
-// The name, SEQ and QUAL words are loaded before the integer fields are
-// formatted, so the loads overlap that work.
-__device__ void build_line(uint8_t* o, const SamDev& d, const LineRec& h, const uint8_t* nm, uint32_t n_nm,
-                           const uint8_t* sq, uint32_t n_sq, const uint8_t* ql, uint32_t n_ql, int lane) {
-    const bool pre = !h.widen && span_fits(nm, n_nm) && span_fits(sq, n_sq) && span_fits(ql, n_ql);
-    SpanWords wn, ws, wq;
-    if (pre) {
-        span_load(wn, nm, n_nm, lane);
-        span_load(ws, sq, n_sq, lane);
-        span_load(wq, ql, n_ql, lane);
+// The reverse strand's bases of four read backwards: A<->T, C<->G, any other
+// byte N.  Bits 1-2 of a letter tell A, C, T and G apart; the letter they
+// stand for is compared with the byte to find the others.
+__device__ __forceinline__ uint32_t complement4(uint32_t x) {
+    const uint32_t i = (x >> 1) & 0x03030303u;
+    const uint32_t sel = __byte_perm(i | (i >> 4), 0, 0x4420);  // one nibble per base
+    const uint32_t d = __byte_perm(0x47544341u, 0, sel) ^ x;
+    const uint32_t other = (((((d & 0x7f7f7f7fu) + 0x7f7f7f7fu) | d) >> 7) & 0x01010101u) * 255u;
+    return (__byte_perm(0x43414754u, 0, sel) & ~other) | (0x4e4e4e4eu & other);
+}
+
+__device__ __forceinline__ uint8_t tail_byte(const SamDev& d, uint32_t j) {
+    if (j < 6) return "\tRG:Z:"[j];
+    return j < 6 + d.rg_n ? d.rg[j - 6] : '\n';
+}
+
+// What the warp needs of a line to write its bytes, filled in by one lane.
+struct __align__(16) LinePlan {
+    const uint8_t *name, *seq, *qual;
+    uint32_t n_nm, n_sq, n_ql;
+    uint32_t fields;  // bytes of the formatted fields, 0: not formatted (slow_line)
+    uint32_t rc;
+    uint32_t pad;
+};
+static_assert(sizeof(LinePlan) == 48, "line plan layout");
+
+// A lane's share of a line's source bytes: two name bytes, eight bases and
+// eight qualities; for lines of up to 64 name bytes and 256 bases that is all
+// of them.
+struct LineRaw {
+    uint32_t n0, n1;
+    span::Span8 seq, qual;
+};
+
+__device__ __forceinline__ void load_raw(LineRaw& x, const LinePlan& q, uint32_t lane) {
+    x.n0 = lane < q.n_nm ? __ldg(q.name + lane) : 0;
+    x.n1 = lane + 32 < q.n_nm ? __ldg(q.name + lane + 32) : 0;
+    x.seq = span::span8_load(q.seq, q.n_sq, lane, q.rc);
+    x.qual = span::span8_load(q.qual, q.n_ql, lane, false);
+}
+
+// The bytes of a line after its fields, by the warp: SEQ, tab, QUAL and the
+// RG tag; tail: this lane's byte of the tag.
+__device__ __forceinline__ void put_rest(uint8_t* o, const SamDev& d, const LinePlan& q, const LineRaw& x,
+                                         uint32_t tail, uint32_t lane) {
+    const uint32_t n_sq = q.n_sq, n_ql = q.n_ql;
+    const bool rc = q.rc;
+    for (uint32_t i = lane; 8 * i < n_sq; i += 32) {
+        const uint32_t left = n_sq - 8 * i;
+        uint2 v = span::span8_bytes(i < 32 ? x.seq : span::span8_load(q.seq, n_sq, i, rc), q.seq, n_sq, rc);
+        if (rc) v = make_uint2(complement4(v.x), complement4(v.y));
+        span::put_bytes(o + 8 * i, v.x, min(4u, left));
+        if (left > 4) span::put_bytes(o + 8 * i + 4, v.y, min(4u, left - 4));
     }
-    uint64_t w = n_nm;
-    if (h.widen) {  // each byte >= 0x80 of the name becomes U+FFFD
-        w = 0;
-        for (uint32_t b = 0; b < n_nm; b += 32) {
-            const uint32_t i = b + lane;
-            const uint8_t c = i < n_nm ? nm[i] : 0;
-            const uint32_t wd = i < n_nm ? (c >= 0x80 ? 3u : 1u) : 0u;
-            uint32_t incl = wd;
-            for (int s = 1; s < 32; s <<= 1) {
-                const uint32_t v = __shfl_up_sync(FULL, incl, s);
-                if (lane >= s) incl += v;
-            }
-            const uint32_t ex = incl - wd;
-            if (wd == 1) {
-                o[w + ex] = c;
-            } else if (wd == 3) {
-                o[w + ex] = 0xef;
-                o[w + ex + 1] = 0xbf;
-                o[w + ex + 2] = 0xbd;
-            }
-            w += __shfl_sync(FULL, incl, 31);
-        }
+    if (lane == 0) o[n_sq] = '\t';
+    uint8_t* oq = o + n_sq + 1;
+    for (uint32_t i = lane; 8 * i < n_ql; i += 32) {
+        const uint32_t left = n_ql - 8 * i;
+        const uint2 v = span::span8_bytes(i < 32 ? x.qual : span::span8_load(q.qual, n_ql, i, false), q.qual, n_ql, false);
+        span::put_bytes(oq + 8 * i, v.x, min(4u, left));
+        if (left > 4) span::put_bytes(oq + 8 * i + 4, v.y, min(4u, left - 4));
     }
-    // FLAG, RNAME, POS, MAPQ, CIGAR, RNEXT, PNEXT, TLEN: every lane knows the
-    // layout
-    const uint32_t d_flag = sdig(h.flag), d_pos = sdig(h.pos1), d_mapq = ndig(h.mapq);
-    const uint32_t d_sl = h.sl > 0 ? ndig(h.sl) + 1 : 0, d_m = h.mapped ? ndig(h.m) : 0;
-    const uint32_t d_sr = h.sr > 0 ? ndig(h.sr) + 1 : 0, d_pn = sdig(h.pnext), d_tl = sdig(h.tlen);
-    const uint32_t cig = h.mapped ? d_sl + d_m + 1 + d_sr : 1;
-    const uint64_t w_contig = w + 2 + d_flag;
-    const uint64_t p_tab3 = w_contig + h.contig_len, p_pos = p_tab3 + 1, p_mapq = p_pos + d_pos + 1;
-    const uint64_t p_cig = p_mapq + d_mapq + 1;
-    const uint64_t w_rnext = p_cig + cig + 1;
-    const uint64_t p_tab7 = w_rnext + h.rnext_len, p_pnext = p_tab7 + 1, p_tlen = p_pnext + d_pn + 1;
-    const uint64_t w_seq = p_tlen + d_tl + 1;
-    // each of lanes 0-7 picks one number, lanes 3-5 and 8-16 one separator;
-    // the picks are selects, the writes one code path for all lanes
-    int64_t v = 0;
-    uint64_t vp = 0, cp = 0;
-    uint32_t vn = 0;
-    uint8_t ch = '\t';
-    bool vb = lane < 8, cb = lane >= 8 && lane <= 16;
-    if (lane == 0) {
-        v = h.flag, vp = w + 1, vn = d_flag;
-    } else if (lane == 1) {
-        v = h.pos1, vp = p_pos, vn = d_pos;
-    } else if (lane == 2) {
-        v = h.mapq, vp = p_mapq, vn = d_mapq;
-    } else if (lane == 3) {
-        vb = cb = h.mapped && h.sl > 0;
-        v = h.sl, vp = p_cig, vn = d_sl - 1, cp = p_cig + d_sl - 1, ch = 'S';
-    } else if (lane == 4) {
-        vb = h.mapped;
-        cb = true;
-        v = h.m, vp = p_cig + d_sl, vn = d_m;
-        cp = h.mapped ? p_cig + d_sl + d_m : p_cig;
-        ch = h.mapped ? 'M' : '*';
-    } else if (lane == 5) {
-        vb = cb = h.mapped && h.sr > 0;
-        v = h.sr, vp = p_cig + d_sl + d_m + 1, vn = d_sr - 1, cp = p_cig + d_sl + d_m + d_sr, ch = 'S';
-    } else if (lane == 6) {
-        v = h.pnext, vp = p_pnext, vn = d_pn;
-    } else if (lane == 7) {
-        v = h.tlen, vp = p_tlen, vn = d_tl;
-    } else {  // the nine tabs
-        cp = lane == 8    ? w
-             : lane == 9  ? w_contig - 1
-             : lane == 10 ? p_tab3
-             : lane == 11 ? p_mapq - 1
-             : lane == 12 ? p_cig - 1
-             : lane == 13 ? w_rnext - 1
-             : lane == 14 ? p_tab7
-             : lane == 15 ? p_tlen - 1
-                          : w_seq - 1;
-    }
-    if (vb) put_int(o + vp, v, vn);
-    if (cb) o[cp] = ch;
-    put_field(o + w_contig, d, h.contig_kind, h.contig_off, h.contig_len, lane);
-    put_field(o + w_rnext, d, h.rnext_kind, h.rnext_off, h.rnext_len, lane);
-    uint8_t* os = o + w_seq;
-    uint8_t* oq = os + n_sq + 1;
-    const bool rc = h.mapped && (h.flag & 16);
-    auto seq_f = [&](uint32_t j, uint8_t c) { os[j] = c; };
-    auto seq_r = [&](uint32_t j, uint8_t c) { os[n_sq - 1 - j] = complement(c); };
-    auto qual_f = [&](uint32_t j, uint8_t c) { oq[j] = c; };
-    if (pre) {
-        span_scatter(wn, n_nm, lane, [&](uint32_t j, uint8_t c) { o[j] = c; });
-        if (rc) span_scatter(ws, n_sq, lane, seq_r);
-        else span_scatter(ws, n_sq, lane, seq_f);
-        span_scatter(wq, n_ql, lane, qual_f);
-    } else {
-        if (!h.widen) for_span_bytes(nm, n_nm, lane, [&](uint32_t j, uint8_t c) { o[j] = c; });
-        if (rc) for_span_bytes(sq, n_sq, lane, seq_r);
-        else for_span_bytes(sq, n_sq, lane, seq_f);
-        for_span_bytes(ql, n_ql, lane, qual_f);
-    }
-    // SEQ <tab> QUAL, then "\tRG:Z:" + id + "\n"
-    if (lane == 0) os[n_sq] = '\t';
     uint8_t* ot = oq + n_ql;
     const uint32_t n_tail = 7 + d.rg_n;
-    for (uint32_t j = lane; j < n_tail; j += 32) {
-        uint8_t c;
-        if (j < 6) c = "\tRG:Z:"[j];
-        else if (j < 6 + d.rg_n) c = d.rg[j - 6];
-        else c = '\n';
-        ot[j] = c;
-    }
+    if (lane < n_tail) ot[lane] = static_cast<uint8_t>(tail);
+    if (n_tail > 32)
+        for (uint32_t j = 32 + lane; j < n_tail; j += 32) ot[j] = tail_byte(d, j);
 }
 
-// One warp per line: the line in the warp's shared-memory stage at its
-// destination's 16-byte phase, then 16-byte stores (byte stores at the
-// ragged ends); lines longer than the stage are built in place.
-__global__ void __launch_bounds__(THREADS) sam_write_kernel(SamDev d, uint64_t n_lines, const uint64_t* ends,
-                                                            const LineRec* recs) {
-    __shared__ __align__(16) uint8_t stage[WARPS][STAGE];
+// The name and fields of a line whose fields do not fit a slot or whose name
+// has bytes >= 0x80 (each becomes U+FFFD); returns their bytes.
+__device__ __noinline__ uint64_t slow_head(uint8_t* o, const SamDev& d, const LineRec& h, const uint8_t* nm, uint32_t n_nm,
+                                           uint32_t lane) {
+    uint64_t w = 0;
+    for (uint32_t b = 0; b < n_nm; b += 32) {
+        const uint32_t i = b + lane;
+        const uint8_t c = i < n_nm ? nm[i] : 0;
+        const uint32_t wd = i < n_nm ? (c >= 0x80 ? 3u : 1u) : 0u;
+        uint32_t incl = wd;
+        for (int s = 1; s < 32; s <<= 1) {
+            const uint32_t v = __shfl_up_sync(FULL, incl, s);
+            if (lane >= s) incl += v;
+        }
+        const uint32_t ex = incl - wd;
+        if (wd == 1) {
+            o[w + ex] = c;
+        } else if (wd == 3) {
+            o[w + ex] = 0xef;
+            o[w + ex + 1] = 0xbf;
+            o[w + ex + 2] = 0xbd;
+        }
+        w += __shfl_sync(FULL, incl, 31);
+    }
+    if (lane == 0) put_fields(o + w, d, h);
+    return w + fields_len(h);
+}
+
+// A warp takes `per` consecutive lines.  One lane per line formats its
+// fields into a slot of shared memory (all 32 lanes busy); the warp then puts
+// the lines together one after the other in its stage and stores it in
+// 16-byte blocks when the next line does not fit.
+// Bound by instruction issue: 1 M lines of 388 B take 0.47 ms; with each
+// line's fields formatted by its warp, eight lanes busy, and byte-wise copies
+// it was 2.04 ms.
+__global__ void __launch_bounds__(WRITE_WARPS * 32) sam_write_kernel(SamDev d, uint64_t n_lines, const uint64_t* ends,
+                                                                    const LineRec* recs, uint32_t per) {
+    __shared__ __align__(16) uint8_t s_stage[WRITE_WARPS][STAGE + 16];
+    __shared__ LinePlan s_plan[WRITE_WARPS][32];
+    __shared__ uint8_t s_slot[WRITE_WARPS][32][SLOT];
     const uint64_t total = ends[n_lines - 1];
     const bool over = total > d.cap;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -542,39 +529,57 @@ __global__ void __launch_bounds__(THREADS) sam_write_kernel(SamDev d, uint64_t n
     // error bits of the layout pass (the overflow bit above only repeats
     // `over`)
     if (over || *static_cast<volatile unsigned long long*>(&d.status[2]) != 0) return;
-    const int lane = threadIdx.x & 31;
-    uint8_t* sb = stage[threadIdx.x >> 5];
-    const uint64_t w0 = (static_cast<uint64_t>(blockIdx.x) * THREADS + threadIdx.x) >> 5;
-    const uint64_t nw = static_cast<uint64_t>(gridDim.x) * WARPS;
-    for (uint64_t L = w0; L < n_lines; L += nw) {
-        const LineRec h = recs[L];
-        const uint64_t r = d.paired ? (L >> 1) + (L & 1) * d.n1 : L;
-        const uint64_t start = L ? ends[L - 1] : 0, len = ends[L] - start;
-        const uint8_t* nm = d.arena + d.name_off[r];
-        const uint8_t* sq = d.arena + d.seq_off[r];
-        const uint8_t* ql = d.arena + d.qual_off[r];
-        const uint32_t n_nm = d.name_len[r], n_sq = d.seq_len[r], n_ql = d.qual_len[r];
-        const uintptr_t gs = reinterpret_cast<uintptr_t>(d.sam) + start, ge = gs + len;
-        const uint32_t ph = static_cast<uint32_t>(gs & 15);
-        if (ph + len > STAGE) {
-            build_line(d.sam + start, d, h, nm, n_nm, sq, n_sq, ql, n_ql, lane);
-            continue;
-        }
-        build_line(sb + ph, d, h, nm, n_nm, sq, n_sq, ql, n_ql, lane);
-        __syncwarp();
-        const uintptr_t a0 = gs - ph;  // sb[0] stands for this aligned address
-        for (uintptr_t c = a0 + 16 * lane; c < ge; c += 512) {
-            const uint32_t so = static_cast<uint32_t>(c - a0);
-            if (c >= gs && c + 16 <= ge) {
-                *reinterpret_cast<uint4*>(c) = *reinterpret_cast<const uint4*>(sb + so);
-            } else {
-                for (int k = 0; k < 16; ++k) {
-                    const uintptr_t x = c + k;
-                    if (x >= gs && x < ge) *reinterpret_cast<uint8_t*>(x) = sb[so + k];
-                }
-            }
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    LinePlan* plan = s_plan[warp];
+    uint8_t(*slot)[SLOT] = s_slot[warp];
+    const uint32_t tail = lane < 7 + d.rg_n ? tail_byte(d, lane) : 0;
+    const uint64_t n_warps = static_cast<uint64_t>(gridDim.x) * WRITE_WARPS;
+    for (uint64_t base = (static_cast<uint64_t>(blockIdx.x) * WRITE_WARPS + warp) * per; base < n_lines;
+         base += n_warps * per) {
+        const uint64_t L = base + lane;
+        uint64_t start = 0;
+        uint32_t bytes = 0;
+        if (lane < per && L < n_lines) {
+            const LineRec h = recs[L];
+            const uint64_t r = d.paired ? (L >> 1) + (L & 1) * d.n1 : L;
+            start = L ? ends[L - 1] : 0;
+            bytes = static_cast<uint32_t>(ends[L] - start);
+            LinePlan q;
+            q.name = d.arena + d.name_off[r];
+            q.seq = d.arena + d.seq_off[r];
+            q.qual = d.arena + d.qual_off[r];
+            q.n_nm = d.name_len[r];
+            q.n_sq = d.seq_len[r];
+            q.n_ql = d.qual_len[r];
+            q.rc = h.mapped && (h.flag & 16);
+            const uint64_t f = fields_len(h);
+            q.fields = !h.widen && f <= SLOT ? static_cast<uint32_t>(f) : 0;
+            if (q.fields) put_fields(slot[lane], d, h);
+            plan[lane] = q;
         }
         __syncwarp();
+        const uint32_t count = static_cast<uint32_t>(n_lines - base < per ? n_lines - base : per);
+        LineRaw next;
+        load_raw(next, plan[0], lane);
+        span::staged_run<STAGE>(d.sam + __shfl_sync(FULL, start, 0), s_stage[warp], bytes, count, lane,
+                                [&](uint8_t* o, uint32_t k) {
+                                    const LineRaw x = next;  // the next line's bytes are on their way
+                                    const LinePlan& q = plan[k];
+                                    if (k + 1 < count) load_raw(next, plan[k + 1], lane);
+                                    const uint32_t n_nm = q.n_nm, fields = q.fields;
+                                    if (!fields) {
+                                        o += slow_head(o, d, recs[base + k], q.name, n_nm, lane);
+                                    } else {
+                                        if (lane < n_nm) o[lane] = static_cast<uint8_t>(x.n0);
+                                        if (lane + 32 < n_nm) o[lane + 32] = static_cast<uint8_t>(x.n1);
+                                        if (n_nm > 64)
+                                            for (uint32_t i = 64 + lane; i < n_nm; i += 32) o[i] = __ldg(q.name + i);
+                                        o += n_nm;
+                                        for (uint32_t i = lane; i < fields; i += 32) o[i] = slot[k][i];
+                                        o += fields;
+                                    }
+                                    put_rest(o, d, q, x, tail, lane);
+                                });
     }
 }
 
@@ -600,15 +605,19 @@ int enqueue_sam(const SamDev& d, void* scratch, size_t scratch_bytes, int sm_cou
     void* temp = s;
     size_t tb = scratch_bytes - static_cast<size_t>(s - static_cast<uint8_t*>(scratch));
     const uint64_t sms = static_cast<uint64_t>(sm_count > 0 ? sm_count : 148);
-    const uint64_t n_units = d.n1;  // pairs, or reads single-end
-    const uint64_t g1w = (n_units + THREADS - 1) / THREADS, g1c = sms * 8;
-    sam_layout_kernel<<<static_cast<unsigned>(g1w < g1c ? g1w : g1c), THREADS, 0, st>>>(d, n_units, line_len, recs);
+    const uint64_t g1w = (n_lines + THREADS - 1) / THREADS, g1c = sms * 8;
+    sam_layout_kernel<<<static_cast<unsigned>(g1w < g1c ? g1w : g1c), THREADS, 0, st>>>(d, n_lines, line_len, recs);
     check_launch(cudaGetLastError(), "sam_layout_kernel");
     check_launch(cub::DeviceScan::InclusiveSum(temp, tb, static_cast<const uint32_t*>(line_len), ends,
                                                static_cast<int64_t>(n_lines), st),
                  "sam scan");
-    const uint64_t g2w = (n_lines + WARPS - 1) / WARPS, g2c = sms * 16;
-    sam_write_kernel<<<static_cast<unsigned>(g2w < g2c ? g2w : g2c), THREADS, 0, st>>>(d, n_lines, ends, recs);
+    // 32 lines a warp where that still gives every SM 32 warps, fewer (down to
+    // 4) for a small batch: its lines spread over more warps
+    uint32_t per = 32;
+    while (per > 4 && (n_lines + per - 1) / per < sms * 32) per /= 2;
+    const uint64_t g2w = (n_lines + WRITE_WARPS * per - 1) / (WRITE_WARPS * per), g2c = sms * 16;
+    sam_write_kernel<<<static_cast<unsigned>(g2w < g2c ? g2w : g2c), WRITE_WARPS * 32, 0, st>>>(d, n_lines, ends, recs,
+                                                                                             per);
     check_launch(cudaGetLastError(), "sam_write_kernel");
     return 4;
 }

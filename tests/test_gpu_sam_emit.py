@@ -197,3 +197,41 @@ def test_pair_reader_split_device_form(ctx):
         np.testing.assert_array_equal(got, want[k], err_msg=k)
     with pytest.raises(MojoAlignError, match="unknown FASTQ rules"):
         _parse(ctx, b"@a\nA\n+\nI\n", rules=2)
+
+
+@pytest.mark.parametrize("paired", [False, True])
+@pytest.mark.parametrize("rg", [b"", b"r" * 24, b"r" * 25, b"r" * 26, b"r" * 300])
+def test_lines_at_the_edges_of_the_lanes_the_slots_and_the_stage(ctx, rg, paired):
+    """Bases and qualities around one lane's eight and a warp's 256, lines
+    around the warp's 2048-byte output stage, names around 32 and 64 bytes,
+    contig names that fill a line's field slot or do not fit it."""
+    from mojoalign_b200.bam import BatchArena
+
+    rng = np.random.default_rng(len(rg))
+    lens = [0, 1, 2, 7, 8, 9, 31, 32, 33, 149, 150, 151, 255, 256, 257, 263, 264, 265] * 3
+    lens += list(range(930, 1010, 5)) + [511, 512, 513] + [100] * 41
+    n1 = len(lens)
+    n_seq = n1 * (2 if paired else 1)
+    names = [b"fchr1", b"r" + b"n" * 14, b"f" + b"c" * 40, b"r" + b"d" * 63, b"f" + b"e" * 200, b"fA"]
+
+    def record(n):
+        seq = rng.choice(np.frombuffer(b"ACGTacgtN.", np.uint8), n, p=[.2, .2, .2, .2] + [1 / 30] * 6).tobytes()
+        name = bytes(rng.integers(65, 90, int(rng.choice([0, 1, 31, 32, 33, 63, 64, 65, 96, 97, 130]))).astype(np.uint8))
+        qual = bytes(rng.integers(33, 74, n).astype(np.uint8))
+        odd = rng.random()
+        if odd < 0.05 and n >= 2:
+            qual = "é".encode() + qual[2:]
+        elif odd < 0.1 and name:
+            name = b"\xff" + name[1:]
+        return name, seq, qual
+
+    arena = BatchArena.from_records([record(int(n)) for n in rng.permutation(lens)] +
+                                    ([record(int(n)) for n in rng.permutation(lens)] if paired else []))
+    rid = rng.integers(-1, len(names), n_seq).astype(np.int32)
+    u32 = lambda hi: rng.integers(0, hi, n_seq).astype(np.uint32)  # noqa: E731
+    pos = np.where(rng.random(n_seq) < 0.1, 4294967295, u32(1 << 28)).astype(np.uint32)
+    hits = {"rid": rid, "pos": pos, "mapq": u32(256), "flag": np.where(rid < 0, 4, 16 * (u32(2) == 1)).astype(np.int32),
+            "sl": u32(3) * u32(20), "sr": u32(3) * u32(20), "nm": u32(9)}
+    want = oracle.emit_sam(hits, n1, paired, oracle_arena(arena), names, rg)
+    got = emit_sam_from_batch(ctx, hits, n1, paired, arena, SamContigs.from_names(names), rg)
+    assert got == want
