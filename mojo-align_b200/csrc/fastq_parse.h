@@ -23,8 +23,9 @@ size_t fastq_scratch_bytes(uint64_t n_bytes);
 
 // Splits buf[0, n) into records (synchronous on st) under `rules`: 0 the
 // BAM path's reader (linear_fastq.mojo), 1 the SAM path's (fastq_batch.py).  newline_buffer(user,
-// bytes) supplies the device array of newline positions once their count is
-// known.  h_status: [0] lines, [1] records, [2] bytes consumed, [3] error (0,
+// bytes) supplies the device array of newline positions (a second time, larger,
+// when the text has more lines than it was sized for; its contents need not
+// survive).  h_status: [0] lines, [1] records, [2] bytes consumed, [3] error (0,
 // or 1/2/3: a record missing its SEQ / + / QUAL line), [4] newlines, [5] the
 // longest SEQ.  Returns the number of kernels launched.
 int fastq_parse_enqueue(const uint8_t* buf, uint64_t n, int at_eof, uint64_t max_records, uint64_t base, int rules,

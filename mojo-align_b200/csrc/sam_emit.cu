@@ -242,7 +242,8 @@ __device__ __forceinline__ uint32_t count_high(const uint8_t* p, uint32_t n) {
 // This lane's part of the 16-byte blocks that cover [lo, hi) (at most 1009
 // bytes), ORed: the bit 0x80 of some byte tells a byte >= 0x80.
 __device__ __forceinline__ uint32_t covered_or(const uint8_t* lo, const uint8_t* hi, uint32_t lane) {
-    const uintptr_t e = reinterpret_cast<uintptr_t>(hi), q = (reinterpret_cast<uintptr_t>(lo) & ~uintptr_t(15)) + 16 * lane;
+    const uintptr_t e = lo < hi ? reinterpret_cast<uintptr_t>(hi) : 0;
+    const uintptr_t q = (reinterpret_cast<uintptr_t>(lo) & ~uintptr_t(15)) + 16 * lane;
     const uint4 zero = make_uint4(0, 0, 0, 0);
     const uint4 v = q < e ? __ldg(reinterpret_cast<const uint4*>(q)) : zero;
     const uint4 w = q + 512 < e ? __ldg(reinterpret_cast<const uint4*>(q + 512)) : zero;

@@ -120,3 +120,60 @@ def test_device_form_every_alignment_and_rows(ctx):
         s = text[int(want["seq_off"][i]):int(want["seq_off"][i]) + int(want["seq_len"][i])]
         assert r[i].tobytes() == s + b"N" * (ml - len(s))
     np.testing.assert_array_equal(lens.cpu().numpy().view(np.uint32), want["seq_len"])
+
+
+@pytest.mark.parametrize("rules", [0, 1])
+@pytest.mark.parametrize("records", [300, 100_000])
+def test_texts_with_many_lines_per_byte(ctx, rules, records):
+    """Records of a few bytes: more newlines than the first sizing of the
+    newline array (one per 32 bytes) holds, cut at every phase of the tiles."""
+    rng = np.random.default_rng(records)
+    parts = [b"@%s\n%s\n+\n%s\n" % (b"n" * int(a), b"A" * int(b), b"I" * int(b))
+             for a, b in zip(rng.integers(0, 3, records), rng.integers(0, 4, records))]
+    text = b"".join(parts)
+    parse = oracle.fastq_parse if rules == 0 else oracle.fastq_parse_pr
+    for cut in (len(text), len(text) - 1, 16384, 16383, 16385, 1000):
+        part = text[:cut]
+        b = np.frombuffer(part, np.uint8)
+        out = {k: np.zeros(records + 2, np.uint64 if k.endswith("off") else np.uint32) for k in KEYS}
+        rec = _lib.ma_fastq_records(*[out[k].ctypes.data for k in KEYS])
+        o3 = (C.c_uint64 * 3)()
+        _lib.check(_lib.lib.ma_fastq_parse_rules(ctx.handle, b.ctypes.data, b.size, 0, records + 2, 5, rules, C.byref(rec),
+                                                 o3), ctx.handle)
+        got = {k: v[:o3[0]] for k, v in out.items()}
+        got.update(n=o3[0], consumed=o3[1], max_len=o3[2])
+        _same(got, parse(part, at_eof=False, base=5))
+
+
+@pytest.mark.parametrize("max_len", [1, 3, 15, 16, 17, 31, 150, 4095, 4097])
+def test_rows_at_every_width_and_phase(ctx, max_len):
+    """Row widths around the 16 bytes a thread makes and the 4096 of a CTA, at
+    several alignments of the source and the rows; nothing outside is written."""
+    import torch
+
+    rng = np.random.default_rng(max_len)
+    n = 70
+    arena = rng.integers(65, 90, 40_000, dtype=np.uint8)
+    lens = rng.integers(0, max_len + 20, n).astype(np.uint32)
+    lens[:4] = [0, max_len, max(max_len - 1, 0), max_len + 1]
+    off = np.array([rng.integers(0, arena.size - int(k) + 1) for k in lens], np.uint64)
+    off[5] = arena.size - int(lens[5])
+    dev = torch.device("cuda", 0)
+    d_off, d_len = torch.from_numpy(off.view(np.int64)).to(dev), torch.from_numpy(lens.view(np.int32)).to(dev)
+    want = np.full((n, max_len), 78, np.uint8)
+    for i in range(n):
+        k = min(int(lens[i]), max_len)
+        want[i, :k] = arena[int(off[i]):int(off[i]) + k]
+    for shift, to in ((0, 0), (1, 3), (6, 8), (15, 15)):
+        d_arena = torch.zeros(arena.size + 16, dtype=torch.uint8, device=dev)
+        d_arena[shift:shift + arena.size] = torch.from_numpy(arena).to(dev)
+        rows = torch.zeros(n * max_len + 48, dtype=torch.uint8, device=dev)
+        out_len = torch.zeros(n, dtype=torch.int32, device=dev)
+        torch.cuda.synchronize()
+        _lib.check(_lib.lib.ma_fastq_rows_device(ctx.handle, d_arena.data_ptr() + shift, d_off.data_ptr(), d_len.data_ptr(),
+                                                 n, max_len, rows.data_ptr() + to, out_len.data_ptr(), None), ctx.handle)
+        torch.cuda.synchronize()
+        got = rows.cpu().numpy()
+        np.testing.assert_array_equal(got[to:to + n * max_len].reshape(n, max_len), want)
+        assert not got[:to].any() and not got[to + n * max_len:].any()
+        np.testing.assert_array_equal(out_len.cpu().numpy().view(np.uint32), lens)
