@@ -1,8 +1,7 @@
 // bgzf_inflate.cuh - inflating the members of a BGZF file on the device, one
-// warp per member (bgzf_inflate.cu: lane 0 decodes tokens, the warp writes
-// their bytes and folds the CRC-32).  The per-member step below is the host
-// form: the same token decoder (inflate.cuh) with the sequential writer, so
-// the host tests run the decoder the kernel runs.
+// CTA per member (bgzf_inflate.cu).  The per-member step below is the host
+// form: the token decoder (inflate.cuh) that the kernel runs on members its
+// parallel form leaves, with the sequential writer; it defines the status.
 #pragma once
 
 #include <cstdint>

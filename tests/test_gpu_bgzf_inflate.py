@@ -78,3 +78,111 @@ def test_device_form_status(ctx):
     assert status[2] == 9 and not np.delete(status, 2).any()
     out = d_out.cpu().numpy().tobytes()
     assert out[:t["out_bytes"]] == text and not any(out[t["out_bytes"]:])
+
+
+def _payloads():
+    """(name, raw deflate stream, its bytes) over block kinds, code shapes and
+    sizes around the kernel's: 4 bytes, 130 per thread, strips of 2048, a
+    member of 65280, streams of several blocks and of several rounds."""
+    import zlib
+
+    def raw(data, level=6, strategy=zlib.Z_DEFAULT_STRATEGY, mem=8, flush_every=0, mode=zlib.Z_FULL_FLUSH):
+        c = zlib.compressobj(level, zlib.DEFLATED, -15, mem, strategy)
+        out = b""
+        if flush_every:
+            for a in range(0, len(data), flush_every):
+                out += c.compress(data[a:a + flush_every]) + c.flush(mode)
+        else:
+            out = c.compress(data)
+        return out + c.flush()
+
+    rng = np.random.default_rng(5)
+    text = random_fastq(9, 1500, crlf=0.1)
+    noise = rng.integers(0, 256, 70_000, dtype=np.uint8).tobytes()
+    skewed = rng.choice(256, 70_000, p=np.r_[np.full(1, .9), np.full(255, .1 / 255)]).astype(np.uint8).tobytes()
+    # Fibonacci-like counts: codes up to 15 bits
+    deep = b"".join(bytes([k]) * int(1.6 ** k) for k in range(1, 23))[:65280]
+    deep = bytes(np.random.default_rng(6).permutation(np.frombuffer(deep, np.uint8)))
+    for n in (0, 1, 3, 4, 5, 129, 130, 131, 2047, 2048, 2049, 65279, 65280, 65281, 65536):
+        yield f"text{n}", raw(text[:n]), text[:n]
+        yield f"noise{n}", raw(noise[:n], 9), noise[:n]
+    for level in (0, 1, 9):
+        yield f"level{level}", raw(text[:65280], level), text[:65280]
+    for name, st in (("fixed", zlib.Z_FIXED), ("huffman", zlib.Z_HUFFMAN_ONLY), ("rle", zlib.Z_RLE), ("filtered", zlib.Z_FILTERED)):
+        for kind, data in (("text", text[:65280]), ("skewed", skewed[:65280]), ("deep", deep), ("noise", noise[:65280])):
+            yield f"{name}_{kind}", raw(data, 6, st), data
+    for n in (1, 2, 3, 258, 259, 300, 65280):
+        yield f"run{n}", raw(b"F" * n), b"F" * n
+        yield f"period{n}", raw((b"ACGTTGCAG" * 8000)[:n], 9), (b"ACGTTGCAG" * 8000)[:n]
+    yield "small_blocks", raw(text[:60000], 6, mem=1), text[:60000]
+    for every in (37, 700, 5000, 30000):
+        yield f"flush{every}", raw(text[:65280], 6, flush_every=every), text[:65280]
+    yield "sync_flush", raw(text[:20000], 1, flush_every=1500, mode=zlib.Z_SYNC_FLUSH), text[:20000]
+    yield "trailing", raw(text[:3000]) + b"rest", text[:3000]
+
+
+def _inflate_raw(ctx, members, lead=0, gap=0):
+    """members: (payload, isize, crc) -> statuses and the output buffer's bytes per member."""
+    import torch
+
+    src, so, sl, do, at = bytearray(b"\0" * 5), [], [], [], lead
+    for p, n, _ in members:
+        so.append(len(src))
+        sl.append(len(p))
+        src += p + b"\xff" * 3
+        do.append(at)
+        at += n + gap
+    dev = torch.device("cuda", 0)
+    put = lambda v, t: torch.from_numpy(np.array(v, t).view(np.int64 if t == np.uint64 else np.int32)).to(dev)  # noqa: E731
+    d_in = torch.frombuffer(src, dtype=torch.uint8).to(dev)
+    d_out = torch.full((at + 64,), 7, dtype=torch.uint8, device=dev)
+    status = torch.full((len(members),), 77, dtype=torch.int32, device=dev)
+    cols = [put(so, np.uint64), put(sl, np.uint32), put(do, np.uint64), put([n for _, n, _ in members], np.uint32),
+            put([c for _, _, c in members], np.uint32)]
+    torch.cuda.synchronize()
+    _lib.check(_lib.lib.ma_bgzf_inflate_device(ctx.handle, d_in.data_ptr(), len(src), *[c.data_ptr() for c in cols],
+                                               len(members), d_out.data_ptr(), at, status.data_ptr(), None), ctx.handle)
+    torch.cuda.synchronize()
+    out = d_out.cpu().numpy()
+    assert (out[:lead] == 7).all() and (out[at:] == 7).all()
+    return status.cpu().numpy(), [out[d:d + n].tobytes() for d, (_, n, _) in zip(do, members)], out, do
+
+
+@pytest.mark.parametrize("lead,gap", [(0, 0), (1, 0), (2, 3), (3, 1)])
+def test_every_block_kind_and_size(ctx, lead, gap):
+    import zlib
+
+    cases = list(_payloads())
+    status, got, out, do = _inflate_raw(ctx, [(p, len(d), zlib.crc32(d)) for _, p, d in cases], lead, gap)
+    for (name, _, data), s, g, at in zip(cases, status, got, do):
+        assert s == 0 and g == data, name
+        assert (out[at + len(data):at + len(data) + gap] == 7).all(), name
+
+
+def test_damaged_members_end_as_on_the_host(ctx, tmp_path_factory):
+    """Truncated, altered and mislabelled members: the status is that of the
+    host-run decoder, or the size or CRC-32 check's."""
+    import zlib
+
+    from test_inflate import _build, inflate
+
+    host = _build(tmp_path_factory, "libinflate_gpu.so", ["-O2"])
+    rng = np.random.default_rng(8)
+    members, want = [], []
+    for name, p, data in _payloads():
+        if len(data) < 100 or len(data) > 65280:
+            continue
+        crc = zlib.crc32(data)
+        made = [(p[:int(rng.integers(0, len(p)))], len(data), crc), (p, len(data) + 1, crc), (p, len(data) - 1, crc),
+                (p, len(data), crc ^ 1)]
+        for _ in range(4):
+            q = bytearray(p)
+            for at in rng.integers(0, len(p) if rng.random() < .5 else min(len(p), 90), int(rng.integers(1, 3))):
+                q[at] ^= 1 << int(rng.integers(0, 8))
+            made.append((bytes(q), len(data), crc))
+        for q, n, c in made:
+            rc, b = inflate(host, q, n)
+            members.append((q, n, c))
+            want.append(rc if rc else 8 if len(b) != n else 0 if zlib.crc32(b) == c else 9)
+    status, _, _, _ = _inflate_raw(ctx, members)
+    np.testing.assert_array_equal(status, want)
