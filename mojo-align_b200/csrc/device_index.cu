@@ -63,15 +63,20 @@ __global__ void relayout_occ_kernel(const uint32_t* __restrict__ bwa, uint64_t s
     OccLine o;
     const unsigned long long* sb = super + (((L * 64) >> super_shift) << 2);
     for (int c = 0; c < 4; ++c) o.cnt[c] = static_cast<uint32_t>(cnt[c] - sb[c]);
+    for (int i = 0; i < 4; ++i) o.w[i] = 0;
     for (int i = 0; i < 4; ++i) {
-        uint64_t p0 = L * 64 + 16 * i;  // first position held by word i
+        uint64_t p0 = L * 64 + 16 * i;  // first position held by bwa's word i
         uint32_t w = 0;
         if (p0 < seq_len) {
             w = rev2(b[8 + 4 * half + i]);
             uint64_t valid = seq_len - p0;
             if (valid < 16) w &= (1u << (2 * valid)) - 1;
         }
-        o.w[i] = w;
+        // 16 symbols to 16 bits of each plane
+        for (int k = 0; k < 16; ++k) {
+            o.w[i >> 1] |= ((w >> (2 * k)) & 1u) << (16 * (i & 1) + k);
+            o.w[2 + (i >> 1)] |= ((w >> (2 * k + 1)) & 1u) << (16 * (i & 1) + k);
+        }
     }
     out[L] = o;
 }

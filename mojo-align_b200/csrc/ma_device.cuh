@@ -6,10 +6,12 @@
 //   occ   one 32-byte line per 64 BWT positions of the stored BWT string
 //         (the sentinel removed, as in bwa): u32 cnt[4] = symbols c in
 //         positions [S, 64*line) where S is the start of the line's
-//         superblock of 2^occ_super_shift positions, then 4 u32 words of
-//         2-bit symbols, 16 per word, least significant first.  An Occ query
-//         is one 32-B sector plus the superblock's count (a table of
-//         4 u64 per superblock, a few entries, cached).
+//         superblock of 2^occ_super_shift positions, then the 64 symbols
+//         as two bit planes: bit p of w[0..1] is the low bit of position p's
+//         symbol, bit p of w[2..3] its high bit, so that the positions of a
+//         symbol are two logic operations per 32.  An Occ query is one 32-B
+//         sector plus the superblock's count (a table of 4 u64 per
+//         superblock, a few entries, cached).
 //   sa    the full suffix array: u32 per row when every row and position
 //         fits 32 bits, else 40-bit values packed three to a 16-byte chunk
 //         (bytes 5*slot .. 5*slot+4 of chunk row/3), one 16-B load either way.
@@ -144,23 +146,23 @@ constexpr uint64_t kEven = 0x5555555555555555ull;
 
 __device__ __forceinline__ uint64_t ldg64(const uint64_t* p) { return __ldg(p); }
 
+// Count of symbol c in positions [64 line, x] of the line (cnt, bw) of x, plus
+// its count before the line.
+__device__ __forceinline__ uint64_t occ_in_line(const DevIndex& ix, const uint4& cnt, const uint4& bw, uint64_t x,
+                                                int c) {
+    const uint32_t base = c == 0 ? cnt.x : c == 1 ? cnt.y : c == 2 ? cnt.z : cnt.w;
+    const uint64_t sb = __ldg(ix.occ_super + ((x >> ix.occ_super_shift) << 2) + c);
+    const uint32_t n0 = (c & 1) ? 0u : ~0u, n1 = (c & 2) ? 0u : ~0u;
+    const uint32_t w = static_cast<uint32_t>(x & 63);
+    const uint32_t upto = (2u << (w & 31)) - 1;  // bits 0 .. w & 31
+    const uint32_t keep_lo = w < 32 ? upto : ~0u, keep_hi = w < 32 ? 0u : upto;
+    return sb + (base + __popc((bw.x ^ n0) & (bw.z ^ n1) & keep_lo) + __popc((bw.y ^ n0) & (bw.w ^ n1) & keep_hi));
+}
+
 // Count of symbol c in stored-BWT positions [0 .. x] (x < seq_len).
 __device__ __forceinline__ uint64_t occ_at(const DevIndex& ix, uint64_t x, int c) {
     const uint4* p = reinterpret_cast<const uint4*>(ix.occ + (x >> 6));
-    uint4 cnt = __ldg(p);
-    uint4 bw = __ldg(p + 1);
-    uint32_t base = c == 0 ? cnt.x : c == 1 ? cnt.y : c == 2 ? cnt.z : cnt.w;
-    const uint64_t sb = __ldg(ix.occ_super + ((x >> ix.occ_super_shift) << 2) + c);
-    uint64_t lo = static_cast<uint64_t>(bw.x) | (static_cast<uint64_t>(bw.y) << 32);
-    uint64_t hi = static_cast<uint64_t>(bw.z) | (static_cast<uint64_t>(bw.w) << 32);
-    uint64_t pat = static_cast<uint64_t>(c) * kEven;
-    uint64_t tl = lo ^ pat, th = hi ^ pat;
-    uint64_t ml = ~(tl | (tl >> 1)) & kEven;
-    uint64_t mh = ~(th | (th >> 1)) & kEven;
-    uint32_t w = static_cast<uint32_t>(x & 63);
-    uint64_t keep_lo = w >= 31 ? ~0ull : ((1ull << (2 * w + 2)) - 1);
-    uint64_t keep_hi = w < 32 ? 0ull : (w >= 63 ? ~0ull : ((1ull << (2 * (w - 32) + 2)) - 1));
-    return sb + static_cast<uint64_t>(base) + __popcll(ml & keep_lo) + __popcll(mh & keep_hi);
+    return occ_in_line(ix, __ldg(p), __ldg(p + 1), x, c);
 }
 
 // Occ(k, c) of the reference: count of c in BWT rows [0..k] (k a row index
@@ -202,8 +204,8 @@ __device__ __forceinline__ bool kmer_interval(uint64_t e, uint64_t& k, uint64_t&
 
 // Symbol of the stored BWT at position x.
 __device__ __forceinline__ int bwt_sym(const OccLine* __restrict__ occ, uint64_t x) {
-    uint32_t w = __ldg(&occ[x >> 6].w[(x >> 4) & 3]);
-    return static_cast<int>((w >> (2 * (x & 15))) & 3);
+    const uint32_t h = static_cast<uint32_t>(x >> 5) & 1, b = static_cast<uint32_t>(x & 31);
+    return static_cast<int>(((__ldg(&occ[x >> 6].w[h]) >> b) & 1) | (((__ldg(&occ[x >> 6].w[2 + h]) >> b) & 1) << 1));
 }
 
 // 32 text bases starting at forward text position p, p in [-512, l_pac+480).

@@ -97,6 +97,33 @@ __device__ __forceinline__ uint32_t compact_even(uint64_t x) {
     return static_cast<uint32_t>(x);
 }
 
+// The base-3 number of K (<= 20) symbols, 2 bits each, first symbol lowest in
+// the word and most significant in the number; a symbol's digit is the number
+// of its bits set (0, 1 or 2).  16 digits are folded pairwise in fields of 4,
+// 8, 16 and 32 bits, the rest one by one.
+__device__ __forceinline__ uint32_t base3_index(uint64_t win, int K) {
+    const uint64_t d = (win & kEven) + ((win >> 1) & kEven);
+    uint32_t idx = 0, rest = static_cast<uint32_t>(d);
+    int i = 0;
+    if (K >= 16) {
+        uint32_t x = rest;
+        x = (x & 0x33333333u) * 3 + ((x >> 2) & 0x33333333u);
+        x = (x & 0x0f0f0f0fu) * 9 + ((x >> 4) & 0x0f0f0f0fu);
+        x = (x & 0x00ff00ffu) * 81 + ((x >> 8) & 0x00ff00ffu);
+        idx = (x & 0xffffu) * 6561 + (x >> 16);
+        rest = static_cast<uint32_t>(d >> 32);
+        i = 16;
+    }
+    for (; i < K; ++i, rest >>= 2) idx = idx * 3 + (rest & 3);
+    return idx;
+}
+
+// The base-4 number of K (<= 14) symbols, first symbol most significant.
+__device__ __forceinline__ uint32_t base4_index(uint64_t win, int K) {
+    const uint32_t r = __brev(static_cast<uint32_t>(win));  // symbols reversed, and the bits of each
+    return (((r >> 1) & 0x55555555u) | ((r & 0x55555555u) << 1)) >> (32 - 2 * K);
+}
+
 // Per-thread traffic tally of the counting kernel variant (S = true).  The
 // timed kernel is the S = false instantiation, where every tally compiles
 // away.
@@ -702,9 +729,7 @@ __device__ __forceinline__ bool search_start(const DevIndex& ix, const ReadView&
         const uint64_t lo = win & kEven, hi = (win >> 1) & kEven;
         const bool has_c = (lo & ~hi) != 0, has_g = (hi & ~lo) != 0;
         if (!(has_c && has_g)) {
-            uint32_t idx = 0;
-            for (int i = 0; i < K3; ++i) idx = idx * 3 + static_cast<uint32_t>(__popcll((win >> (2 * i)) & 3));
-            const uint64_t kl = __ldg(ix.kmer3[has_c ? 1 : 0] + idx);
+            const uint64_t kl = __ldg(ix.kmer3[has_c ? 1 : 0] + base3_index(win, K3));
             if constexpr (S) t.kmer_loads++;
             if (kmer_interval(kl, q.k, q.l)) {
                 have = true;
@@ -716,9 +741,7 @@ __device__ __forceinline__ bool search_start(const DevIndex& ix, const ReadView&
         const int s0 = e - ix.kmer_k + 1;
         if (window_bits(rd.nf, s0, ix.kmer_k) != 0) return false;
         const uint64_t win = window_bits(rd.fwd, s0, ix.kmer_k);
-        uint32_t idx = 0;
-        for (int i = 0; i < ix.kmer_k; ++i) idx = (idx << 2) | static_cast<uint32_t>((win >> (2 * i)) & 3);
-        const uint64_t kl = __ldg(ix.kmer + idx);
+        const uint64_t kl = __ldg(ix.kmer + base4_index(win, ix.kmer_k));
         if constexpr (S) t.kmer_loads++;
         if (kmer_interval(kl, q.k, q.l)) {  // an untabled entry leaves (k, l) = (0, seq_len)
             have = true;
@@ -766,8 +789,27 @@ __device__ __forceinline__ bool search_next(const DevIndex& ix, const ReadView& 
         const int64_t ll = q.l != ix.seq_len ? static_cast<int64_t>((q.l - (q.l >= ix.primary)) >> 6) : -2;
         t.occ_lines += (lk >= 0) + (ll >= 0 && ll != lk);
     }
-    if (q.k != 0) ok = occ_row(ix, q.k - 1, cc);
-    const uint64_t ol = occ_row(ix, q.l, cc);
+    uint64_t ol;
+    if (q.l == ix.seq_len) {
+        if (q.k != 0) ok = occ_row(ix, q.k - 1, cc);
+        ol = ix.L2[cc + 1] - ix.L2[cc];
+    } else {
+        // rows k - 1 and l, mostly of one Occ line once the interval is small
+        const uint64_t x1 = q.l - (q.l >= ix.primary ? 1 : 0);
+        const uint4* p1 = reinterpret_cast<const uint4*>(ix.occ + (x1 >> 6));
+        const uint4 c1 = __ldg(p1), b1 = __ldg(p1 + 1);
+        if (q.k != 0) {
+            const uint64_t x0 = q.k - 1 - (q.k - 1 >= ix.primary ? 1 : 0);
+            uint4 c0 = c1, b0 = b1;
+            if ((x0 >> 6) != (x1 >> 6)) {
+                const uint4* p0 = reinterpret_cast<const uint4*>(ix.occ + (x0 >> 6));
+                c0 = __ldg(p0);
+                b0 = __ldg(p0 + 1);
+            }
+            ok = occ_in_line(ix, c0, b0, x0, cc);
+        }
+        ol = occ_in_line(ix, c1, b1, x1, cc);
+    }
     const uint64_t Lc = ix.L2[cc];
     q.k = Lc + ok + 1;
     q.l = Lc + ol;
