@@ -325,7 +325,6 @@ struct Locus {
     uint64_t uk, ul;
     uint32_t ord_row;
     int32_t us, e, rev;
-    ContigHint hint;
 };
 
 constexpr int S2_WARPS = 8;   // warps per block of the stage-2 kernel
@@ -447,7 +446,6 @@ __global__ void __launch_bounds__(S2_WARPS * 32, MINB) seed_stage2_kernel(DevInd
                     L.us = o_s;
                     L.e = o_e;
                     L.rev = rev;
-                    L.hint = contig_hint(ix, b0);
                     s_loci[rank] = L;
                     if constexpr (S) tally_locus(t, b0, cl.adj_cap, qlen);
                 }
@@ -490,7 +488,7 @@ __global__ void __launch_bounds__(S2_WARPS * 32, MINB) seed_stage2_kernel(DevInd
                         const Locus L = s_loci[own];
                         const uint64_t before = lb.key;
                         eval_adj<S>(ix, rd, L.b0, L.rev, bit - cl.adj_cap, cl.budget, cl.clip_cap, L.ord_row, lb,
-                                    L.uk, L.ul, L.us, L.e, prune, L.hint, t);
+                                    L.uk, L.ul, L.us, L.e, prune, t);
                         if (lb.key != before) lb_tag = L.b0 * 2 + L.rev;
                     }
                 }

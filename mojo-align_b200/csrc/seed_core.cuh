@@ -296,22 +296,6 @@ __device__ __forceinline__ void tally_locus(Tally& t, int64_t b0, int adj_cap, i
     if (hi >= lo) t.pac_sectors += static_cast<uint32_t>(((hi >> 2) >> 5) - ((lo >> 2) >> 5) + 1);
 }
 
-// Contig of a locus, looked up once for all of its shifts.
-struct ContigHint {
-    int64_t crid, coff, clen;
-};
-
-__device__ __forceinline__ ContigHint contig_hint(const DevIndex& ix, int64_t b0) {
-    int64_t probe = b0 < 0 ? 0 : b0;
-    if (probe >= static_cast<int64_t>(ix.l_pac)) probe = static_cast<int64_t>(ix.l_pac) - 1;
-    ContigHint h{contig_of(ix, probe), 0, 0};
-    if (h.crid >= 0) {
-        h.coff = static_cast<int64_t>(__ldg(ix.coff + h.crid));
-        h.clen = static_cast<int64_t>(__ldg(ix.clen + h.crid));
-    }
-    return h;
-}
-
 __device__ __forceinline__ void set_best(Best& best, uint64_t key, int64_t crid, int64_t pos, int sl, int sr,
                                          uint32_t mapq, int flag, uint64_t uk, uint64_t ul, int us, int e) {
     best.key = key;
@@ -387,44 +371,43 @@ __device__ __noinline__ int soft_clip_recount(const uint64_t* __restrict__ pacw,
 // or the deletion probe's offsets) into `best` by its (nm, ordinal) key.
 // prune_nm: a candidate of this call can only matter when its nm is below
 // prune_nm (every candidate of the call comes after the current best in the
-// reference's order); 1 << 20 disables pruning.  `hint` is the contig of
-// b0; a shift that stays inside it needs no contig search.
+// reference's order); 1 << 20 disables pruning.  The contig is searched for
+// only once the core compare, which most shifts fail, has not ruled the shift
+// out: the reference drops a shift whose clips at its contig's ends exceed
+// clip_cap, and a read that overhangs the text by more than that does so on
+// any contig (the text's ends are contig ends), so the compares read at most
+// clip_cap bases past them.
 template <bool S>
 __device__ void eval_adj(const DevIndex& ix, const ReadView& rd, int64_t b0, int is_rev, int adj, int budget,
                          int clip_cap, uint32_t ord_row, Best& best, uint64_t uk, uint64_t ul, int us, int e,
-                         int prune_nm, const ContigHint& hint, Tally& t) {
+                         int prune_nm, Tally& t) {
     if constexpr (S) t.shifts++;
     const int qlen = rd.qlen;
     const uint64_t* q = is_rev ? rd.rc : rd.fwd;
     const uint64_t* qn = is_rev ? rd.nr : rd.nf;
     const int64_t bstart = b0 + adj;
-    int64_t crid = hint.crid, coff = hint.coff, clen = hint.clen;
-    if (crid < 0 || bstart < coff || bstart >= coff + clen) {
-        // the contig holding the clamped probe (binary search, L1536-1549)
-        int64_t probe = bstart < 0 ? 0 : bstart;
-        if (probe >= static_cast<int64_t>(ix.l_pac)) probe = static_cast<int64_t>(ix.l_pac) - 1;
-        crid = contig_of(ix, probe);
-        if (crid < 0) return;
-        coff = static_cast<int64_t>(__ldg(ix.coff + crid));
-        clen = static_cast<int64_t>(__ldg(ix.clen + crid));
-    }
+    if (bstart < -clip_cap || bstart + qlen > static_cast<int64_t>(ix.l_pac) + clip_cap) return;
+    const bool del_probe = adj == 0 && is_rev == 0;
+    // Exact pruning.  sl0, sr0 and every soft clip are at most clip_cap, so
+    // the full compare and any clipped recount both span read positions
+    // [clip_cap, qlen - clip_cap); their mismatches bound nm from below.  A
+    // shift without deletion probe only matters with a core below both the
+    // budget and the best so far: count no further.
+    const int cap = del_probe ? budget + 1 : (prune_nm < budget + 1 ? prune_nm : budget + 1);
+    const int core = count_mm<S>(ix.pacw, q, qn, bstart, clip_cap, qlen - clip_cap, cap, t);
+    if (core >= cap && !(del_probe && prune_nm > 1)) return;
+    // the contig holding the clamped probe (binary search, L1536-1549)
+    int64_t probe = bstart < 0 ? 0 : bstart;
+    if (probe >= static_cast<int64_t>(ix.l_pac)) probe = static_cast<int64_t>(ix.l_pac) - 1;
+    const int64_t crid = contig_of(ix, probe);
+    if (crid < 0) return;
+    const int64_t coff = static_cast<int64_t>(__ldg(ix.coff + crid)), clen = static_cast<int64_t>(__ldg(ix.clen + crid));
     const int64_t local = bstart - coff;
     const int64_t sl0 = local < 0 ? -local : 0;
     const int64_t sr0 = local + qlen > clen ? local + qlen - clen : 0;
     if (!(sl0 + sr0 < qlen && sl0 <= clip_cap && sr0 <= clip_cap)) return;
     const uint32_t ord = (ord_row + static_cast<uint32_t>(adj + 12)) * KIND_SPAN;
-    const bool del_probe = adj == 0 && is_rev == 0;
     const bool del_room = del_probe && prune_nm > 1 && bstart + qlen + 1 <= coff + clen;
-    // Exact pruning.  sl0, sr0 and every soft clip are at most clip_cap, so
-    // the full compare and any clipped recount both span read positions
-    // [clip_cap, qlen - clip_cap); their mismatches bound nm from below.
-    if (!del_probe) {
-        // a shift without deletion probe only matters with a core below
-        // both the budget and the best so far: count no further
-        const int cap = prune_nm < budget + 1 ? prune_nm : budget + 1;
-        if (count_mm<S>(ix.pacw, q, qn, bstart, clip_cap, qlen - clip_cap, cap, t) >= cap) return;
-    }
-    const int core = del_probe ? count_mm<S>(ix.pacw, q, qn, bstart, clip_cap, qlen - clip_cap, budget + 1, t) : 0;
     if (core > budget) {
         // neither compare is accepted: only the deletion probe remains
         if (del_room)
@@ -548,7 +531,6 @@ __device__ void eval_locus(const DevIndex& ix, const ReadView& rd, int64_t b0, i
                            int budget, int clip_cap, uint32_t ord_row, Best& best, uint64_t uk, uint64_t ul,
                            int us, int e, Tally& t) {
     if constexpr (S) tally_locus(t, b0, adj_cap, rd.qlen);
-    const ContigHint hint = contig_hint(ix, b0);
     const uint64_t b_start = best.key >> ORD_SHIFT;
     uint32_t live = live_shifts<S>(ix, rd, b0, is_rev, adj_cap, budget, clip_cap,
                                    b_start < (1u << 20) ? static_cast<int>(b_start) : (1 << 20), t);
@@ -557,7 +539,7 @@ __device__ void eval_locus(const DevIndex& ix, const ReadView& rd, int64_t b0, i
         live &= live - 1;
         const uint64_t bn = best.key >> ORD_SHIFT;
         eval_adj<S>(ix, rd, b0, is_rev, adj, budget, clip_cap, ord_row, best, uk, ul, us, e,
-                    bn < (1u << 20) ? static_cast<int>(bn) : (1 << 20), hint, t);
+                    bn < (1u << 20) ? static_cast<int>(bn) : (1 << 20), t);
     }
 }
 

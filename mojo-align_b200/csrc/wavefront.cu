@@ -1,13 +1,13 @@
-// wavefront.cu - seed_kernels 2, 3 and 4: the seed/extend search as rounds of
+// wavefront.cu - seed_kernels 2 to 4: the seed/extend search as rounds of
 // data-parallel passes over the whole batch (fm_seed_extend_kernel,
 // fq2bam-meth/src/linear_gpu_fm.mojo:1156-1837, with the candidate order
 // and exactness argument of seed_core.cuh).
 //
 // Round k covers right endpoints [resume, resume + width) of every read
 // still active (width w0 in round 0, w after it):
-//   search   one thread per (read, endpoint): duplicate prediction, backward
-//            search, SA rows -> candidate loci appended to a batch-wide
-//            locus list (one atomic per warp);
+//   search   per (read, endpoint): duplicate prediction, backward search, SA
+//            rows -> candidate loci appended to a batch-wide locus list (one
+//            atomic per warp);
 //   eval     one thread per (locus, shift): the shift's candidates (full
 //            compare, soft-clip retry, deletion probe) and an atomicMin of
 //            the best key per read, packed with the locus' list index;
@@ -55,11 +55,9 @@ struct WLocus {
     int64_t b0;
     uint64_t uk;         // first SA row of the seed's interval
     uint32_t read, ord_row;
-    int32_t crid_rev;    // contig * 2 + strand (contig -1: -2 | strand)
+    int32_t rev;         // strand
     uint16_t us;         // seed start
     uint16_t e_dl;       // right endpoint (bits 0-10) | (ul - uk) << 11
-    __device__ int crid() const { return crid_rev >> 1; }
-    __device__ int rev() const { return crid_rev & 1; }
     __device__ int e() const { return e_dl & 0x7FF; }
     __device__ uint64_t ul() const { return uk + (e_dl >> 11); }
 };
@@ -164,131 +162,43 @@ __device__ __forceinline__ bool fresh_locus(const DevIndex& ix, const Wave& w, i
     return true;
 }
 
-// Search: one thread per (active read, endpoint of the round).  The loop
-// is warp-uniform (whole warps step together) for the warp-wide append.
-template <bool S, int MINB>
-__global__ void __launch_bounds__(256, MINB) wf_search_kernel(DevIndex ix, DevReads R, DevParams P, Wave w,
-                                                        const uint32_t* __restrict__ act, int width,
-                                                        unsigned long long* __restrict__ tally_out) {
-    Tally t{};
-    const uint64_t n_items = static_cast<uint64_t>(w.counters[C_ACTIVE]) * static_cast<uint64_t>(width);
-    const int lane = threadIdx.x & 31;
-    const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-    const bool can_predict = ix.summary && ix.kmer3_k > 0 && ix.kmer3_k <= P.seed_len;
-    for (uint64_t base = (blockIdx.x * static_cast<uint64_t>(blockDim.x)) + (threadIdx.x & ~31u); base < n_items;
-         base += stride) {
-        const uint64_t item = base + lane;
-        Seed sd{0, 0, -1, false};
-        int64_t r = 0;
-        int ei = 0, e = 0, qlen = 0, n_memo = 0;
-        ReadView rd{};
-        if (item < n_items) {
-            const uint64_t a = item < (1ull << 32) ? static_cast<uint32_t>(item) / static_cast<uint32_t>(width)
-                                                   : item / static_cast<uint64_t>(width);
-            const int j = static_cast<int>(item - a * static_cast<uint64_t>(width));
-            r = act[a];
-            rd = read_view(R, r);
-            qlen = rd.qlen;
-            ei = static_cast<int>(w.resume[r]) + j;
-            if (ei < endpoint_count(P, qlen)) {
-                e = P.seed_len - 1 + ei * P.seed_stride;
-                n_memo = w.memo_n[r];
-                // a read with no hit yet gains little from predicting its
-                // rejected loci again: only reads with a best try the memo
-                const int64_t best_tag = w.best_tag[r];
-                const bool dup = can_predict && best_tag != -1 &&
-                                 predicted_duplicate<S>(ix, rd, e, P, best_tag, w.memo + r * MEMO1,
-                                                        n_memo < PREDICT_MEMO ? n_memo : PREDICT_MEMO, t);
-                if constexpr (S) t.skipped += dup;
-                if (!dup) sd = search_endpoint<S>(ix, rd, e, P, t);
-            }
-        }
-        // every SA row takes a list slot (one atomic per warp); rows that
-        // give no new locus leave their slot dead
-        const uint32_t n_rows = sd.found ? static_cast<uint32_t>(sd.l - sd.k + 1) : 0u;
-        uint32_t incl = n_rows;
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-            if (lane >= o) incl += v;
-        }
-        const uint32_t warp_total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-        unsigned long long wbase = 0;
-        if (lane == 31 && warp_total) wbase = atomicAdd(loci_count(w), static_cast<unsigned long long>(warp_total));
-        wbase = __shfl_sync(0xFFFFFFFFu, wbase, 31);
-        // the warp's rows, 32 at a time, one per lane (seeds have 1..16 rows)
-        for (uint32_t c0 = 0; c0 < warp_total; c0 += 32) {
-            const uint32_t idx = c0 + lane;
-            int owner = 0;  // first lane whose inclusive row count exceeds idx
-            for (int step = 16; step >= 1; step >>= 1) {
-                const uint32_t v = __shfl_sync(0xFFFFFFFFu, incl, owner + step - 1);
-                if (v <= idx) owner += step;
-            }
-            const int own = owner < 32 ? owner : 31;
-            const uint64_t o_k = __shfl_sync(0xFFFFFFFFu, sd.k, own);
-            const uint64_t o_l = __shfl_sync(0xFFFFFFFFu, sd.l, own);
-            const int o_s = __shfl_sync(0xFFFFFFFFu, sd.s, own);
-            const int o_e = __shfl_sync(0xFFFFFFFFu, e, own);
-            const int o_ei = __shfl_sync(0xFFFFFFFFu, ei, own);
-            const int o_qlen = __shfl_sync(0xFFFFFFFFu, qlen, own);
-            const int o_memo = __shfl_sync(0xFFFFFFFFu, n_memo, own);
-            const int64_t o_r = __shfl_sync(0xFFFFFFFFu, r, own);
-            const uint32_t o_first = __shfl_sync(0xFFFFFFFFu, incl - n_rows, own);
-            if (idx >= warp_total) continue;
-            const uint64_t hi = o_k + (idx - o_first);
-            const uint64_t slot = static_cast<uint64_t>(wbase) + idx;
-            if (slot >= w.locus_cap) {
-                w.overflow[o_r] = 1;
-                continue;
-            }
-            const uint64_t sa_pos = sa_at(ix, hi);
-            if constexpr (S) t.sa_loads++;
-            WLocus L;
-            int64_t b0;
-            int rev;
-            if (!fresh_locus(ix, w, o_r, o_memo, sa_pos, o_s, o_e, o_qlen, b0, rev)) {
-                L.read = DEAD_LOCUS;
-                w.loci[slot] = L;
-                continue;
-            }
-            L.b0 = b0;
-            L.uk = o_k;
-            L.read = static_cast<uint32_t>(o_r);
-            L.ord_row = (static_cast<uint32_t>(o_ei) * 16 + static_cast<uint32_t>(hi - o_k)) * ADJ_SPAN;
-            L.us = static_cast<uint16_t>(o_s);
-            L.e_dl = static_cast<uint16_t>(o_e | ((o_l - o_k) << 11));
-            L.crid_rev = static_cast<int32_t>(contig_hint(ix, b0).crid) * 2 + rev;
-            w.loci[slot] = L;
-            if constexpr (S) tally_locus(t, b0, clamps_for(P, o_qlen).adj_cap, o_qlen);
-            const uint32_t m = atomicAdd(&w.memo_next[o_r], 1u);
-            if (m < static_cast<uint32_t>(MEMO1)) w.memo[o_r * MEMO1 + m] = static_cast<uint64_t>(b0 * 2 + rev);
-        }
-    }
-    flush_tally<S>(t, tally_out);
-}
-
-// Search with lane refill (seed_kernel 3): the same items as
-// wf_search_kernel, but each lane steps its own endpoint's search and takes
-// a new item when its search ends.  Search lengths differ by two orders of
-// magnitude (a table hit ends at once; a seed in a repeat steps back to the
-// read's start), so a warp that waits for its longest lane runs most steps
-// with few lanes busy.  Here the warp alternates two passes:
-//   refill  when at least REFILL_MIN lanes are idle (or all are), the idle
-//           lanes take the next items of the warp's chunk sequence and run
-//           the duplicate prediction and the table steps;
-//   step    the busy lanes take one backward step each.
-// Seeds found are staged in shared memory and appended to the locus list at
-// least 32 rows at a time (one atomic per flush, one lane per row), as in
-// wf_search_kernel.  Which lane or pass finds a seed does not change the
-// round's result: the eval keys carry the candidate order.
-constexpr int REFILL_MIN = 16;    // idle lanes that trigger a refill pass
-constexpr int REFILL_STAGE = 64;  // staged seeds per warp (flushed above 32)
+// Search: the round's items are (active read, endpoint) pairs.  Most end at
+// their table lookup, the others step back one base at a time for anything
+// from one to a hundred steps, and each seed found has 1 to 16 rows: a thread
+// that took an item through all three would leave most of its warp waiting
+// (12.6 lanes of 32 active per instruction).  So each warp keeps two lists in
+// shared memory and every pass runs with its lanes full:
+//   lookup  32 items, one per lane: duplicate prediction and the table steps;
+//           searches that go on are pushed on the warp's list of searches;
+//   step    32 searches from that list, one per lane, one backward step at a
+//           time; a lane whose search ends takes the next one.  With the list
+//           empty, items left and fewer than STEP_MIN lanes busy, the busy
+//           ones are put back until further lookups have filled the list;
+//   rows    the SA rows of the seeds found, one per lane, once more than
+//           SEED_STAGE - 32 seeds wait (or nothing else is left): one list
+//           slot per row (one atomic per pass); rows that give no new locus
+//           leave their slot dead.
+// Which pass finds a seed does not change the round's result: the eval keys
+// carry the candidate order.
+// 2 M uneven reads on 250 Mbp (62 M lookups, 56 M steps, 103 M rows): 8.8 ms,
+// 10.1 ms with a thread per item through all three; 800 k reads of 250 bases
+// 2.05 and 2.7 ms.  Bound by the latency of the gathers.
 constexpr int SEARCH_WARPS = 8;   // 256 threads
+constexpr int SEARCH_LIST = 64;   // searches under way per warp
+constexpr int SEED_STAGE = 64;    // seeds waiting per warp
+constexpr int STEP_MIN = 20;
 
-struct StagedSeed {  // 24 bytes
-    uint64_t k;
-    uint32_t read, rows_end;  // rows_end: staged rows up to and including this seed
-    uint16_t s, e, ei, qlen;
+struct SearchLists {
+    // a search: k | s << 35 | e << 45, rows - 1 | last << 35 (SeedSearch's, plus one),
+    // last_k | endpoint index << 35, read
+    uint64_t a[SEARCH_LIST], b[SEARCH_LIST], c[SEARCH_LIST];
+    uint32_t read[SEARCH_LIST];
+    // a seed: its first row, read, staged rows up to and including it, then
+    // start | right endpoint << 16 and endpoint index | read length << 16
+    uint64_t seed_k[SEED_STAGE];
+    uint32_t seed_read[SEED_STAGE], rows_end[SEED_STAGE], s_e[SEED_STAGE], ei_len[SEED_STAGE];
 };
+static_assert(SEARCH_WARPS * sizeof(SearchLists) <= 32768, "six blocks per SM leave room for the L1 cache");
 
 // Words of read r for the backward steps (qlen is not needed there).
 __device__ __forceinline__ ReadView step_view(const DevReads& R, uint32_t r) {
@@ -303,157 +213,188 @@ __device__ __forceinline__ ReadView step_view(const DevReads& R, uint32_t r) {
 }
 
 template <bool S, int MINB>
-__global__ void __launch_bounds__(256, MINB) wf_search_refill_kernel(DevIndex ix, DevReads R, DevParams P, Wave w,
-                                                               const uint32_t* __restrict__ act, int width,
-                                                               unsigned long long* __restrict__ tally_out) {
-    __shared__ StagedSeed s_stage[SEARCH_WARPS][REFILL_STAGE];
+__global__ void __launch_bounds__(256, MINB) wf_search_kernel(DevIndex ix, DevReads R, DevParams P, Wave w,
+                                                        const uint32_t* __restrict__ act, int width,
+                                                        unsigned long long* __restrict__ tally_out) {
+    __shared__ SearchLists s_lists[SEARCH_WARPS];
     constexpr unsigned FULL = 0xFFFFFFFFu;
+    constexpr uint64_t MASK35 = (1ull << 35) - 1;
     Tally t{};
     const uint64_t n_items = static_cast<uint64_t>(w.counters[C_ACTIVE]) * static_cast<uint64_t>(width);
     const int lane = threadIdx.x & 31;
     const unsigned lt_mask = (1u << lane) - 1;
-    const uint64_t n_warps = static_cast<uint64_t>(gridDim.x) * SEARCH_WARPS;
     const bool can_predict = ix.summary && ix.kmer3_k > 0 && ix.kmer3_k <= P.seed_len;
-    StagedSeed* stage = s_stage[threadIdx.x >> 5];
-    // the warp's items: chunks of 32 items, warp g takes chunks g, g + n_warps, ...
-    uint64_t chunk = static_cast<uint64_t>(blockIdx.x) * SEARCH_WARPS + (threadIdx.x >> 5);
-    uint32_t off = 0;          // items of the chunk handed out
-    int n_staged = 0;          // warp-uniform
-    uint32_t staged_rows = 0;  // warp-uniform
-    // the lane's search
-    bool busy = false;
-    SeedSearch q;
-    uint32_t r = 0;
-    int e_ei = 0;  // right endpoint | endpoint index << 16
+    SearchLists& q = s_lists[threadIdx.x >> 5];
+    // the warp's items: 32 at a time, warp g takes groups g, g + n_warps, ...
+    const uint64_t group_stride = static_cast<uint64_t>(gridDim.x) * (SEARCH_WARPS * 32);
+    uint64_t base = (static_cast<uint64_t>(blockIdx.x) * SEARCH_WARPS + (threadIdx.x >> 5)) * 32;
+    int n_search = 0, n_seeds = 0;  // entries of the lists (warp-uniform)
+    uint32_t n_rows = 0;
+    // pushes the seeds of the lanes that found one
+    auto push_seeds = [&](const Seed& sd, uint32_t r, int e, int ei) {
+        const unsigned fb = __ballot_sync(FULL, sd.found);
+        if (!fb) return;
+        const uint32_t rows = sd.found ? static_cast<uint32_t>(sd.l - sd.k + 1) : 0u;
+        uint32_t incl = rows;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(FULL, incl, o);
+            if (lane >= o) incl += v;
+        }
+        if (sd.found) {
+            const int i = n_seeds + __popc(fb & lt_mask);
+            q.seed_k[i] = sd.k;
+            q.seed_read[i] = r;
+            q.rows_end[i] = n_rows + incl;
+            q.s_e[i] = static_cast<uint32_t>(sd.s) | static_cast<uint32_t>(e) << 16;
+            q.ei_len[i] = static_cast<uint32_t>(ei) | __ldg(R.lens + r) << 16;
+        }
+        n_seeds += __popc(fb);
+        n_rows += __shfl_sync(FULL, incl, 31);
+    };
+    // pushes the searches of the lanes that are `on`
+    auto push_search = [&](bool on, const SeedSearch& c, uint32_t r, int e, int ei) {
+        const unsigned ob = __ballot_sync(FULL, on);
+        if (on) {
+            const int i = n_search + __popc(ob & lt_mask);
+            q.a[i] = c.k | static_cast<uint64_t>(c.s) << 35 | static_cast<uint64_t>(e) << 45;
+            q.b[i] = (c.l - c.k) | static_cast<uint64_t>(c.last + 1) << 35;
+            q.c[i] = c.last_k | static_cast<uint64_t>(ei) << 35;
+            q.read[i] = r;
+        }
+        n_search += __popc(ob);
+    };
     for (;;) {
-        const unsigned idle = __ballot_sync(FULL, !busy);
-        const uint64_t cur = chunk * 32 + off;
-        const bool more = off < 32 && cur < n_items;
-        if (!more && idle == FULL && n_staged == 0) break;
-        bool fin = false;  // this lane's search ended in this pass
-        Seed sd{0, 0, -1, false};
-        if (more && (__popc(idle) >= REFILL_MIN || idle == FULL)) {
-            const uint64_t left = min(static_cast<uint64_t>(32 - off), n_items - cur);
-            const unsigned take = min(static_cast<uint64_t>(__popc(idle)), left);
-            const unsigned rank = __popc(idle & lt_mask);
-            if (!busy && rank < take) {
-                const uint64_t item = cur + rank;
+        const bool more = base < n_items;
+        const bool look = more && n_search <= SEARCH_LIST - 32;
+        if (n_seeds > SEED_STAGE - 32 || (!more && n_search == 0)) {
+            // ---- rows ----
+            if (n_seeds == 0) break;
+            __syncwarp();
+            unsigned long long wbase = 0;
+            if (lane == 0) wbase = atomicAdd(loci_count(w), static_cast<unsigned long long>(n_rows));
+            wbase = __shfl_sync(FULL, wbase, 0);
+            for (uint32_t idx = lane; idx < n_rows; idx += 32) {
+                int lo = 0, hi = n_seeds - 1;  // first seed whose rows_end exceeds idx
+                while (lo < hi) {
+                    const int mid = (lo + hi) >> 1;
+                    if (q.rows_end[mid] > idx) hi = mid;
+                    else lo = mid + 1;
+                }
+                const uint32_t first = lo ? q.rows_end[lo - 1] : 0u;
+                const uint32_t r = q.seed_read[lo];
+                const uint64_t slot = static_cast<uint64_t>(wbase) + idx;
+                if (slot >= w.locus_cap) {
+                    w.overflow[r] = 1;
+                    continue;
+                }
+                const uint64_t k = q.seed_k[lo], sa_pos = sa_at(ix, k + (idx - first));
+                if constexpr (S) t.sa_loads++;
+                const uint32_t s_e = q.s_e[lo], ei_len = q.ei_len[lo];
+                const int s = static_cast<int>(s_e & 0xFFFF), e = static_cast<int>(s_e >> 16);
+                const int qlen = static_cast<int>(ei_len >> 16);
+                WLocus L;
+                int64_t b0;
+                int rev;
+                if (!fresh_locus(ix, w, r, w.memo_n[r], sa_pos, s, e, qlen, b0, rev)) {
+                    w.loci[slot].read = DEAD_LOCUS;
+                    continue;
+                }
+                L.b0 = b0;
+                L.uk = k;
+                L.read = r;
+                L.ord_row = ((ei_len & 0xFFFF) * 16 + (idx - first)) * ADJ_SPAN;
+                L.us = static_cast<uint16_t>(s);
+                L.e_dl = static_cast<uint16_t>(e | ((q.rows_end[lo] - first - 1) << 11));
+                L.rev = rev;
+                w.loci[slot] = L;
+                if constexpr (S) tally_locus(t, b0, clamps_for(P, qlen).adj_cap, qlen);
+                const uint32_t m = atomicAdd(&w.memo_next[r], 1u);
+                if (m < static_cast<uint32_t>(MEMO1)) w.memo[static_cast<uint64_t>(r) * MEMO1 + m] = static_cast<uint64_t>(b0 * 2 + rev);
+            }
+            __syncwarp();
+            n_seeds = 0;
+            n_rows = 0;
+        } else if (look) {
+            // ---- lookup ----
+            const uint64_t item = base + lane;
+            base += group_stride;
+            Seed sd{0, 0, -1, false};
+            SeedSearch c{};
+            bool go_on = false;
+            uint32_t r = 0;
+            int ei = 0, e = 0;
+            if (item < n_items) {
                 const uint64_t a = item < (1ull << 32) ? static_cast<uint32_t>(item) / static_cast<uint32_t>(width)
                                                        : item / static_cast<uint64_t>(width);
                 const int j = static_cast<int>(item - a * static_cast<uint64_t>(width));
                 r = act[a];
                 const ReadView rd = read_view(R, r);
-                const int ei = static_cast<int>(w.resume[r]) + j;
-                fin = true;
+                ei = static_cast<int>(w.resume[r]) + j;
                 if (ei < endpoint_count(P, rd.qlen)) {
-                    const int e = P.seed_len - 1 + ei * P.seed_stride;
-                    e_ei = e | ei << 16;
-                    const int n_memo = w.memo_n[r];
+                    e = P.seed_len - 1 + ei * P.seed_stride;
+                    // a read with no hit yet gains little from predicting its
+                    // rejected loci again: only reads with a best try the memo
                     const int64_t best_tag = w.best_tag[r];
-                    const bool dup = can_predict && best_tag != -1 &&
-                                     predicted_duplicate<S>(ix, rd, e, P, best_tag, w.memo + r * MEMO1,
-                                                            n_memo < PREDICT_MEMO ? n_memo : PREDICT_MEMO, t);
-                    if constexpr (S) t.skipped += dup;
-                    if (!dup) {
-                        busy = search_start<S>(ix, rd, e, P, q, sd, t);
-                        fin = !busy;
+                    bool dup = false;
+                    if (can_predict && best_tag != -1) {
+                        const int n_memo = w.memo_n[r];
+                        dup = predicted_duplicate<S>(ix, rd, e, P, best_tag, w.memo + static_cast<uint64_t>(r) * MEMO1,
+                                                     n_memo < PREDICT_MEMO ? n_memo : PREDICT_MEMO, t);
                     }
+                    if constexpr (S) t.skipped += dup;
+                    if (!dup) go_on = search_start<S>(ix, rd, e, P, c, sd, t);
                 }
             }
-            off += take;
-            if (off >= 32 || chunk * 32 + off >= n_items) {  // the warp's next chunk
-                chunk += n_warps;
-                off = 0;
+            push_search(go_on, c, r, e, ei);
+            push_seeds(sd, r, e, ei);
+            __syncwarp();
+        } else {
+            // ---- step ----
+            bool busy = false;
+            SeedSearch c{};
+            uint32_t r = 0;
+            int ei = 0, e = 0;
+            for (;;) {
+                // idle lanes take searches from the end of the list
+                const unsigned idle = __ballot_sync(FULL, !busy);
+                const int rank = __popc(idle & lt_mask);
+                if (!busy && rank < n_search) {
+                    const int i = n_search - 1 - rank;
+                    const uint64_t a = q.a[i], b = q.b[i], d = q.c[i];
+                    c.k = a & MASK35;
+                    c.l = c.k + (b & MASK35);
+                    c.last_k = d & MASK35;
+                    c.s = static_cast<int>(a >> 35) & 0x3FF;
+                    c.last = static_cast<int>(b >> 35) - 1;
+                    e = static_cast<int>(a >> 45);
+                    ei = static_cast<int>(d >> 35);
+                    r = q.read[i];
+                    busy = true;
+                }
+                n_search -= min(n_search, __popc(idle));
+                const int n_busy = __popc(__ballot_sync(FULL, busy));
+                if (n_busy == 0) break;
+                if (n_seeds > SEED_STAGE - 32 || (n_search == 0 && more && n_busy < STEP_MIN)) {
+                    __syncwarp();
+                    push_search(busy, c, r, e, ei);
+                    break;
+                }
+                Seed sd{0, 0, -1, false};
+                if (busy) busy = search_next<S>(ix, step_view(R, r), e, P, c, sd, t);
+                push_seeds(sd, r, e, ei);
             }
-        } else if (busy) {
-            busy = search_next<S>(ix, step_view(R, r), e_ei & 0xFFFF, P, q, sd, t);
-            fin = !busy;
+            __syncwarp();
         }
-        // stage the seeds found in this pass (at most 32: n_staged <= 32 here)
-        const bool found = fin && sd.found;
-        const unsigned fb = __ballot_sync(FULL, found);
-        if (fb) {
-            const uint32_t n_rows = found ? static_cast<uint32_t>(sd.l - sd.k + 1) : 0u;
-            uint32_t incl = n_rows;
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t v = __shfl_up_sync(FULL, incl, o);
-                if (lane >= o) incl += v;
-            }
-            if (found) {
-                StagedSeed g;
-                g.k = sd.k;
-                g.read = r;
-                g.rows_end = staged_rows + incl;
-                g.s = static_cast<uint16_t>(sd.s);
-                g.e = static_cast<uint16_t>(e_ei & 0xFFFF);
-                g.ei = static_cast<uint16_t>(e_ei >> 16);
-                g.qlen = static_cast<uint16_t>(__ldg(R.lens + r));
-                stage[n_staged + __popc(fb & lt_mask)] = g;
-            }
-            n_staged += __popc(fb);
-            staged_rows += __shfl_sync(FULL, incl, 31);
-        }
-        if (n_staged == 0) continue;
-        if (staged_rows < 32 && n_staged <= REFILL_STAGE - 32) {
-            // keep staging unless the warp's items are all searched
-            const bool out_of_items = off >= 32 || chunk * 32 + off >= n_items;
-            if (!out_of_items || __ballot_sync(FULL, busy)) continue;
-        }
-        // flush: one list slot per staged row, 32 rows at a time
-        __syncwarp();
-        unsigned long long wbase = 0;
-        if (lane == 0) wbase = atomicAdd(loci_count(w), static_cast<unsigned long long>(staged_rows));
-        wbase = __shfl_sync(FULL, wbase, 0);
-        for (uint32_t idx = lane; idx < staged_rows; idx += 32) {
-            int lo = 0, hi = n_staged - 1;  // first staged seed whose rows_end exceeds idx
-            while (lo < hi) {
-                const int mid = (lo + hi) >> 1;
-                if (stage[mid].rows_end > idx) hi = mid;
-                else lo = mid + 1;
-            }
-            const StagedSeed g = stage[lo];
-            const uint32_t first = lo ? stage[lo - 1].rows_end : 0u;
-            const uint64_t row = g.k + (idx - first);
-            const int64_t o_r = g.read;
-            const uint64_t slot = static_cast<uint64_t>(wbase) + idx;
-            if (slot >= w.locus_cap) {
-                w.overflow[o_r] = 1;
-                continue;
-            }
-            const uint64_t sa_pos = sa_at(ix, row);
-            if constexpr (S) t.sa_loads++;
-            WLocus L;
-            int64_t b0;
-            int rev;
-            if (!fresh_locus(ix, w, o_r, w.memo_n[o_r], sa_pos, g.s, g.e, g.qlen, b0, rev)) {
-                L.read = DEAD_LOCUS;
-                w.loci[slot] = L;
-                continue;
-            }
-            L.b0 = b0;
-            L.uk = g.k;
-            L.read = g.read;
-            L.ord_row = (static_cast<uint32_t>(g.ei) * 16 + (idx - first)) * ADJ_SPAN;
-            L.us = g.s;
-            L.e_dl = static_cast<uint16_t>(g.e | ((g.rows_end - first - 1) << 11));
-            L.crid_rev = static_cast<int32_t>(contig_hint(ix, b0).crid) * 2 + rev;
-            w.loci[slot] = L;
-            if constexpr (S) tally_locus(t, b0, clamps_for(P, g.qlen).adj_cap, g.qlen);
-            const uint32_t m = atomicAdd(&w.memo_next[o_r], 1u);
-            if (m < static_cast<uint32_t>(MEMO1)) w.memo[o_r * MEMO1 + m] = static_cast<uint64_t>(b0 * 2 + rev);
-        }
-        __syncwarp();
-        n_staged = 0;
-        staged_rows = 0;
     }
     flush_tally<S>(t, tally_out);
 }
 
-// Eval: one thread per locus filters its shifts (live_shifts); the shifts
-// left in the warp are spread over its lanes.  Candidates are pruned
-// against the read's best from earlier rounds; the round's minimum key per
-// read is an atomicMin of (nm, ordinal, locus index) packed in 64 bits.  The
-// loop over loci is warp-uniform for the redistribution.
+// Eval: one thread per locus filters its shifts (live_shifts); the live
+// shifts (a fraction of a shift per locus at genome scale) are staged per warp
+// in shared memory and evaluated 32 at a time, so the full compares run with
+// every lane busy.  Candidates are pruned against the read's best from earlier
+// rounds; the round's minimum key per read is an atomicMin of (nm, ordinal,
+// locus index) packed in 64 bits.
 constexpr int EVAL_THREADS = 256;
 
 // One shift (adj) of the locus at list index li: its candidates, pruned
@@ -467,17 +408,11 @@ __device__ __forceinline__ void eval_shift(const DevIndex& ix, const DevReads& R
     const Clamps cl = clamps_for(P, rd.qlen);
     const uint64_t bn = w.best_key[r] >> ORD_SHIFT;
     const int prune = bn < (1u << 20) ? static_cast<int>(bn) : (1 << 20);
-    const int crid = L.crid();
-    ContigHint hint{crid, 0, 0};
-    if (crid >= 0) {
-        hint.coff = static_cast<int64_t>(__ldg(ix.coff + crid));
-        hint.clen = static_cast<int64_t>(__ldg(ix.clen + crid));
-    }
     Best lb;
     lb.key = ~0ull;
     lb.crid = -1;
-    eval_adj<S>(ix, rd, L.b0, L.rev(), adj, cl.budget, cl.clip_cap, L.ord_row, lb, L.uk, L.ul(), L.us, L.e(), prune,
-                hint, t);
+    eval_adj<S>(ix, rd, L.b0, L.rev, adj, cl.budget, cl.clip_cap, L.ord_row, lb, L.uk, L.ul(), L.us, L.e(), prune,
+                t);
     if (lb.key != ~0ull) {
         const uint64_t nm = lb.key >> ORD_SHIFT;
         const uint64_t ord = lb.key & ((1ull << ORD_SHIFT) - 1);
@@ -486,69 +421,10 @@ __device__ __forceinline__ void eval_shift(const DevIndex& ix, const DevReads& R
     }
 }
 
-template <bool S, int MINB>
-__global__ void __launch_bounds__(EVAL_THREADS, MINB) wf_eval_kernel(DevIndex ix, DevReads R, DevParams P, Wave w,
-                                                               unsigned long long* __restrict__ tally_out) {
-    __shared__ WLocus s_loci[EVAL_THREADS];
-    constexpr unsigned FULL = 0xFFFFFFFFu;
-    Tally t{};
-    uint64_t n_loci = *loci_count(w);
-    if (n_loci > w.locus_cap) n_loci = w.locus_cap;
-    const int adj_cap = clamps_for(P, 1 << 20).adj_cap;  // read-independent
-    const int lane = threadIdx.x & 31;
-    WLocus* wl = s_loci + (threadIdx.x & ~31u);
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < n_loci; base += stride) {
-        const uint32_t li = base + lane;
-        uint32_t live = 0;
-        if (li < n_loci) {
-            const WLocus L = w.loci[li];
-            wl[lane] = L;
-            const int64_t r = L.read;
-            if (L.read != DEAD_LOCUS && !w.overflow[r]) {
-                const ReadView rd = read_view(R, r);
-                const Clamps cl = clamps_for(P, rd.qlen);
-                const uint64_t bn = w.best_key[r] >> ORD_SHIFT;
-                const int prune = bn < (1u << 20) ? static_cast<int>(bn) : (1 << 20);
-                live = live_shifts<S>(ix, rd, L.b0, L.rev(), adj_cap, cl.budget, cl.clip_cap, prune, t);
-            }
-        }
-        __syncwarp();
-        const int n_live = __popc(live);
-        int incl = n_live;
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(FULL, incl, o);
-            if (lane >= o) incl += v;
-        }
-        const int total = __shfl_sync(FULL, incl, 31);
-        for (int c = 0; c < total; c += 32) {
-            const int idx = c + lane;
-            int owner = 0;  // first lane whose inclusive count exceeds idx
-            for (int step = 16; step >= 1; step >>= 1) {
-                const int v = __shfl_sync(FULL, incl, owner + step - 1);
-                if (v <= idx) owner += step;
-            }
-            const int own = owner < 32 ? owner : 31;
-            const uint32_t o_live = __shfl_sync(FULL, live, own);
-            const int o_first = __shfl_sync(FULL, incl - n_live, own);
-            if (idx < total) {
-                const int adj = static_cast<int>(__fns(o_live, 0, idx - o_first + 1)) - adj_cap;
-                eval_shift<S>(ix, R, P, w, wl[own], base + own, adj, t);
-            }
-        }
-        __syncwarp();
-    }
-    flush_tally<S>(t, tally_out);
-}
-
-// Eval with staged shifts (seed_kernels 3 and 4): the filter pass as in
-// wf_eval_kernel, but the live shifts (a fraction of a shift per locus at
-// genome scale) are staged per warp in shared memory and evaluated 32 at a
-// time, so the full compares run with every lane busy.
 constexpr int SHIFT_STAGE = 64;  // staged shifts per warp: locus index << 5 | shift
 
 template <bool S, int MINB>
-__global__ void __launch_bounds__(EVAL_THREADS, MINB) wf_eval_staged_kernel(DevIndex ix, DevReads R, DevParams P,
+__global__ void __launch_bounds__(EVAL_THREADS, MINB) wf_eval_kernel(DevIndex ix, DevReads R, DevParams P,
                                                                       Wave w,
                                                                       unsigned long long* __restrict__ tally_out) {
     __shared__ uint64_t s_shift[EVAL_THREADS / 32][SHIFT_STAGE];
@@ -574,7 +450,7 @@ __global__ void __launch_bounds__(EVAL_THREADS, MINB) wf_eval_staged_kernel(DevI
                 const Clamps cl = clamps_for(P, rd.qlen);
                 const uint64_t bn = w.best_key[r] >> ORD_SHIFT;
                 const int prune = bn < (1u << 20) ? static_cast<int>(bn) : (1 << 20);
-                rem = live_shifts<S>(ix, rd, L.b0, L.rev(), adj_cap, cl.budget, cl.clip_cap, prune, t);
+                rem = live_shifts<S>(ix, rd, L.b0, L.rev, adj_cap, cl.budget, cl.clip_cap, prune, t);
             }
         }
         for (;;) {
@@ -661,23 +537,17 @@ __global__ void __launch_bounds__(256) wf_finalize_kernel(DevIndex ix, DevReads 
                     const int adj = static_cast<int>(ord / KIND_SPAN) - static_cast<int>(L.ord_row) - 12;
                     const uint64_t bn = old >> ORD_SHIFT;
                     const int prune = bn < (1u << 20) ? static_cast<int>(bn) : (1 << 20);
-                    const int crid = L.crid();
-                    ContigHint hint{crid, 0, 0};
-                    if (crid >= 0) {
-                        hint.coff = static_cast<int64_t>(__ldg(ix.coff + crid));
-                        hint.clen = static_cast<int64_t>(__ldg(ix.clen + crid));
-                    }
                     Best lb;
                     lb.key = ~0ull;
                     lb.crid = -1;
-                    eval_adj<S>(ix, rd, L.b0, L.rev(), adj, cl.budget, cl.clip_cap, L.ord_row, lb, L.uk, L.ul(),
-                                L.us, L.e(), prune, hint, t);
+                    eval_adj<S>(ix, rd, L.b0, L.rev, adj, cl.budget, cl.clip_cap, L.ord_row, lb, L.uk, L.ul(),
+                                L.us, L.e(), prune, t);
                     if (lb.key != rkey) {
                         atomicExch(err, 3);  // the recomputed candidate must be the round's minimum
                     } else {
                         write_hit(out, r, lb, qlen);
                         w.best_key[r] = lb.key;
-                        w.best_tag[r] = L.b0 * 2 + L.rev();
+                        w.best_tag[r] = L.b0 * 2 + L.rev;
                         const uint64_t nm = lb.key >> ORD_SHIFT;
                         if (nm == 0) {
                             stop = true;
@@ -729,10 +599,9 @@ int grid_blocks(K kernel, int sm_count) {
 
 // Register budget of the search / eval kernels (result-neutral): blocks of
 // 256 threads asked per SM (1 = the compiler's choice).
-template <bool S, int MS, int ME, int MR>
+template <bool S, int MS, int ME>
 int launch_rounds(const DevIndex& ix, const DevReads& R, const DevParams& P, const DevOut& out, const Wave& w,
-                  int max_len, int w0, int wn, int max_rounds, int growth, bool refill, bool staged, int sm_count,
-                  int* d_err,
+                  int max_len, int w0, int wn, int max_rounds, int growth, int sm_count, int* d_err,
                   unsigned long long* tally, WaveTimer* timer, cudaStream_t st) {
     const int n_end_max = endpoint_count_host(P, max_len);
     // round widths: w0, then wn (doubling from the third round with growth)
@@ -746,9 +615,7 @@ int launch_rounds(const DevIndex& ix, const DevReads& R, const DevParams& P, con
     }
     if (max_rounds > 0 && rounds > max_rounds) rounds = max_rounds;
     static const int g_search = grid_blocks(wf_search_kernel<S, MS>, sm_count);
-    static const int g_refill = grid_blocks(wf_search_refill_kernel<S, MR>, sm_count);
     static const int g_eval = grid_blocks(wf_eval_kernel<S, ME>, sm_count);  // EVAL_THREADS = 256
-    static const int g_eval_staged = grid_blocks(wf_eval_staged_kernel<S, ME>, sm_count);
     static const int g_fin = grid_blocks(wf_finalize_kernel<S>, sm_count);
     const unsigned init_blocks = static_cast<unsigned>((R.n_seq + 255) / 256);
     wf_init_kernel<<<init_blocks ? init_blocks : 1, 256, 0, st>>>(w, out, R.lens, R.n_seq);
@@ -763,11 +630,9 @@ int launch_rounds(const DevIndex& ix, const DevReads& R, const DevParams& P, con
         }
         const bool timed = timer && k < WaveTimer::MAX_ROUNDS;
         if (timed) cudaEventRecord(timer->e[3 * k], st);
-        if (refill) wf_search_refill_kernel<S, MR><<<g_refill, 256, 0, st>>>(ix, R, P, w, act, width, tally);
-        else wf_search_kernel<S, MS><<<g_search, 256, 0, st>>>(ix, R, P, w, act, width, tally);
+        wf_search_kernel<S, MS><<<g_search, 256, 0, st>>>(ix, R, P, w, act, width, tally);
         if (timed) cudaEventRecord(timer->e[3 * k + 1], st);
-        if (staged) wf_eval_staged_kernel<S, ME><<<g_eval_staged, 256, 0, st>>>(ix, R, P, w, tally);
-        else wf_eval_kernel<S, ME><<<g_eval, 256, 0, st>>>(ix, R, P, w, tally);
+        wf_eval_kernel<S, ME><<<g_eval, 256, 0, st>>>(ix, R, P, w, tally);
         if (timed) cudaEventRecord(timer->e[3 * k + 2], st);
         wf_finalize_kernel<S><<<g_fin, 256, 0, st>>>(ix, R, P, out, w, act, nxt, width, k == rounds - 1, d_err,
                                                      tally);
@@ -807,16 +672,14 @@ int launch_seed_wavefront(const DevIndex& ix, const DevReads& R, const DevParams
     const int wn = t.wave_endpoints > 0 ? t.wave_endpoints : 1;
     int launches = 0;
     const int mr = t.wave_max_rounds, gr = t.wave_growth;
-    const bool refill = t.seed_kernel == 3;                         // lane-refill search
-    const bool staged = t.seed_kernel == 3 || t.seed_kernel == 4;  // staged-shift eval
     if (d_tally)
-        launches = launch_rounds<true, 1, 1, 1>(ix, R, P, out, w, max_len, w0, wn, mr, gr, refill, staged, sm_count, d_err, d_tally, timer, st);
+        launches = launch_rounds<true, 1, 1>(ix, R, P, out, w, max_len, w0, wn, mr, gr, sm_count, d_err, d_tally, timer, st);
     else if (t.reg_level == 1)
-        launches = launch_rounds<false, 5, 4, 4>(ix, R, P, out, w, max_len, w0, wn, mr, gr, refill, staged, sm_count, d_err, nullptr, timer, st);
+        launches = launch_rounds<false, 5, 4>(ix, R, P, out, w, max_len, w0, wn, mr, gr, sm_count, d_err, nullptr, timer, st);
     else if (t.reg_level == 2)
-        launches = launch_rounds<false, 6, 5, 5>(ix, R, P, out, w, max_len, w0, wn, mr, gr, refill, staged, sm_count, d_err, nullptr, timer, st);
+        launches = launch_rounds<false, 6, 5>(ix, R, P, out, w, max_len, w0, wn, mr, gr, sm_count, d_err, nullptr, timer, st);
     else
-        launches = launch_rounds<false, 1, 1, 1>(ix, R, P, out, w, max_len, w0, wn, mr, gr, refill, staged, sm_count, d_err, nullptr, timer, st);
+        launches = launch_rounds<false, 1, 1>(ix, R, P, out, w, max_len, w0, wn, mr, gr, sm_count, d_err, nullptr, timer, st);
     // reads that overflowed the locus list or outlived the rounds (their
     // tallies in the second half of the tally array, their time between
     // the timer's stage-2 events)
