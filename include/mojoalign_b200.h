@@ -317,8 +317,8 @@ int ma_last_launch_count(const ma_ctx* ctx);
  *                         after the first (1..256, default 8).
  *   wave_loci_per_read    wavefront locus list capacity per read of the
  *                         batch (1..64, default 4; at least 1024 entries);
- *                         reads whose loci do not fit a round are finished
- *                         by the stage-2 warps.
+ *                         reads whose loci do not fit a round wait for the
+ *                         next one, and for the stage-2 warps after the last.
  *   wave_max_rounds       wavefront rounds before the reads still active
  *                         go to the stage-2 warps (0 = as many as the
  *                         longest read needs, default).
@@ -327,6 +327,10 @@ int ma_last_launch_count(const ma_ctx* ctx);
  *                         fuller rounds for the reads that stay active
  *                         longest; default); 0: every later round covers
  *                         wave_endpoints.
+ * With stage1_endpoints and all wave_* fields at their defaults ma_map_batch
+ * and ma_map_batch_device fit the rounds to the call: batches too small to
+ * fill the GPU take one round, or two to three wide ones, and the locus list
+ * is longer (up to 256 entries per read within 64 MB, 8 within 512 MB).
  */
 typedef struct ma_tuning {
     int32_t seed_kernel;

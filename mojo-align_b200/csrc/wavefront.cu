@@ -18,8 +18,8 @@
 // in the reference's order, so pruning against that best and taking the
 // minimum key over the round gives the reference's hit.  A read whose loci
 // do not fit the list is left out of its round (its memo and best roll
-// back) and finished by the stage-2 warp kernel from that round's first
-// endpoint, as are reads still active after the last round.
+// back) and starts the next one from the same endpoint; reads still active
+// after the last round are finished by the stage-2 warp kernel.
 #include <cuda_runtime.h>
 
 #include "ma_device.cuh"
@@ -519,10 +519,12 @@ __global__ void __launch_bounds__(256) wf_finalize_kernel(DevIndex ix, DevReads 
             const Clamps cl = clamps_for(P, qlen);
             const int n_end = endpoint_count(P, qlen);
             if (w.overflow[r]) {
-                // left out of this round: roll back and let stage 2 redo it
+                // left out of this round: roll back; the next round takes the
+                // same endpoints up again, stage 2 after the last one
                 w.overflow[r] = 0;
                 w.memo_next[r] = w.memo_n[r];
-                to_stage2 = true;
+                if (last_round) to_stage2 = true;
+                else to_next = true;
             } else {
                 const uint32_t mn = w.memo_next[r];
                 w.memo_n[r] = static_cast<uint8_t>(mn < static_cast<uint32_t>(MEMO1) ? mn : MEMO1);
@@ -585,6 +587,9 @@ __global__ void __launch_bounds__(256) wf_finalize_kernel(DevIndex ix, DevReads 
     flush_tally<S>(t, tally_out);
 }
 
+// See wave_tuning below.
+constexpr int64_t WAVE_ONE = 131072, WAVE_ITEMS = 4 << 20, WAVE_LOCI = 2 << 20, WAVE_LOCI_MOST = 16 << 20;
+
 int endpoint_count_host(const DevParams& P, int qlen) {
     return qlen >= P.seed_len ? (qlen - P.seed_len) / P.seed_stride + 1 : 0;
 }
@@ -612,6 +617,12 @@ int launch_rounds(const DevIndex& ix, const DevReads& R, const DevParams& P, con
         covered += width;
         if (rounds == 0) width = wn;
         else if (growth && width < 4096) width *= 2;
+    }
+    // a large batch gets one more round for the reads that had to wait for list
+    // space (10 us when there are none): a warp each would take longer
+    if (R.n_seq > WAVE_ONE && rounds > 1) {
+        widths[rounds] = widths[rounds - 1];
+        ++rounds;
     }
     if (max_rounds > 0 && rounds > max_rounds) rounds = max_rounds;
     static const int g_search = grid_blocks(wf_search_kernel<S, MS>, sm_count);
@@ -651,6 +662,40 @@ int launch_rounds(const DevIndex& ix, const DevReads& R, const DevParams& P, con
 
 size_t wavefront_scratch_bytes(int64_t n_seq, int loci_per_read) {
     return wave_layout(nullptr, n_seq, locus_capacity(n_seq, loci_per_read), nullptr);
+}
+
+// The round widths and the locus list of a call under the default tuning,
+// fitted to its size; any other tuning is taken as it is.  A round costs the
+// latency of its longest search whatever its width, narrow rounds save the
+// searches of reads that a hit ends or predicts: a batch that does not fill
+// the GPU is better off with few wide ones.  Kernel time of all rounds, 2x150
+// pairs on 250 Mbp:
+//   32 pairs     5 rounds (1, 8, 16, 32, 64 endpoints) 0.27 ms, one round 0.09
+//   2 k pairs    5 rounds 0.74 ms, two rounds (2, the rest) 0.31
+//   16 k pairs   1.03 and 0.51 ms
+//   400 k 2x250  4.6 (8 endpoints, doubling) and 5.2 ms (16 endpoints)
+// So a batch of up to WAVE_ONE items (reads x endpoints) takes one round, and
+// a later round covers up to WAVE_ITEMS items.  Wide rounds need longer locus
+// lists: up to 256 entries per read while the list stays below 2 M entries (64
+// MB), 8 while it stays below 16 M (512 MB): 800 k reads of 250 bases take 4.3
+// ms with 8 entries and 4.9 with 4, whose list fills up.
+
+ma_tuning wave_tuning(const ma_tuning& asked, int64_t n_seq, int max_len, const DevParams& P) {
+    ma_tuning t = asked;
+    if (t.stage1_endpoints != 1 || t.wave_endpoints != 8 || t.wave_loci_per_read != 4 || t.wave_max_rounds != 0 ||
+        t.wave_growth != 1 || n_seq < 1)
+        return t;
+    const int64_t n_end = endpoint_count_host(P, max_len);
+    if (n_seq * n_end <= WAVE_ONE) {
+        t.stage1_endpoints = static_cast<int32_t>(n_end > 1 ? n_end : 1);
+    } else if (WAVE_ITEMS / n_seq > t.wave_endpoints) {
+        t.stage1_endpoints = 2;
+        t.wave_endpoints = static_cast<int32_t>(WAVE_ITEMS / n_seq < n_end ? WAVE_ITEMS / n_seq : n_end);
+    }
+    int64_t loci = WAVE_LOCI / n_seq < 256 ? WAVE_LOCI / n_seq : 256;
+    if (loci < 8 && n_seq * 8 <= WAVE_LOCI_MOST) loci = 8;
+    if (loci > t.wave_loci_per_read) t.wave_loci_per_read = static_cast<int32_t>(loci);
+    return t;
 }
 
 // The wavefront form; `scratch` holds wavefront_scratch_bytes(n_seq,

@@ -322,3 +322,14 @@ def test_config0_in_full(ctx, config0_ref):
     g = compare(prefix, ctx, rb.bases, rb.lens, rb.n1, False, 150, BENCH_PARAMS, bs=(1, 0),
                 tunings=[TUNINGS[0], TUNINGS[5]])
     assert 0.9 < (g.rid >= 0).mean() < 0.97  # the 5% random reads stay unmapped
+
+
+@pytest.mark.parametrize("n1,paired,max_len", [(1, False, 150), (40, True, 150), (900, True, 150), (1986, False, 150),
+                                               (1987, False, 150), (3000, True, 250), (70_000, False, 100)])
+def test_default_rounds_at_every_batch_size(ctx, small_ref, n1, paired, max_len):
+    """The default tuning fits its rounds to the call: one round up to 131072
+    (read, endpoint) items (66 endpoints of 150 bases: 1985 reads), two wide
+    ones above, and the widths of a large batch."""
+    fa, prefix = small_ref
+    rb = sim(fa, n1, paired, max_len=max_len, seed=n1, len_fixed=max_len)
+    compare(prefix, ctx, rb.bases, rb.lens, n1, paired, max_len, BENCH_PARAMS, tunings=[()])
