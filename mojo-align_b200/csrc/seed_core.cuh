@@ -486,21 +486,23 @@ __device__ uint32_t live_shifts(const DevIndex& ix, const ReadView& rd, int64_t 
     const uint32_t W2 = __funnelshift_r(w2, w3, sa), W3 = __funnelshift_r(w3, w4, sa);
     const uint32_t W4 = __funnelshift_r(w4, w5, sa);
     const uint32_t mb_odd = mb << 1;
+    auto stays = [&](int i) {  // fewer mismatches than the cap in shift i's halves
+        const uint32_t a = i < 16 ? W0 : W1, b = i < 16 ? W1 : W2, c = i < 16 ? W2 : W3, d = i < 16 ? W3 : W4;
+        const uint32_t sh = static_cast<uint32_t>(i & 15) * 2;
+        const uint32_t ta = qa ^ __funnelshift_r(a, b, sh);
+        const uint32_t tb = qb ^ __funnelshift_r(b, c, sh);
+        const uint32_t tc = qc ^ __funnelshift_r(c, d, sh);
+        const uint32_t xab = ((ta | (ta >> 1)) & ma) | ((tb | (tb << 1)) & mb_odd);
+        return __popc(xab) + __popc((tc | (tc >> 1)) & mc) < cap;
+    };
     uint32_t live = 0;
+    if (A == 17) {  // the default, with its shift amounts as constants
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {  // A <= 25: shifts 0..15 and 16..A-1
-        const uint32_t a = k == 0 ? W0 : W1, b = k == 0 ? W1 : W2;
-        const uint32_t c = k == 0 ? W2 : W3, d = k == 0 ? W3 : W4;
-        const int hi = A < 16 * k + 16 ? A : 16 * k + 16;
-        for (int i = 16 * k; i < hi; ++i) {
-            const uint32_t sh = static_cast<uint32_t>(i - 16 * k) * 2;
-            const uint32_t ta = qa ^ __funnelshift_r(a, b, sh);
-            const uint32_t tb = qb ^ __funnelshift_r(b, c, sh);
-            const uint32_t tc = qc ^ __funnelshift_r(c, d, sh);
-            const uint32_t xab = ((ta | (ta >> 1)) & ma) | ((tb | (tb << 1)) & mb_odd);
-            const uint32_t xc = (tc | (tc >> 1)) & mc;
-            if (__popc(xab) + __popc(xc) < cap) live |= 1u << i;
-        }
+        for (int i = 0; i < 17; ++i)
+            if (stays(i)) live |= 1u << i;
+    } else {
+        for (int i = 0; i < A; ++i)
+            if (stays(i)) live |= 1u << i;
     }
     if (!is_rev && !((live >> adj_cap) & 1u)) {
         // the deletion probe's bound from the exact mismatch bits (N bases

@@ -152,15 +152,22 @@ __global__ void wf_round_begin_kernel(Wave w) {
     *loci_count(w) = 0;
 }
 
-// Whether an SA row of a found seed gives a locus not evaluated before.
-__device__ __forceinline__ bool fresh_locus(const DevIndex& ix, const Wave& w, int64_t r, int n_memo, uint64_t sa_pos,
-                                            int us, int e, int qlen, int64_t& b0, int& rev) {
-    if (!locus_of_row(ix, sa_pos, us, e, qlen, b0, rev)) return false;
-    const uint64_t tag = static_cast<uint64_t>(b0 * 2 + rev);
-    for (int m = 0; m < n_memo; ++m)
-        if (w.memo[r * MEMO1 + m] == tag) return false;
-    return true;
-}
+// A read's memo (MEMO1 loci, 64 bytes), all of it in flight at once; entries
+// from n on are not valid.
+struct MemoRow {
+    ulonglong2 v[MEMO1 / 2];
+    __device__ __forceinline__ MemoRow(const Wave& w, uint32_t r) {
+        const ulonglong2* p = reinterpret_cast<const ulonglong2*>(w.memo + static_cast<uint64_t>(r) * MEMO1);
+#pragma unroll
+        for (int i = 0; i < MEMO1 / 2; ++i) v[i] = p[i];
+    }
+    __device__ __forceinline__ bool holds(uint64_t tag, int n) const {
+        bool found = false;
+#pragma unroll
+        for (int i = 0; i < MEMO1 / 2; ++i) found |= (2 * i < n && v[i].x == tag) || (2 * i + 1 < n && v[i].y == tag);
+        return found;
+    }
+};
 
 // Search: the round's items are (active read, endpoint) pairs.  Most end at
 // their table lookup, the others step back one base at a time for anything
@@ -180,7 +187,7 @@ __device__ __forceinline__ bool fresh_locus(const DevIndex& ix, const Wave& w, i
 //           leave their slot dead.
 // Which pass finds a seed does not change the round's result: the eval keys
 // carry the candidate order.
-// 2 M uneven reads on 250 Mbp (62 M lookups, 56 M steps, 103 M rows): 8.8 ms,
+// 2 M uneven reads on 250 Mbp (62 M lookups, 56 M steps, 103 M rows): 8.1 ms,
 // 10.1 ms with a thread per item through all three; 800 k reads of 250 bases
 // 2.05 and 2.7 ms.  Bound by the latency of the gathers.
 constexpr int SEARCH_WARPS = 8;   // 256 threads
@@ -287,6 +294,8 @@ __global__ void __launch_bounds__(256, MINB) wf_search_kernel(DevIndex ix, DevRe
                     w.overflow[r] = 1;
                     continue;
                 }
+                const MemoRow memo(w, r);  // in flight together with the SA row
+                const int n_memo = w.memo_n[r];
                 const uint64_t k = q.seed_k[lo], sa_pos = sa_at(ix, k + (idx - first));
                 if constexpr (S) t.sa_loads++;
                 const uint32_t s_e = q.s_e[lo], ei_len = q.ei_len[lo];
@@ -295,7 +304,8 @@ __global__ void __launch_bounds__(256, MINB) wf_search_kernel(DevIndex ix, DevRe
                 WLocus L;
                 int64_t b0;
                 int rev;
-                if (!fresh_locus(ix, w, r, w.memo_n[r], sa_pos, s, e, qlen, b0, rev)) {
+                if (!locus_of_row(ix, sa_pos, s, e, qlen, b0, rev) ||
+                    memo.holds(static_cast<uint64_t>(b0 * 2 + rev), n_memo)) {
                     w.loci[slot].read = DEAD_LOCUS;
                     continue;
                 }
