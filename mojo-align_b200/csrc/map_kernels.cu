@@ -487,8 +487,9 @@ __global__ void __launch_bounds__(S2_WARPS * 32, MINB) seed_stage2_kernel(DevInd
                         const int bit = static_cast<int>(__fns(o_live, 0, idx - o_first + 1));
                         const Locus L = s_loci[own];
                         const uint64_t before = lb.key;
-                        eval_adj<S>(ix, rd, L.b0, L.rev, bit - cl.adj_cap, cl.budget, cl.clip_cap, L.ord_row, lb,
-                                    L.uk, L.ul, L.us, L.e, prune, t);
+                        const Shift sh{L.b0, L.rev, bit - cl.adj_cap, cl.budget, cl.clip_cap, prune,
+                                       L.ord_row, L.uk, L.ul, L.us, L.e};
+                        eval_shift_whole<S>(ix, rd, sh, lb, t);
                         if (lb.key != before) lb_tag = L.b0 * 2 + L.rev;
                     }
                 }

@@ -311,16 +311,15 @@ __device__ __forceinline__ void set_best(Best& best, uint64_t key, int64_t crid,
     best.e = e;
 }
 
-// The deletion probe of a failed forward shift (L1729-1825), kept out of
-// line: it is rare on the hot path.  Every read position mismatches under
-// shift 0 or under shift +1 for every g unless it matches under one of
-// them, so nm_d(g) >= 1 + popc(M0 & M1) for all g; when that bound already
-// exceeds the budget or cannot beat the best so far, no offset is tried.
+// Whether the deletion probe of a failed forward shift (L1729-1825) can fold
+// a candidate.  Every read position mismatches under shift 0 or under shift +1
+// for every g unless it matches under one of them, so nm_d(g) >= 1 + popc(M0 &
+// M1) for all g; when that bound already exceeds the budget or cannot beat the
+// best so far, no offset is tried.
 template <bool S>
-__device__ __noinline__ void deletion_candidates(const uint64_t* __restrict__ pacw, const uint64_t* q,
-                                                 const uint64_t* qn, int64_t bstart, int qlen, int budget,
-                                                 int prune_nm, uint32_t ord, int64_t crid, int64_t local,
-                                                 Best& best, uint64_t uk, uint64_t ul, int us, int e, Tally& t) {
+__device__ __forceinline__ bool deletion_possible(const uint64_t* __restrict__ pacw, const uint64_t* q,
+                                                  const uint64_t* qn, int64_t bstart, int qlen, int budget,
+                                                  int prune_nm, Tally& t) {
     const int nw = (qlen + 31) >> 5;
     const int stop = prune_nm < budget + 1 ? prune_nm : budget + 1;  // 1 + bound >= stop: nothing to gain
     int both = 0;
@@ -330,13 +329,9 @@ __device__ __noinline__ void deletion_candidates(const uint64_t* __restrict__ pa
         if (bstart < 0) m0 |= range_mask(w, 0, static_cast<int>(-bstart));
         if (bstart + 1 < 0) m1 |= range_mask(w, 0, static_cast<int>(-(bstart + 1)));
         both += __popcll(m0 & m1 & range_mask(w, 0, qlen));
-        if (1 + both >= stop) return;
+        if (1 + both >= stop) return false;
     }
-    deletion_scan<S>(pacw, q, qn, bstart, qlen, budget, t, [&](int g, int nmd) {
-        if (nmd > budget) return;
-        const uint64_t key = (static_cast<uint64_t>(nmd) << ORD_SHIFT) | (ord + 1 + g / 4);
-        if (key < best.key) set_best(best, key, crid, local, 0, 0, 20u, 0, uk, ul, us, e);
-    });
+    return true;
 }
 
 // Soft-clip retry of L1591-1694: sl grows to the first matching in-contig
@@ -367,70 +362,155 @@ __device__ __noinline__ int soft_clip_recount(const uint64_t* __restrict__ pacw,
 }
 
 // One shift adj of one locus (b0, strand): the body of the reference's adj
-// loop, linear_gpu_fm.mojo:1528-1826.  Folds the candidate (full compare,
-// or the deletion probe's offsets) into `best` by its (nm, ordinal) key.
-// prune_nm: a candidate of this call can only matter when its nm is below
+// loop, linear_gpu_fm.mojo:1528-1826, in parts that a caller may run at
+// different times: the core compare, which most shifts fail, the full compare
+// with its clips, the deletion probe's bound and its offsets.
+// prune_nm: a candidate of this shift can only matter when its nm is below
 // prune_nm (every candidate of the call comes after the current best in the
-// reference's order); 1 << 20 disables pruning.  The contig is searched for
-// only once the core compare, which most shifts fail, has not ruled the shift
-// out: the reference drops a shift whose clips at its contig's ends exceed
-// clip_cap, and a read that overhangs the text by more than that does so on
-// any contig (the text's ends are contig ends), so the compares read at most
-// clip_cap bases past them.
+// reference's order); 1 << 20 disables pruning.
+struct Shift {
+    int64_t b0;
+    int is_rev, adj, budget, clip_cap, prune_nm;
+    uint32_t ord_row;
+    uint64_t uk, ul;
+    int us, e;
+    __device__ __forceinline__ int64_t bstart() const { return b0 + adj; }
+    __device__ __forceinline__ bool del_probe() const { return adj == 0 && is_rev == 0; }
+    __device__ __forceinline__ uint32_t ord() const { return (ord_row + static_cast<uint32_t>(adj + 12)) * KIND_SPAN; }
+};
+enum : int { SHIFT_DEAD = 0, SHIFT_FULL = 1, SHIFT_DELETION = 2, SHIFT_OFFSETS = 3 };  // what is left to try
+
+// Exact pruning by the core.  The reference drops a shift whose clips at its
+// contig's ends exceed clip_cap, and a read that overhangs the text by more
+// than that does so on any contig (the text's ends are contig ends), so the
+// compares read at most clip_cap bases past them.  The contig clips and every
+// soft clip are at most clip_cap, so the full compare and any clipped recount
+// both span read positions [clip_cap, qlen - clip_cap); their mismatches bound
+// nm from below.  A shift without deletion probe only matters with a core
+// below both the budget and the best so far: count no further.
 template <bool S>
-__device__ void eval_adj(const DevIndex& ix, const ReadView& rd, int64_t b0, int is_rev, int adj, int budget,
-                         int clip_cap, uint32_t ord_row, Best& best, uint64_t uk, uint64_t ul, int us, int e,
-                         int prune_nm, Tally& t) {
+__device__ __forceinline__ int shift_core(const DevIndex& ix, const ReadView& rd, const Shift& c, Tally& t) {
     if constexpr (S) t.shifts++;
     const int qlen = rd.qlen;
-    const uint64_t* q = is_rev ? rd.rc : rd.fwd;
-    const uint64_t* qn = is_rev ? rd.nr : rd.nf;
-    const int64_t bstart = b0 + adj;
-    if (bstart < -clip_cap || bstart + qlen > static_cast<int64_t>(ix.l_pac) + clip_cap) return;
-    const bool del_probe = adj == 0 && is_rev == 0;
-    // Exact pruning.  sl0, sr0 and every soft clip are at most clip_cap, so
-    // the full compare and any clipped recount both span read positions
-    // [clip_cap, qlen - clip_cap); their mismatches bound nm from below.  A
-    // shift without deletion probe only matters with a core below both the
-    // budget and the best so far: count no further.
-    const int cap = del_probe ? budget + 1 : (prune_nm < budget + 1 ? prune_nm : budget + 1);
-    const int core = count_mm<S>(ix.pacw, q, qn, bstart, clip_cap, qlen - clip_cap, cap, t);
-    if (core >= cap && !(del_probe && prune_nm > 1)) return;
-    // the contig holding the clamped probe (binary search, L1536-1549)
+    const int64_t bstart = c.bstart();
+    if (bstart < -c.clip_cap || bstart + qlen > static_cast<int64_t>(ix.l_pac) + c.clip_cap) return SHIFT_DEAD;
+    const int most = c.budget + 1;
+    const int cap = c.del_probe() ? most : (c.prune_nm < most ? c.prune_nm : most);
+    const int core = count_mm<S>(ix.pacw, c.is_rev ? rd.rc : rd.fwd, c.is_rev ? rd.nr : rd.nf, bstart, c.clip_cap,
+                                 qlen - c.clip_cap, cap, t);
+    if (core < cap) return SHIFT_FULL;
+    // neither compare is accepted: only the deletion probe remains
+    return c.del_probe() && c.prune_nm > 1 ? SHIFT_DELETION : SHIFT_DEAD;
+}
+
+// The contig holding the clamped probe (binary search, L1536-1549); false when
+// there is none or the clips at its ends rule the shift out.
+struct ShiftContig {
+    int64_t crid, coff, clen;
+};
+__device__ __forceinline__ bool shift_contig(const DevIndex& ix, int64_t bstart, int qlen, int clip_cap,
+                                             ShiftContig& k) {
     int64_t probe = bstart < 0 ? 0 : bstart;
     if (probe >= static_cast<int64_t>(ix.l_pac)) probe = static_cast<int64_t>(ix.l_pac) - 1;
-    const int64_t crid = contig_of(ix, probe);
-    if (crid < 0) return;
-    const int64_t coff = static_cast<int64_t>(__ldg(ix.coff + crid)), clen = static_cast<int64_t>(__ldg(ix.clen + crid));
-    const int64_t local = bstart - coff;
+    k.crid = contig_of(ix, probe);
+    if (k.crid < 0) return false;
+    k.coff = static_cast<int64_t>(__ldg(ix.coff + k.crid));
+    k.clen = static_cast<int64_t>(__ldg(ix.clen + k.crid));
+    const int64_t local = bstart - k.coff;
     const int64_t sl0 = local < 0 ? -local : 0;
-    const int64_t sr0 = local + qlen > clen ? local + qlen - clen : 0;
-    if (!(sl0 + sr0 < qlen && sl0 <= clip_cap && sr0 <= clip_cap)) return;
-    const uint32_t ord = (ord_row + static_cast<uint32_t>(adj + 12)) * KIND_SPAN;
-    const bool del_room = del_probe && prune_nm > 1 && bstart + qlen + 1 <= coff + clen;
-    if (core > budget) {
-        // neither compare is accepted: only the deletion probe remains
-        if (del_room)
-            deletion_candidates<S>(ix.pacw, q, qn, bstart, qlen, budget, prune_nm, ord, crid, local, best, uk, ul,
-                                   us, e, t);
-        return;
-    }
-    // whether the compare is accepted decides the deletion probe, so only
-    // shifts without one can stop here
-    if (core >= prune_nm && !del_probe) return;
-    int nm = count_mm<S>(ix.pacw, q, qn, bstart, static_cast<int>(sl0), static_cast<int>(qlen - sr0), budget + 1, t);
-    int sl = static_cast<int>(sl0), sr = static_cast<int>(sr0);
-    if (nm > budget && clip_cap > 0)
-        nm = soft_clip_recount<S>(ix.pacw, q, qn, bstart, qlen, local, clen, sl, sr, clip_cap, budget, &sl, &sr, t);
+    const int64_t sr0 = local + qlen > k.clen ? local + qlen - k.clen : 0;
+    return sl0 + sr0 < qlen && sl0 <= clip_cap && sr0 <= clip_cap;
+}
+
+// The full compare and its clipped recount; folds an accepted candidate into
+// `best` by its (nm, ordinal) key.  What is left: SHIFT_DELETION or
+// SHIFT_DEAD.
+template <bool S>
+__device__ __forceinline__ int shift_full(const DevIndex& ix, const ReadView& rd, const Shift& c, Best& best, Tally& t) {
+    const int qlen = rd.qlen;
+    const int64_t bstart = c.bstart();
+    ShiftContig k;
+    if (!shift_contig(ix, bstart, qlen, c.clip_cap, k)) return SHIFT_DEAD;
+    const uint64_t* q = c.is_rev ? rd.rc : rd.fwd;
+    const uint64_t* qn = c.is_rev ? rd.nr : rd.nf;
+    const int64_t local = bstart - k.coff;
+    int sl = static_cast<int>(local < 0 ? -local : 0);
+    int sr = static_cast<int>(local + qlen > k.clen ? local + qlen - k.clen : 0);
+    int nm = count_mm<S>(ix.pacw, q, qn, bstart, sl, qlen - sr, c.budget + 1, t);
+    if (nm > c.budget && c.clip_cap > 0)
+        nm = soft_clip_recount<S>(ix.pacw, q, qn, bstart, qlen, local, k.clen, sl, sr, c.clip_cap, c.budget, &sl, &sr, t);
     const int alen = qlen - sl - sr;
-    if (nm <= budget && alen >= 24) {
-        const uint64_t key = (static_cast<uint64_t>(nm) << ORD_SHIFT) | ord;
+    if (nm <= c.budget && alen >= 24) {
+        const uint64_t key = (static_cast<uint64_t>(nm) << ORD_SHIFT) | c.ord();
         if (key < best.key)
-            set_best(best, key, crid, local + sl, sl, sr, nm == 0 ? 60u : 20u, is_rev * 16, uk, ul, us, e);
-    } else if (del_room) {
-        deletion_candidates<S>(ix.pacw, q, qn, bstart, qlen, budget, prune_nm, ord, crid, local, best, uk, ul, us,
-                               e, t);
+            set_best(best, key, k.crid, local + sl, sl, sr, nm == 0 ? 60u : 20u, c.is_rev * 16, c.uk, c.ul, c.us, c.e);
+        return SHIFT_DEAD;
     }
+    return c.del_probe() && c.prune_nm > 1 ? SHIFT_DELETION : SHIFT_DEAD;
+}
+
+// Whether any of the deletion probe's offsets can give a candidate.
+template <bool S>
+__device__ __forceinline__ int shift_deletion(const DevIndex& ix, const ReadView& rd, const Shift& c, Tally& t) {
+    const int64_t bstart = c.bstart();
+    if (!deletion_possible<S>(ix.pacw, c.is_rev ? rd.rc : rd.fwd, c.is_rev ? rd.nr : rd.nf, bstart, rd.qlen, c.budget,
+                              c.prune_nm, t))
+        return SHIFT_DEAD;
+    ShiftContig k;
+    return shift_contig(ix, bstart, rd.qlen, c.clip_cap, k) && bstart + rd.qlen + 1 <= k.coff + k.clen ? SHIFT_OFFSETS
+                                                                                                       : SHIFT_DEAD;
+}
+
+// The deletion probe's offsets, folded into `best`.
+template <bool S>
+__device__ __forceinline__ void shift_offsets(const DevIndex& ix, const ReadView& rd, const Shift& c, Best& best,
+                                              Tally& t) {
+    const int64_t bstart = c.bstart();
+    ShiftContig k;
+    if (!shift_contig(ix, bstart, rd.qlen, c.clip_cap, k)) return;
+    const uint32_t ord = c.ord();
+    deletion_scan<S>(ix.pacw, c.is_rev ? rd.rc : rd.fwd, c.is_rev ? rd.nr : rd.nf, bstart, rd.qlen, c.budget, t,
+                     [&](int g, int nmd) {
+                         if (nmd > c.budget) return;
+                         const uint64_t key = (static_cast<uint64_t>(nmd) << ORD_SHIFT) | (ord + 1 + g / 4);
+                         if (key < best.key)
+                             set_best(best, key, k.crid, bstart - k.coff, 0, 0, 20u, 0, c.uk, c.ul, c.us, c.e);
+                     });
+}
+
+// The candidate of a known key (nm, ordinal) of shift c, for the hit's fields:
+// the full compare again, or for a deletion offset its place and a check of
+// its count.  False when the shift does not give that candidate.
+template <bool S>
+__device__ __forceinline__ bool shift_candidate(const DevIndex& ix, const ReadView& rd, const Shift& c, uint64_t key,
+                                                Best& best, Tally& t) {
+    const uint32_t kind = static_cast<uint32_t>(key & ((1ull << ORD_SHIFT) - 1)) - c.ord();
+    best.key = ~0ull;
+    best.crid = -1;
+    if (kind == 0) {
+        shift_full<S>(ix, rd, c, best, t);
+        return best.key == key;
+    }
+    const int64_t bstart = c.bstart();
+    ShiftContig k;
+    if (!shift_contig(ix, bstart, rd.qlen, c.clip_cap, k)) return false;
+    const int g = 4 * static_cast<int>(kind - 1), nm = static_cast<int>(key >> ORD_SHIFT);
+    if (bstart >= 0) {  // text positions below 0 never match (deletion_scan); not counted again here
+        const int left = count_mm<S>(ix.pacw, rd.fwd, rd.nf, bstart, 0, g < rd.qlen ? g : rd.qlen, nm + 1, t);
+        const int right = count_mm<S>(ix.pacw, rd.fwd, rd.nf, bstart + 1, g, rd.qlen, nm + 1, t);
+        if (1 + left + right != nm) return false;
+    }
+    set_best(best, key, k.crid, bstart - k.coff, 0, 0, 20u, 0, c.uk, c.ul, c.us, c.e);
+    return true;
+}
+
+// All parts at once.
+template <bool S>
+__device__ void eval_shift_whole(const DevIndex& ix, const ReadView& rd, const Shift& c, Best& best, Tally& t) {
+    int left = shift_core<S>(ix, rd, c, t);
+    if (left == SHIFT_FULL) left = shift_full<S>(ix, rd, c, best, t);
+    if (left == SHIFT_DELETION) left = shift_deletion<S>(ix, rd, c, t);
+    if (left == SHIFT_OFFSETS) shift_offsets<S>(ix, rd, c, best, t);
 }
 
 // Shifts of one locus that can fold a candidate into a best of nm prune_nm
@@ -459,7 +539,7 @@ __device__ uint32_t live_shifts(const DevIndex& ix, const ReadView& rd, int64_t 
     const int h0 = c0 >> 4;
     const int hl = (c1 - 1) >> 4;  // last half holding core bases
     const int nh = hl - h0 + 1 < 3 ? hl - h0 + 1 : 3;
-    // loci whose filter window leaves the text are left to eval_adj
+    // loci whose filter window leaves the text are left to the compares
     if (b0 - adj_cap + 16 * h0 < 0 || b0 + adj_cap + 1 + 16 * (h0 + nh) > static_cast<int64_t>(ix.l_pac)) return all;
     // the text of every shift's halves lies in six 16-base words from wlo:
     // shift i starts s0 + i bases into them
@@ -540,8 +620,9 @@ __device__ void eval_locus(const DevIndex& ix, const ReadView& rd, int64_t b0, i
         const int adj = __ffs(live) - 1 - adj_cap;
         live &= live - 1;
         const uint64_t bn = best.key >> ORD_SHIFT;
-        eval_adj<S>(ix, rd, b0, is_rev, adj, budget, clip_cap, ord_row, best, uk, ul, us, e,
-                    bn < (1u << 20) ? static_cast<int>(bn) : (1 << 20), t);
+        const Shift c{b0, is_rev, adj, budget, clip_cap, bn < (1u << 20) ? static_cast<int>(bn) : (1 << 20),
+                      ord_row, uk, ul, us, e};
+        eval_shift_whole<S>(ix, rd, c, best, t);
     }
 }
 

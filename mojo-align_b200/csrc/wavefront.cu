@@ -399,106 +399,122 @@ __global__ void __launch_bounds__(256, MINB) wf_search_kernel(DevIndex ix, DevRe
     flush_tally<S>(t, tally_out);
 }
 
-// Eval: one thread per locus filters its shifts (live_shifts); the live
-// shifts (a fraction of a shift per locus at genome scale) are staged per warp
-// in shared memory and evaluated 32 at a time, so the full compares run with
-// every lane busy.  Candidates are pruned against the read's best from earlier
-// rounds; the round's minimum key per read is an atomicMin of (nm, ordinal,
-// locus index) packed in 64 bits.
+// Eval: one thread per locus filters its shifts (live_shifts); what is left
+// goes through the parts of a shift (seed_core.cuh) in lists of the warp, in
+// shared memory, each part run with 32 entries, one per lane: the core
+// compare of the live shifts (a fraction of a shift per locus at genome
+// scale), the full compare of those that pass, the deletion probe's bound of
+// those that need it and its offsets where the bound allows one.  With the parts run one after the other by the lane that had
+// the shift, the rare long ones kept the warp at 16 lanes of 32.  Candidates
+// are pruned against the read's best from earlier rounds; the round's minimum
+// key per read is an atomicMin of (nm, ordinal, locus index) packed in 64 bits.
+// 102 M loci, 31 M live shifts of 2 M uneven reads: 6.7 ms, 8.0 ms before.
 constexpr int EVAL_THREADS = 256;
+constexpr int SHIFT_LIST = 64;  // entries per list and warp: locus index << 5 | shift
+enum : int { L_CORE = 0, L_FULL = SHIFT_FULL, L_DELETION = SHIFT_DELETION, L_OFFSETS = SHIFT_OFFSETS };
 
-// One shift (adj) of the locus at list index li: its candidates, pruned
-// against the read's best from earlier rounds, and the atomicMin of the
-// round key.
-template <bool S>
-__device__ __forceinline__ void eval_shift(const DevIndex& ix, const DevReads& R, const DevParams& P, const Wave& w,
-                                           const WLocus& L, uint32_t li, int adj, Tally& t) {
-    const int64_t r = L.read;
-    const ReadView rd = read_view(R, r);
-    const Clamps cl = clamps_for(P, rd.qlen);
+// The largest nm that can still matter for read r.
+__device__ __forceinline__ int prune_of(const Wave& w, uint32_t r) {
     const uint64_t bn = w.best_key[r] >> ORD_SHIFT;
-    const int prune = bn < (1u << 20) ? static_cast<int>(bn) : (1 << 20);
-    Best lb;
-    lb.key = ~0ull;
-    lb.crid = -1;
-    eval_adj<S>(ix, rd, L.b0, L.rev, adj, cl.budget, cl.clip_cap, L.ord_row, lb, L.uk, L.ul(), L.us, L.e(), prune,
-                t);
-    if (lb.key != ~0ull) {
-        const uint64_t nm = lb.key >> ORD_SHIFT;
-        const uint64_t ord = lb.key & ((1ull << ORD_SHIFT) - 1);
-        atomicMin(reinterpret_cast<unsigned long long*>(w.round_key + r),
-                  static_cast<unsigned long long>((nm << (ORD_SHIFT + w.idx_bits)) | (ord << w.idx_bits) | li));
-    }
+    return bn < (1u << 20) ? static_cast<int>(bn) : (1 << 20);
 }
 
-constexpr int SHIFT_STAGE = 64;  // staged shifts per warp: locus index << 5 | shift
-
 template <bool S, int MINB>
-__global__ void __launch_bounds__(EVAL_THREADS, MINB) wf_eval_kernel(DevIndex ix, DevReads R, DevParams P,
-                                                                      Wave w,
-                                                                      unsigned long long* __restrict__ tally_out) {
-    __shared__ uint64_t s_shift[EVAL_THREADS / 32][SHIFT_STAGE];
+__global__ void __launch_bounds__(EVAL_THREADS, MINB) wf_eval_kernel(DevIndex ix, DevReads R, DevParams P, Wave w,
+                                                               unsigned long long* __restrict__ tally_out) {
+    __shared__ uint64_t s_list[EVAL_THREADS / 32][4][SHIFT_LIST];
     constexpr unsigned FULL = 0xFFFFFFFFu;
     Tally t{};
     uint64_t n_loci = *loci_count(w);
     if (n_loci > w.locus_cap) n_loci = w.locus_cap;
     const int adj_cap = clamps_for(P, 1 << 20).adj_cap;  // read-independent
     const int lane = threadIdx.x & 31;
-    uint64_t* stage = s_shift[threadIdx.x >> 5];
-    int staged = 0;  // warp-uniform
+    const unsigned lt_mask = (1u << lane) - 1;
+    uint64_t(*list)[SHIFT_LIST] = s_list[threadIdx.x >> 5];
+    int n[4] = {0, 0, 0, 0};  // entries of each list (warp-uniform)
+    uint32_t rem = 0, li = 0;  // the lane's locus and its live shifts not yet listed
     const uint32_t stride = gridDim.x * blockDim.x;
-    // one more pass after the warp's last loci empties the stage
-    for (uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u);; base += stride) {
-        const bool have = base < n_loci;
-        const uint32_t li = base + lane;
-        uint32_t rem = 0;  // the lane's live shifts not yet staged
-        if (have && li < n_loci) {
-            const WLocus L = w.loci[li];
-            const int64_t r = L.read;
-            if (L.read != DEAD_LOCUS && !w.overflow[r]) {
-                const ReadView rd = read_view(R, r);
+    uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u);
+    for (;;) {
+        const bool have = base < n_loci, pending = __any_sync(FULL, rem != 0);
+        // a full list first, the last part's before the others; then the shifts
+        // waiting, the next loci, and in the end what the lists still hold
+        int part = -1;
+        if (n[L_OFFSETS] >= 32) part = L_OFFSETS;
+        else if (n[L_DELETION] >= 32) part = L_DELETION;
+        else if (n[L_FULL] >= 32) part = L_FULL;
+        else if (n[L_CORE] >= 32) part = L_CORE;
+        else if (!pending && !have) part = n[L_CORE] ? L_CORE : n[L_FULL] ? L_FULL : n[L_DELETION] ? L_DELETION : L_OFFSETS;
+        if (part >= 0) {
+            const int count = part == L_CORE ? n[L_CORE] : part == L_FULL ? n[L_FULL]
+                              : part == L_DELETION ? n[L_DELETION] : n[L_OFFSETS];
+            if (count == 0) break;
+            __syncwarp();
+            const int from = count > 32 ? count - 32 : 0;  // the last 32 entries
+            const bool on = lane < count - from;
+            const uint64_t v = on ? list[part][from + lane] : 0;
+            if (part == L_CORE) n[L_CORE] = from;
+            else if (part == L_FULL) n[L_FULL] = from;
+            else if (part == L_DELETION) n[L_DELETION] = from;
+            else n[L_OFFSETS] = from;
+            int left = SHIFT_DEAD;
+            if (on) {
+                const uint32_t i = static_cast<uint32_t>(v >> 5);
+                const WLocus L = w.loci[i];
+                const ReadView rd = read_view(R, L.read);
                 const Clamps cl = clamps_for(P, rd.qlen);
-                const uint64_t bn = w.best_key[r] >> ORD_SHIFT;
-                const int prune = bn < (1u << 20) ? static_cast<int>(bn) : (1 << 20);
-                rem = live_shifts<S>(ix, rd, L.b0, L.rev, adj_cap, cl.budget, cl.clip_cap, prune, t);
+                const Shift c{L.b0, L.rev, static_cast<int>(v & 31) - adj_cap, cl.budget, cl.clip_cap,
+                              prune_of(w, L.read), L.ord_row, L.uk, L.ul(), L.us, L.e()};
+                if (part == L_CORE) {
+                    left = shift_core<S>(ix, rd, c, t);
+                } else if (part == L_DELETION) {
+                    left = shift_deletion<S>(ix, rd, c, t);
+                } else {
+                    Best lb;
+                    lb.key = ~0ull;
+                    if (part == L_FULL) left = shift_full<S>(ix, rd, c, lb, t);
+                    else shift_offsets<S>(ix, rd, c, lb, t);
+                    if (lb.key != ~0ull) {
+                        const uint64_t nm = lb.key >> ORD_SHIFT, ord = lb.key & ((1ull << ORD_SHIFT) - 1);
+                        atomicMin(reinterpret_cast<unsigned long long*>(w.round_key + L.read),
+                                  static_cast<unsigned long long>((nm << (ORD_SHIFT + w.idx_bits)) | (ord << w.idx_bits) | i));
+                    }
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int k = L_FULL; k <= L_OFFSETS; ++k) {
+                const unsigned kb = __ballot_sync(FULL, left == k);
+                if (left == k) list[k][n[k] + __popc(kb & lt_mask)] = v;
+                n[k] += __popc(kb);
+            }
+        } else if (pending) {
+            // as many live shifts as fit (lanes in order)
+            const int k = __popc(rem);
+            int incl = k;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(FULL, incl, o);
+                if (lane >= o) incl += v;
+            }
+            int at = n[L_CORE] + incl - k;
+            while (rem && at < SHIFT_LIST) {
+                list[L_CORE][at++] = static_cast<uint64_t>(li) << 5 | static_cast<uint32_t>(__ffs(rem) - 1);
+                rem &= rem - 1;
+            }
+            const int total = n[L_CORE] + __shfl_sync(FULL, incl, 31);
+            n[L_CORE] = total < SHIFT_LIST ? total : SHIFT_LIST;
+        } else {
+            li = base + lane;
+            base += stride;
+            if (li < n_loci) {
+                const WLocus L = w.loci[li];
+                if (L.read != DEAD_LOCUS && !w.overflow[L.read]) {
+                    const ReadView rd = read_view(R, L.read);
+                    const Clamps cl = clamps_for(P, rd.qlen);
+                    rem = live_shifts<S>(ix, rd, L.b0, L.rev, adj_cap, cl.budget, cl.clip_cap, prune_of(w, L.read), t);
+                }
             }
         }
-        for (;;) {
-            // stage as many live shifts as fit (lanes in order)
-            if (__ballot_sync(FULL, rem != 0)) {
-                const int n = __popc(rem);
-                int incl = n;
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int v = __shfl_up_sync(FULL, incl, o);
-                    if (lane >= o) incl += v;
-                }
-                int at = staged + incl - n;
-                while (rem && at < SHIFT_STAGE) {
-                    stage[at++] = static_cast<uint64_t>(li) << 5 | static_cast<uint32_t>(__ffs(rem) - 1);
-                    rem &= rem - 1;
-                }
-                const int total = staged + __shfl_sync(FULL, incl, 31);
-                staged = total < SHIFT_STAGE ? total : SHIFT_STAGE;
-            }
-            const bool pending = __ballot_sync(FULL, rem != 0) != 0;
-            if (staged < 32 && (have || staged == 0)) break;
-            // evaluate the first 32 (or the last few) staged shifts, one per lane
-            const int n = staged < 32 ? staged : 32;
-            __syncwarp();
-            if (lane < n) {
-                const uint64_t v = stage[lane];
-                const uint32_t sli = static_cast<uint32_t>(v >> 5);
-                eval_shift<S>(ix, R, P, w, w.loci[sli], sli, static_cast<int>(v & 31) - adj_cap, t);
-            }
-            __syncwarp();
-            const uint64_t v = lane < staged - n ? stage[n + lane] : 0;
-            __syncwarp();
-            if (lane < staged - n) stage[lane] = v;
-            staged -= n;
-            __syncwarp();
-            if (!pending && staged < 32 && have) break;
-        }
-        if (!have) break;
     }
     flush_tally<S>(t, tally_out);
 }
@@ -506,7 +522,7 @@ __global__ void __launch_bounds__(EVAL_THREADS, MINB) wf_eval_kernel(DevIndex ix
 // Finalize: one thread per active read (warp-uniform loop for the list
 // appends).  last_round: reads with endpoints left go to stage 2.
 template <bool S>
-__global__ void __launch_bounds__(256) wf_finalize_kernel(DevIndex ix, DevReads R, DevParams P, DevOut out, Wave w,
+__global__ void __launch_bounds__(256, 4) wf_finalize_kernel(DevIndex ix, DevReads R, DevParams P, DevOut out, Wave w,
                                                           const uint32_t* __restrict__ act,
                                                           uint32_t* __restrict__ next, int width, int last_round,
                                                           int* __restrict__ err,
@@ -550,11 +566,8 @@ __global__ void __launch_bounds__(256) wf_finalize_kernel(DevIndex ix, DevReads 
                     const uint64_t bn = old >> ORD_SHIFT;
                     const int prune = bn < (1u << 20) ? static_cast<int>(bn) : (1 << 20);
                     Best lb;
-                    lb.key = ~0ull;
-                    lb.crid = -1;
-                    eval_adj<S>(ix, rd, L.b0, L.rev, adj, cl.budget, cl.clip_cap, L.ord_row, lb, L.uk, L.ul(),
-                                L.us, L.e(), prune, t);
-                    if (lb.key != rkey) {
+                    const Shift c{L.b0, L.rev, adj, cl.budget, cl.clip_cap, prune, L.ord_row, L.uk, L.ul(), L.us, L.e()};
+                    if (!shift_candidate<S>(ix, rd, c, rkey, lb, t)) {
                         atomicExch(err, 3);  // the recomputed candidate must be the round's minimum
                     } else {
                         write_hit(out, r, lb, qlen);
