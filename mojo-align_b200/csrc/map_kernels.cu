@@ -1,6 +1,6 @@
 // map_kernels.cu - the mapping kernels of the linear bisulfite FM path.
 //
-//   pack_reads_kernel     _cvt + pack_bases_kernel
+//   pack_rows_kernel      _cvt + pack_bases_kernel
 //                         (linear_fastq.mojo:37-46, linear_gpu_fm.mojo:1136-1154),
 //                         fused into a 2-bit packing of both strands
 //   seed_extend_kernel    fm_seed_extend_kernel (linear_gpu_fm.mojo:1156-1837)
@@ -20,76 +20,34 @@ namespace ma {
 
 namespace {
 
-// Word w of packed read row `row` (len bases, conversion `mode`): forward
-// codes, reverse-complement codes and the two non-ACGT masks, each at
-// `words` stride from `out`.
-__device__ __forceinline__ void pack_word(const uint8_t* __restrict__ row, int len, int mode, int w, int words,
-                                          uint64_t* __restrict__ out) {
-    uint64_t f = 0, fn = 0, rw = 0, rn = 0;
-    for (int i = 0; i < 32; ++i) {
-        const int j = 32 * w + i;
-        if (j >= len) break;
-        const int c = code_of(cvt_base(row[j], mode));
-        if (c > 3) fn |= 1ull << (2 * i);
-        else f |= static_cast<uint64_t>(c) << (2 * i);
-        const int c2 = code_of(cvt_base(row[len - 1 - j], mode));
-        if (c2 > 3) rn |= 1ull << (2 * i);
-        else rw |= static_cast<uint64_t>(3 - c2) << (2 * i);
+// 2-bit codes (bits 0,2,..,30) and N flags (bits 0,2,..,30) of 16 ASCII
+// bases: A/a 0, C/c 1, G/g 2, T/t 3; the code of a byte that is no base is
+// to be ignored.  Bits 1-2 of the ASCII letters give the codes,
+// ((b >> 1) ^ (b >> 2)) & 3; a byte is a base exactly when its upper-case
+// form equals the letter of its code (a byte permute of "ACGT" by the
+// codes).  A product puts the fields of a word's four bytes side by side in
+// its top byte: every partial product has bits of its own, so nothing
+// carries.
+__device__ __forceinline__ void codes16(const uint32_t (&v)[4], uint32_t& codes, uint32_t& nflags) {
+    uint32_t pc[4], pn[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const uint32_t c = ((v[q] >> 1) ^ (v[q] >> 2)) & 0x03030303u;
+        const uint32_t pairs = c | (c >> 4);  // nibbles of bytes 0,1 in byte 0, of bytes 2,3 in byte 2
+        const uint32_t x = (v[q] & 0xDFDFDFDFu) ^ __byte_perm(0x54474341u, 0u, __byte_perm(pairs, 0u, 0x4420));
+        const uint32_t nz = (((x & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | x) & 0x80808080u;  // high bit: byte not a base
+        pc[q] = c * 0x01041040u;
+        pn[q] = (nz >> 7) * 0x01041040u;
     }
-    out[w] = f;
-    out[words + w] = rw;
-    out[2 * words + w] = fn;
-    out[3 * words + w] = rn;
+    codes = __byte_perm(__byte_perm(pc[0], pc[1], 0x0073), __byte_perm(pc[2], pc[3], 0x0073), 0x5410);
+    nflags = __byte_perm(__byte_perm(pn[0], pn[1], 0x0073), __byte_perm(pn[2], pn[3], 0x0073), 0x5410);
 }
 
-// Source row r (stride max_len) lands at batch row dst1 + r for the first
-// n1 rows and dst2 + (r - n1) after them; lens are read at the batch row.  A
-// plain batch uses dst1 = 0, dst2 = n1.
-__global__ void __launch_bounds__(256) pack_reads_kernel(const uint8_t* __restrict__ bases,
-                                                         const uint32_t* __restrict__ lens, int64_t n_seq,
-                                                         int64_t n1, int max_len, int words, int bs_r1,
-                                                         int bs_r2, int64_t dst1, int64_t dst2,
-                                                         uint64_t* __restrict__ packed, int* __restrict__ err) {
-    const int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    const int64_t r = t / words;
-    const int w = static_cast<int>(t - r * words);
-    if (r >= n_seq) return;
-    const int64_t d = r < n1 ? dst1 + r : dst2 + (r - n1);
-    int len = static_cast<int>(lens[d]);
-    if (len > max_len) {
-        atomicExch(err, 1);
-        len = max_len;
-    }
-    pack_word(bases + r * static_cast<int64_t>(max_len), len, r < n1 ? bs_r1 : bs_r2, w, words,
-              packed + d * 4 * static_cast<int64_t>(words));
-}
-
-// Four bases at base[x .. x+3] (reversed: base[x+3] first) from 4-byte
-// aligned loads; base must be 4-byte aligned.
-__device__ __forceinline__ uint32_t load4(const uint8_t* base, int x, bool reversed) {
-    const uint32_t* a = reinterpret_cast<const uint32_t*>(base + (x & ~3));
-    const uint32_t o = static_cast<uint32_t>(x & 3) * 0x1111u;
-    return __byte_perm(a[0], a[1], (reversed ? 0x0123u : 0x3210u) + o);
-}
-
-// 2-bit codes (bits 0,2,4,6) and N flags (bits 0,2,4,6) of four ASCII bases
-// after conversion `mode` (linear_fastq.mojo:37-46): A/a 0, C/c 1, G/g 2,
-// T/t 3 (C -> T under C2T, G -> A under G2A), anything else N (code 0).
-// Bits 1-2 of the ASCII letters give the codes, ((b >> 1) ^ (b >> 2)) & 3;
-// a byte is a base exactly when its upper-case form equals the letter of
-// its code (a byte permute of "ACGT" by the codes).
-__device__ __forceinline__ void codes4(uint32_t v, int mode, uint32_t& codes, uint32_t& nflags) {
-    const uint32_t u = v & 0xDFDFDFDFu;
-    uint32_t c = ((v >> 1) ^ (v >> 2)) & 0x03030303u;
-    const uint32_t sel = (c & 0x3u) | ((c >> 4) & 0x30u) | ((c >> 8) & 0x300u) | ((c >> 12) & 0x3000u);
-    const uint32_t x = u ^ __byte_perm(0x54474341u, 0u, sel);
-    const uint32_t nz = (((x & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | x) & 0x80808080u;  // high bit: byte not a base
-    if (mode == MA_BS_C2T) c |= (c & ~(c >> 1) & 0x01010101u) << 1;
-    if (mode == MA_BS_G2A) c &= ~(((c >> 1) & ~c & 0x01010101u) << 1);
-    const uint32_t nb = nz >> 7;
-    c &= ~(nb * 3u);
-    codes = (c & 0x3u) | ((c >> 6) & 0xCu) | ((c >> 12) & 0x30u) | ((c >> 18) & 0xC0u);
-    nflags = (nb & 0x1u) | ((nb >> 6) & 0x4u) | ((nb >> 12) & 0x10u) | ((nb >> 18) & 0x40u);
+// Fields p .. p+31 of a stream of 16 two-bit fields a word.
+__device__ __forceinline__ uint64_t fields32(const uint32_t* s, int p) {
+    const uint32_t* a = s + (p >> 4);
+    const int sh = 2 * (p & 15);
+    return __funnelshift_r(a[0], a[1], sh) | static_cast<uint64_t>(__funnelshift_r(a[1], a[2], sh)) << 32;
 }
 
 // Order of the 32 two-bit fields of a word reversed.
@@ -98,136 +56,151 @@ __device__ __forceinline__ uint64_t reverse_fields(uint64_t x) {
     return ((y >> 1) & kEven) | ((y & kEven) << 1);
 }
 
-// One packed read from a staged row (`row` = its offset in the 4-byte
-// aligned `base`): forward words from the bytes 4 bases at a time, then the
-// reverse-complement words from the forward ones (fields reversed, shifted
-// by 32 * ceil(len / 32) - len bases, complemented).  Reads may touch up to
-// 7 bytes after the row's last base.
-__device__ __forceinline__ void pack_row_staged(const uint8_t* base, int row, int len, int mode, int words,
-                                                uint64_t* __restrict__ out) {
-    const int wr = (len + 31) >> 5;     // words holding bases
-    const int sh = 2 * (32 * wr - len);  // bits the reversed stream is shifted by
-    uint64_t r_prev = 0, rn_prev = 0;    // reversed word j - 1
-    for (int k = wr - 1; k >= 0; --k) {  // j = wr - 1 - k ascending
-        uint64_t f = 0, fn = 0;
-        for (int g = 0; g < 8; ++g) {
-            if (32 * k + 4 * g >= len) break;
-            uint32_t c, n;
-            codes4(load4(base, row + 32 * k + 4 * g, false), mode, c, n);
-            f |= static_cast<uint64_t>(c) << (8 * g);
-            fn |= static_cast<uint64_t>(n) << (8 * g);
-        }
-        const int nv = len - 32 * k;
-        const uint64_t keep = nv >= 32 ? ~0ull : ((1ull << (2 * nv)) - 1);
-        f &= keep;
-        fn &= keep;
-        out[k] = f;
-        out[2 * words + k] = fn;
-        const uint64_t r = reverse_fields(f), rn = reverse_fields(fn);
-        const int j = wr - 1 - k;
-        if (j > 0) {
-            // reverse-complement word j - 1 from reversed words j - 1 and j
-            const uint64_t sr = sh ? ((r_prev >> sh) | (r << (64 - sh))) : r_prev;
-            const uint64_t sn = sh ? ((rn_prev >> sh) | (rn << (64 - sh))) : rn_prev;
-            out[words + j - 1] = (sr ^ ~0ull) & ~(sn * 3ull);
-            out[3 * words + j - 1] = sn;
-        }
-        r_prev = r;
-        rn_prev = rn;
-    }
-    if (wr > 0) {
-        const int nv = len - 32 * (wr - 1);
-        const uint64_t keep = nv >= 32 ? ~0ull : ((1ull << (2 * nv)) - 1);
-        const uint64_t sr = r_prev >> sh, sn = rn_prev >> sh;
-        out[words + wr - 1] = (sr ^ ~0ull) & ~(sn * 3ull) & keep;
-        out[3 * words + wr - 1] = sn & keep;
-    }
-    for (int w = wr; w < words; ++w) {
-        out[w] = 0;
-        out[words + w] = 0;
-        out[2 * words + w] = 0;
-        out[3 * words + w] = 0;
-    }
+// Word j of the field-reversed stream of a row's wr forward words: reversed
+// words j and j + 1 of the row, joined at the sh = 2 * (32 * wr - len) bits
+// that the last forward word leaves empty.
+__device__ __forceinline__ uint64_t reversed_word(const uint64_t* fwd, int wr, int sh, int j) {
+    const uint64_t lo = reverse_fields(fwd[wr - 1 - j]) >> sh;
+    return sh && j + 1 < wr ? lo | (reverse_fields(fwd[wr - 2 - j]) << (64 - sh)) : lo;
 }
 
-// Staged form of pack_reads_kernel: a block copies the bytes of its rows
-// (one contiguous range of the row-major input) into shared memory with
-// 16-byte loads, then packs one row per thread from there.
-// rows_per_block * max_len must fit PACK_STAGE bytes.
+// Packs PackParts (a plain batch is one part with block0 = 0).  Part j
+// holds c pairs (or single reads) staged at byte `src` of `bases`: its c
+// first mates, then its c second mates, rows of stride max_len.  Its pair i
+// lands at batch row dst + i and, when paired, n1_batch + dst + i; lens are
+// read at the batch row.  A block takes rows_per_block rows of one part.
+// Their bytes are one contiguous range: a thread codes 16 of them at a time
+// into a stream of 2-bit fields in shared memory.  A thread then takes a
+// forward word of 32 bases from the stream and applies the row's conversion
+// (linear_fastq.mojo:37-46: C -> T under C2T, G -> A under G2A), a thread
+// derives a reverse-complement word from two forward ones, and the finished
+// rows, one contiguous range again (two where the block spans both mates),
+// leave with 16-byte stores.
+//
+// Bound by DRAM and the issue of the byte work (about 20 instructions for
+// four bases).  Work is split by word, not by row: uneven rows hold up no
+// warp, shared memory is read without conflicts (whole words at a stride of
+// a row's bytes cost 8 passes a load: 487 us below) and the stores are
+// coalesced.  2 M rows of 300 bytes 369 us (3.4 TB/s; 674 with a thread for
+// a row), 800 k rows of 250 118 us (228), serving groups of 400 k rows of
+// 150 109 us (561 with a thread for a word read byte by byte).
 constexpr int PACK_THREADS = 256;
-constexpr int PACK_STAGE = 40960;
-constexpr int PACK_SLACK = 16;  // before and after the staged bytes
+constexpr int PACK_SHARED = 24576;  // bytes that a block's streams and packed rows take together
+
+// words of a stream of rows * max_len bases: up to 15 fields before the
+// first, two words read past the last
+__host__ __device__ constexpr int pack_stream_words(int rows, int max_len) {
+    return ((rows * max_len + 30) / 16 + 2 + 3) & ~3;
+}
 
 __global__ void __launch_bounds__(PACK_THREADS) pack_rows_kernel(const uint8_t* __restrict__ bases,
-                                                                const uint32_t* __restrict__ lens, int64_t n_seq,
-                                                                int64_t n1, int max_len, int words,
-                                                                int rows_per_block, int bs_r1, int bs_r2,
-                                                                int64_t dst1, int64_t dst2,
+                                                                const uint32_t* __restrict__ lens,
+                                                                const PackPart* __restrict__ parts, int n_parts,
+                                                                PackPart one, int paired, int64_t n1_batch,
+                                                                int words, int rows_per_block,
                                                                 uint64_t* __restrict__ packed,
                                                                 int* __restrict__ err) {
-    __shared__ __align__(16) uint8_t s_rows[PACK_SLACK + PACK_STAGE + 16 + PACK_SLACK];
-    const int64_t r0 = static_cast<int64_t>(blockIdx.x) * rows_per_block;
-    if (r0 >= n_seq) return;
-    const int nr = static_cast<int>(n_seq - r0 < rows_per_block ? n_seq - r0 : rows_per_block);
-    const uint8_t* g = bases + r0 * static_cast<int64_t>(max_len);
-    const int bytes = nr * max_len;
-    // s_rows[PACK_SLACK + off + j] = g[j]; off lines up the 16-byte
-    // boundaries of g with those of s_rows
-    const int off = static_cast<int>(reinterpret_cast<uintptr_t>(g) & 15);
-    const int head = off ? (16 - off < bytes ? 16 - off : bytes) : 0;
-    const int n16 = (bytes - head) >> 4;
-    uint8_t* st = s_rows + PACK_SLACK + off;
-    for (int j = threadIdx.x; j < head; j += blockDim.x) st[j] = g[j];
-    const uint4* g16 = reinterpret_cast<const uint4*>(g + head);
-    uint4* s16 = reinterpret_cast<uint4*>(st + head);
-    for (int k = threadIdx.x; k < n16; k += blockDim.x) s16[k] = __ldg(g16 + k);
-    for (int j = head + 16 * n16 + threadIdx.x; j < bytes; j += blockDim.x) st[j] = g[j];
-    __syncthreads();
-    for (int lr = threadIdx.x; lr < nr; lr += blockDim.x) {
-        const int64_t r = r0 + lr;
-        const int64_t d = r < n1 ? dst1 + r : dst2 + (r - n1);
-        int len = static_cast<int>(lens[d]);
+    __shared__ __align__(16) uint8_t s_mem[PACK_SHARED];
+    __shared__ int s_len[PACK_THREADS];
+    PackPart pp = one;
+    if (parts) {  // last part with block0 <= this block
+        int lo = 0, hi = n_parts - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (parts[mid].block0 <= blockIdx.x) lo = mid;
+            else hi = mid - 1;
+        }
+        pp = parts[lo];
+    }
+    const int max_len = static_cast<int>(pp.max_len);
+    const int64_t r0 = static_cast<int64_t>(blockIdx.x - pp.block0) * rows_per_block;
+    const int64_t rows = paired ? 2 * static_cast<int64_t>(pp.c) : pp.c;
+    if (r0 >= rows) return;
+    const int nr = static_cast<int>(rows - r0 < rows_per_block ? rows - r0 : rows_per_block);
+    // local rows [0, cut) are first mates at batch rows d1 + lr, the rest
+    // second mates at d2 + lr
+    const int64_t left = static_cast<int64_t>(pp.c) - r0;
+    const int cut = static_cast<int>(left < 0 ? 0 : left < nr ? left : nr);
+    const int64_t d1 = static_cast<int64_t>(pp.dst) + r0;
+    const int64_t d2 = n1_batch + pp.dst + (r0 - pp.c);
+    if (static_cast<int>(threadIdx.x) < nr) {
+        const int lr = threadIdx.x;
+        int len = static_cast<int>(lens[(lr < cut ? d1 : d2) + lr]);
         if (len > max_len) {
             atomicExch(err, 1);
             len = max_len;
         }
-        pack_row_staged(s_rows, PACK_SLACK + off + lr * max_len, len, r < n1 ? bs_r1 : bs_r2, words,
-                        packed + d * 4 * static_cast<int64_t>(words));
+        s_len[lr] = len;
     }
-}
-
-// A batch merged from several requests.  Part j holds c pairs (or single
-// reads) staged at byte `src` of `bases`: its c first mates, then its c
-// second mates, rows of stride max_len.  Its pair i lands at batch row
-// dst + i and, when paired, n1_batch + dst + i.  Source rows of all parts
-// are numbered consecutively from 0 (part j's first row is row0).
-__global__ void __launch_bounds__(256) pack_parts_kernel(const uint8_t* __restrict__ bases,
-                                                         const uint32_t* __restrict__ lens,
-                                                         const PackPart* __restrict__ parts, int n_parts,
-                                                         int64_t n_rows, int64_t n1_batch, int words,
-                                                         uint64_t* __restrict__ packed, int* __restrict__ err) {
-    const int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    const int64_t r = t / words;
-    const int w = static_cast<int>(t - r * words);
-    if (r >= n_rows) return;
-    int lo = 0, hi = n_parts - 1;  // last part with row0 <= r
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (parts[mid].row0 <= r) lo = mid;
-        else hi = mid - 1;
+    const int n_stream = pack_stream_words(rows_per_block, max_len);
+    uint32_t* s_code = reinterpret_cast<uint32_t*>(s_mem);  // base j of the range at field off + j
+    uint32_t* s_n = s_code + n_stream;
+    uint64_t* s_out = reinterpret_cast<uint64_t*>(s_n + n_stream);
+    const uint8_t* g = bases + pp.src + r0 * max_len;
+    const int bytes = nr * max_len;
+    const int off = static_cast<int>(reinterpret_cast<uintptr_t>(g) & 15);
+    const int chunks = (off + bytes + 15) >> 4;
+#pragma unroll 2
+    for (int c = threadIdx.x; c < chunks; c += PACK_THREADS) {
+        const int j = 16 * c - off;  // first byte of the aligned 16
+        uint32_t v[4] = {0, 0, 0, 0};
+        if (j >= 0 && j + 16 <= bytes) {
+            const uint4 x = __ldcs(reinterpret_cast<const uint4*>(g + j));
+            v[0] = x.x;
+            v[1] = x.y;
+            v[2] = x.z;
+            v[3] = x.w;
+        } else {
+            for (int i = 0; i < 16; ++i)
+                if (j + i >= 0 && j + i < bytes) v[i >> 2] |= static_cast<uint32_t>(g[j + i]) << (8 * (i & 3));
+        }
+        codes16(v, s_code[c], s_n[c]);
     }
-    const PackPart pp = parts[lo];
-    const int64_t local = r - pp.row0;
-    const bool second = local >= pp.c;
-    const int64_t i = second ? local - pp.c : local;
-    const int64_t d = second ? n1_batch + pp.dst + i : pp.dst + i;
-    int len = static_cast<int>(lens[d]);
-    if (len > static_cast<int>(pp.max_len)) {
-        atomicExch(err, 1);
-        len = static_cast<int>(pp.max_len);
+    __syncthreads();
+    const int items = nr * words;  // below 2^13, so t / words is exact as a product
+    const uint32_t inv = (1u << 18) / static_cast<uint32_t>(words) + 1;
+    for (int t = threadIdx.x; t < items; t += PACK_THREADS) {
+        const int lr = static_cast<int>((static_cast<uint32_t>(t) * inv) >> 18), k = t - lr * words;
+        const int nv = s_len[lr] - 32 * k;  // bases of this word
+        uint64_t f = 0, fn = 0;
+        if (nv > 0) {
+            const int mode = lr < cut ? pp.bs_r1 : pp.bs_r2;
+            const int p = off + lr * max_len + 32 * k;
+            const uint64_t keep = nv >= 32 ? ~0ull : ((1ull << (2 * nv)) - 1);
+            f = fields32(s_code, p);
+            fn = fields32(s_n, p) & keep;
+            if (mode == MA_BS_C2T) f |= (f & ~(f >> 1) & kEven) << 1;
+            if (mode == MA_BS_G2A) f &= ~(((f >> 1) & ~f & kEven) << 1);
+            f &= keep & ~(fn * 3ull);
+        }
+        uint64_t* o = s_out + lr * 4 * words + k;
+        o[0] = f;
+        o[2 * words] = fn;
     }
-    pack_word(bases + pp.src + local * static_cast<int64_t>(pp.max_len), len, second ? pp.bs_r2 : pp.bs_r1, w,
-              words, packed + d * 4 * static_cast<int64_t>(words));
+    __syncthreads();
+    for (int t = threadIdx.x; t < items; t += PACK_THREADS) {
+        const int lr = static_cast<int>((static_cast<uint32_t>(t) * inv) >> 18), j = t - lr * words;
+        const int len = s_len[lr];
+        const int wr = (len + 31) >> 5;  // words holding bases
+        uint64_t r = 0, rn = 0;
+        uint64_t* o = s_out + lr * 4 * words;
+        if (j < wr) {
+            const int sh = 2 * (32 * wr - len);
+            const int nv = len - 32 * j;
+            rn = reversed_word(o + 2 * words, wr, sh, j);
+            r = ~reversed_word(o, wr, sh, j) & ~(rn * 3ull);
+            if (nv < 32) r &= (1ull << (2 * nv)) - 1;
+        }
+        o[words + j] = r;
+        o[3 * words + j] = rn;
+    }
+    __syncthreads();
+    // a packed row is 2 * words 16-byte pieces
+    const int pieces = 2 * words;
+    const uint4* s = reinterpret_cast<const uint4*>(s_out);
+    uint4* o1 = reinterpret_cast<uint4*>(packed) + d1 * pieces;
+    uint4* o2 = reinterpret_cast<uint4*>(packed) + d2 * pieces;
+    for (int t = threadIdx.x; t < nr * pieces; t += PACK_THREADS) (t < cut * pieces ? o1 : o2)[t] = s[t];
 }
 
 // Stage 1: one thread per read, right endpoints [0, ep_limit).  A read
@@ -634,29 +607,36 @@ unsigned grid_for(int64_t n, int block) {
 
 }  // namespace
 
+// Rows that one block of pack_rows_kernel takes: what fits its shared
+// memory (15 rows of 1024 bases, 104 of 150), no more than a thread each.
+int pack_rows_per_block(int max_len, int words) {
+    const int rows = (PACK_SHARED - 64) / ((max_len + 1) / 2 + 32 * words);
+    return rows < PACK_THREADS ? rows : PACK_THREADS;
+}
+
 // Host launchers (stream-ordered).  Returns the number of kernels launched.
 int launch_pack(const uint8_t* d_bases, const uint32_t* d_lens, int64_t n_seq, int64_t n1, int max_len, int words,
                 int bs_r1, int bs_r2, uint64_t* d_packed, int* d_err, cudaStream_t st) {
-    int rows = PACK_STAGE / max_len;
-    if (rows > PACK_THREADS) rows = PACK_THREADS;
-    if (rows >= 1) {
-        pack_rows_kernel<<<grid_for(n_seq, rows), PACK_THREADS, 0, st>>>(d_bases, d_lens, n_seq, n1, max_len, words,
-                                                                        rows, bs_r1, bs_r2, 0, n1, d_packed, d_err);
-    } else {  // rows longer than the stage
-        const int64_t n = n_seq * words;
-        pack_reads_kernel<<<grid_for(n, 256), 256, 0, st>>>(d_bases, d_lens, n_seq, n1, max_len, words, bs_r1,
-                                                            bs_r2, 0, n1, d_packed, d_err);
-    }
+    PackPart one{};
+    one.c = static_cast<uint32_t>(n1);
+    one.max_len = static_cast<uint32_t>(max_len);
+    one.bs_r1 = bs_r1;
+    one.bs_r2 = bs_r2;
+    const int rows = pack_rows_per_block(max_len, words);
+    pack_rows_kernel<<<grid_for(n_seq, rows), PACK_THREADS, 0, st>>>(d_bases, d_lens, nullptr, 0, one, n_seq > n1,
+                                                                    n1, words, rows, d_packed, d_err);
     return 1;
 }
 
-// Packs the parts of a merged batch (see pack_parts_kernel); d_lens is the
-// batch's length array, already at the batch rows.
+// Packs the parts of a merged batch (see pack_rows_kernel), n_blocks blocks
+// of `rows` rows (pack_rows_per_block of the longest part) in all; d_lens is
+// the batch's length array, already at the batch rows.
 int launch_pack_parts(const uint8_t* d_bases, const uint32_t* d_lens, const PackPart* d_parts, int n_parts,
-                      int64_t n_rows, int64_t n1_batch, int words, uint64_t* d_packed, int* d_err, cudaStream_t st) {
-    const int64_t n = n_rows * words;
-    pack_parts_kernel<<<grid_for(n, 256), 256, 0, st>>>(d_bases, d_lens, d_parts, n_parts, n_rows, n1_batch, words,
-                                                        d_packed, d_err);
+                      uint32_t n_blocks, int rows, bool paired, int64_t n1_batch, int words, uint64_t* d_packed,
+                      int* d_err, cudaStream_t st) {
+    if (n_blocks == 0) return 0;
+    pack_rows_kernel<<<n_blocks, PACK_THREADS, 0, st>>>(d_bases, d_lens, d_parts, n_parts, PackPart{}, paired ? 1 : 0,
+                                                       n1_batch, words, rows, d_packed, d_err);
     return 1;
 }
 
@@ -794,7 +774,6 @@ int launch_rescue(const DevIndex& ix, const DevReads& R, const DevParams& P, con
 void load_noalloc_kernels(int level) {
     cudaFuncAttributes a;
     cudaFuncGetAttributes(&a, pack_rows_kernel);
-    cudaFuncGetAttributes(&a, pack_reads_kernel);
     cudaFuncGetAttributes(&a, mate_rescue_kernel);
     if (level == 1) {
         cudaFuncGetAttributes(&a, seed_stage1_kernel<false, SeedKernels<false, 1>::B1>);

@@ -36,7 +36,9 @@ const DevIndex* index_device_view(const ma_index* idx, int* device);
 void ctx_launch_config(const ma_ctx* ctx, int* device, int* sm_count, ma_tuning* tuning);
 void set_thread_error(const std::string& msg);
 int launch_pack_parts(const uint8_t* d_bases, const uint32_t* d_lens, const PackPart* d_parts, int n_parts,
-                      int64_t n_rows, int64_t n1_batch, int words, uint64_t* d_packed, int* d_err, cudaStream_t st);
+                      uint32_t n_blocks, int rows, bool paired, int64_t n1_batch, int words, uint64_t* d_packed,
+                      int* d_err, cudaStream_t st);
+int pack_rows_per_block(int max_len, int words);
 int launch_seed_extend(const DevIndex& ix, const DevReads& R, const DevParams& P, const DevOut& out,
                        unsigned long long* d_tally, int level, cudaStream_t st);
 size_t two_stage_scratch_bytes(int64_t n_seq);
@@ -295,7 +297,8 @@ void issue_group(ma_server* s, Group& g) {
     const uint64_t out_bytes = 7 * out_stride + sizeof(int);
     if (in_bytes > hs.in_cap || out_bytes > hs.out_cap) fail(MA_ERR_INTERNAL, "group exceeds its host staging");
     cudaStream_t st = s->test_mode ? nullptr : s->streams[static_cast<size_t>(g.slot)];
-    int64_t row0 = 0;
+    const int pack_rows = pack_rows_per_block(32 * g.words, g.words);
+    uint32_t block0 = 0;
     for (size_t j = 0; j < g.parts.size(); ++j) {
         const Part& pt = g.parts[j];
         const Request& rq = *pt.rq;
@@ -304,14 +307,14 @@ void issue_group(ma_server* s, Group& g) {
         if (g.paired) std::memcpy(hl + g.n1 + pt.dst, rq.lens + rq.n1 + pt.a, pt.c * 4ull);
         PackPart pp{};
         pp.src = pt.src;
-        pp.row0 = row0;
+        pp.block0 = block0;
         pp.c = pt.c;
         pp.max_len = rq.max_len;
         pp.bs_r1 = rq.bs_r1;
         pp.bs_r2 = rq.bs_r2;
         pp.dst = pt.dst;
         hp[j] = pp;
-        row0 += static_cast<int64_t>(pt.c) * rq.mates();
+        block0 += static_cast<uint32_t>((static_cast<int64_t>(pt.c) * rq.mates() + pack_rows - 1) / pack_rows);
         const uint8_t* r1 = rq.bases + static_cast<size_t>(pt.a) * rq.max_len;
         const uint8_t* r2 = rq.bases + (static_cast<size_t>(rq.n1) + pt.a) * rq.max_len;
         if (s->test_mode) {
@@ -338,8 +341,8 @@ void issue_group(ma_server* s, Group& g) {
     const uint32_t* d_lens = reinterpret_cast<const uint32_t*>(dev + g.L.lens);
     int* d_err = reinterpret_cast<int*>(dev + g.L.err);
     launch_pack_parts(reinterpret_cast<const uint8_t*>(dev + g.L.bases), d_lens,
-                      reinterpret_cast<const PackPart*>(dev + g.L.parts), static_cast<int>(g.parts.size()), row0, g.n1,
-                      g.words, packed, d_err, st);
+                      reinterpret_cast<const PackPart*>(dev + g.L.parts), static_cast<int>(g.parts.size()), block0,
+                      pack_rows, g.paired, g.n1, g.words, packed, d_err, st);
     DevReads R{packed, d_lens, g.words, n_seq};
     DevOut o{reinterpret_cast<int32_t*>(dev + g.L.out[0]), reinterpret_cast<uint32_t*>(dev + g.L.out[1]),
              reinterpret_cast<uint32_t*>(dev + g.L.out[2]), reinterpret_cast<int32_t*>(dev + g.L.out[3]),

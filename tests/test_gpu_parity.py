@@ -333,3 +333,39 @@ def test_default_rounds_at_every_batch_size(ctx, small_ref, n1, paired, max_len)
     fa, prefix = small_ref
     rb = sim(fa, n1, paired, max_len=max_len, seed=n1, len_fixed=max_len)
     compare(prefix, ctx, rb.bases, rb.lens, n1, paired, max_len, BENCH_PARAMS, tunings=[()])
+
+
+@pytest.mark.parametrize("max_len,n1,skew", [(1, 3, 0), (31, 300, 1), (33, 257, 7), (150, 104, 13), (151, 73, 0),
+                                             (250, 1000, 8), (1024, 15, 15), (1023, 32, 3)])
+def test_packed_rows_at_block_edges(ctx, small_ref, max_len, n1, skew):
+    """Pairs whose mates meet inside a block's rows, every length from 0 to
+    max_len, bytes of both cases and of no base, at each alignment of the
+    first row; a block packs up to 256 rows (104 of 150 bases, 15 of 1024)."""
+    torch = pytest.importorskip("torch")
+    from mojoalign_b200 import MapResult, map_batch_device
+
+    fa, prefix = small_ref
+    rb = sim(fa, n1, True, max_len=max(max_len, 40), seed=max_len, len_fixed=max(max_len, 40))
+    bases = np.ascontiguousarray(rb.bases.reshape(2 * n1, -1)[:, :max_len])
+    rng = np.random.default_rng(max_len)
+    low = rng.random(bases.shape) < 0.1
+    bases[low] |= 0x20
+    other = rng.random(bases.shape) < 0.002
+    bases[other] = rng.integers(0, 256, int(other.sum()), dtype=np.uint8)
+    lens = (max_len - (np.arange(2 * n1) * 7) % (max_len + 1)).astype(np.uint32)
+    lens[::3] = max_len
+    o = oracle.OracleIndex(prefix).map(bases.reshape(-1), lens, n1, True, max_len, 1, 2, BENCH_PARAMS.as_list())
+    gi = gpu_index(ctx, prefix, 12, 12)
+    buf = torch.zeros(bases.size + 16, dtype=torch.uint8, device="cuda")
+    d_bases = buf[skew:skew + bases.size]
+    d_bases.copy_(torch.from_numpy(bases.reshape(-1)))
+    d_lens = torch.from_numpy(lens.view(np.int32)).cuda()
+    out = {f: torch.zeros(2 * n1, dtype=torch.int32, device="cuda") for f in MapResult.FIELDS}
+    torch.cuda.synchronize()
+    map_batch_device(ctx, gi, d_bases.data_ptr(), d_lens.data_ptr(), n1, True, max_len,
+                     {f: t.data_ptr() for f, t in out.items()}, 1, 2, BENCH_PARAMS,
+                     stream=torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    for f in MapResult.FIELDS:
+        got = out[f].cpu().numpy().view(o[f].dtype)
+        assert np.array_equal(got, o[f]), f
