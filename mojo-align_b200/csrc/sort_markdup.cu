@@ -9,8 +9,8 @@
 // records on the host.  Here everything stays in HBM:
 //   - the three stable 64-bit key sorts (coordinate; dlo, then dhi carried
 //     into that order) are LSD radix sorts of 8-bit digits carrying u32
-//     record indices (radix_sort.cuh; digits that are equal in every key
-//     are skipped); a stable LSD sort gives exactly the reference's order,
+//     record indices (radix_sort.cuh; bits that decide no order are
+//     skipped); a stable LSD sort gives exactly the reference's order,
 //     ties broken by record index;
 //   - mark_dups_kernel: one thread per position of the duplicate-key order;
 //     the first record of every run of equal (dhi, dlo) walks its run, picks
@@ -58,14 +58,17 @@ __global__ void mark_dups_kernel(const uint64_t* sdhi, const uint32_t* merged, c
     const uint64_t i = static_cast<uint64_t>(blockIdx.x) * THREADS + threadIdx.x;
     if (i >= n) return;
     const uint64_t h = sdhi[i];
-    const uint64_t l = dlo[merged[i]];
-    if (i > 0 && sdhi[i - 1] == h && dlo[merged[i - 1]] == l) return;  // not the first of its run
-    uint64_t end = i + 1;
-    while (end < n && sdhi[end] == h && dlo[merged[end]] == l) ++end;
-    if (h == ~0ull) {  // unplaced records are never duplicates
-        for (uint64_t j = i; j < end; ++j) is_dup[merged[j]] = 0;
+    const bool after = i > 0 && sdhi[i - 1] == h, more = i + 1 < n && sdhi[i + 1] == h;
+    // unplaced records are never duplicates, nor is one that no neighbour
+    // shares its upper key with: nothing is gathered for it
+    if (h == ~0ull || (!after && !more)) {
+        is_dup[merged[i]] = 0;
         return;
     }
+    const uint64_t l = dlo[merged[i]];
+    if (after && dlo[merged[i - 1]] == l) return;  // not the first of its run
+    uint64_t end = i + 1;
+    while (end < n && sdhi[end] == h && dlo[merged[end]] == l) ++end;
     uint32_t best_pair = pair[merged[i]], best_score = score[merged[i]];
     for (uint64_t j = i; j < end; ++j) {
         const uint32_t o = merged[j];
@@ -225,12 +228,10 @@ int enqueue_sort_markdup(const SortDev& s, void* scratch, size_t scratch_bytes, 
     int launches = 0;
     if (s.marked) check_launch(cudaMemsetAsync(s.marked, 0, sizeof(unsigned long long), st), "memset");
     // coordinate order (L469-525)
-    iota_kernel<<<grid_for(n), THREADS, 0, st>>>(sc.idx_a, n);
-    launches += 1 + radix_sort(sc, s.coord, sc.keys_out, sc.idx_a, s.perm, n, st);
+    launches += radix_sort(sc, s.coord, sc.keys_out, nullptr, s.perm, n, st);
     if (s.do_markdup) {
         // duplicate-key order: dlo, then dhi carried along (L311-360)
-        iota_kernel<<<grid_for(n), THREADS, 0, st>>>(sc.idx_a, n);
-        launches += 1 + radix_sort(sc, s.dlo, sc.keys_out, sc.idx_a, sc.idx_b, n, st);
+        launches += radix_sort(sc, s.dlo, sc.keys_out, nullptr, sc.idx_b, n, st);
         permute_kernel<<<grid_for(n), THREADS, 0, st>>>(s.dhi, sc.idx_b, sc.key2, n);
         uint32_t* merged = s.dup_perm ? s.dup_perm : sc.idx_a;
         launches += 1 + radix_sort(sc, sc.key2, sc.keys_out, sc.idx_b, merged, n, st);

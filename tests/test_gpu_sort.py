@@ -173,3 +173,28 @@ def test_gather_copies_records_of_every_size_and_phase(ctx, n):
         want.append(r)
     got = gather_sorted(ctx, chunks, tile, SortResult(dup, perm, None, 0))
     np.testing.assert_array_equal(got, np.concatenate(want))
+
+
+@pytest.mark.parametrize("mask", [0x5555555555555555, 0x8000000000000001, 0x0FF0000000000FF0, 0x00000000000001FF,
+                                  0xFFFFFFFF00000000])
+@pytest.mark.parametrize("n", [33, 4096, 12_289])
+def test_sort_by_any_set_of_bits(ctx, mask, n):
+    """Bits in runs of every kind, and upper bits that are all set in the
+    unplaced records (where they follow one another), give the stable order."""
+    rng = np.random.default_rng(n)
+    m = random_tile_meta(3, n, dup_rate=0.3)
+    key = rng.integers(0, 2**64 - 1, n, dtype=np.uint64, endpoint=True) & np.uint64(mask)
+    key[rng.random(n) < 0.2] |= np.uint64(0xFFFFFF0000000000)
+    m["coord"] = key
+    # neighbours that share the upper duplicate key and not the lower one, and unplaced records
+    m["dhi"] = rng.integers(0, n // 8 + 2, n, dtype=np.uint64) << np.uint64(17)
+    m["dlo"] = rng.integers(0, 3, n, dtype=np.uint64) << np.uint64(40)
+    un = rng.random(n) < 0.25
+    m["dhi"][un] = np.uint64(2**64 - 1)
+    m["dlo"][un] = np.nonzero(un)[0] // 2
+    want = oracle.sort_markdup(**m)
+    got = sort_markdup(ctx, _tile(m), dup_perm=True)
+    np.testing.assert_array_equal(got.perm, np.argsort(key, kind="stable").astype(np.uint32))
+    np.testing.assert_array_equal(got.is_dup, want[0])
+    np.testing.assert_array_equal(got.dup_perm, want[2])
+    assert got.n_marked == want[3]
