@@ -36,7 +36,7 @@ from concurrent.futures import ThreadPoolExecutor
 
 import numpy as np
 
-from . import pinned
+from . import pinned, streams
 from .fqio import ParallelWriter, open_fastq
 from ._lib import (MA_FASTQ_RULES_STREAM, check, lib, ma_bam_meta, ma_bam_tile, ma_fastq_arena, ma_fastq_records,
                    ma_hits)
@@ -131,7 +131,7 @@ class _DeviceFeed:
         self.fh = open(path, "rb")
         self.cap = chunk
         self.dev = torch.empty(chunk + 16, dtype=torch.uint8, device=torch.device("cuda", ctx.device))
-        self.stream = torch.cuda.Stream(device=self.dev.device)
+        self.stream = streams.take(self.dev.device)
         # compressed bytes of one fill at most a quarter of the piece (BGZF
         # members inflate to at most 64 KB; FASTQ compresses 2-4x)
         self._cbuf = pinned.take(max(chunk // 4, 1 << 20))
@@ -257,6 +257,8 @@ class _DeviceFeed:
             self._tail.close()
         pinned.give(self._cbuf)
         self._cbuf = None
+        self.stream.synchronize()
+        streams.give(self.stream)
 
 
 class _Grow:
@@ -303,6 +305,13 @@ def _feed(path: str, chunk: int, torch, ctx, device_inflate: bool):
     return _Feed(path, chunk, torch)
 
 
+def _wait(jobs: list):
+    """Waits for all of `jobs`, then raises the first one's exception."""
+    for e in [j.exception() for j in jobs]:
+        if e is not None:
+            raise e
+
+
 def mapped_chunks(ctx, index, params, fq1, fq2, bs_r1, bs_r2, rules, batch_pairs, chunk_bytes, stream, tm,
                   before_map=None, device_inflate: bool = True):
     """Yields MappedChunk for consecutive pieces of the FASTQ file(s): the
@@ -325,17 +334,27 @@ def mapped_chunks(ctx, index, params, fq1, fq2, bs_r1, bs_r2, rules, batch_pairs
     feeds = [_feed(str(fq1), chunk_bytes, torch, ctx, device_inflate)] + (
         [_feed(str(fq2), chunk_bytes, torch, ctx, device_inflate)] if paired else [])
     tm.setdefault("fastq_h2d_bytes", 0)
-    pool = ThreadPoolExecutor(max_workers=1)  # reads the next piece while the GPU maps this one
-    pending = None
+    # reads the next piece while the GPU maps this one: host readers side by
+    # side, device inflation (which shares the context) one file at a time
+    pool = ThreadPoolExecutor(max_workers=len(feeds))
+    inflating = [f for f in feeds if isinstance(f, _DeviceFeed)]
+    reading = [[f] for f in feeds if not isinstance(f, _DeviceFeed)]
+    jobs = ([inflating] if inflating else []) + reading
+    pending = []
+
+    def refill(job, used):
+        for f in job:
+            f.consume(used[f])
+            f.fill()
+
     o3 = (C.c_uint64 * 3)()
     try:
-        for f in feeds:
+        pending = [pool.submit(f.fill) for f, in reading]
+        for f in inflating:
             f.fill()
         while True:
             t0 = time.perf_counter()
-            if pending is not None:
-                pending.result()
-                pending = None
+            _wait(pending)
             tm["read_wait"] += time.perf_counter() - t0
             if not feeds[0].len:
                 return
@@ -382,13 +401,7 @@ def mapped_chunks(ctx, index, params, fq1, fq2, bs_r1, bs_r2, rules, batch_pairs
                     u = int(o3[1])
                 used.append(u)
             stream.synchronize()
-
-            def refill(used=used):
-                for f, u in zip(feeds, used):
-                    f.consume(u)
-                    f.fill()
-
-            pending = pool.submit(refill)
+            pending = [pool.submit(refill, job, dict(zip(feeds, used))) for job in jobs]
             max_len = max(max(c[2] for c in counts), params.seed_len)
             if max_len > MAX_LEN_CAP:
                 raise RuntimeError("read longer than FM base cap (1024)")
@@ -413,8 +426,8 @@ def mapped_chunks(ctx, index, params, fq1, fq2, bs_r1, bs_r2, rules, batch_pairs
             yield chunk
             del chunk, d_buf, rows, lens, out
     finally:
-        if pending is not None:
-            pending.exception()
+        for job in pending:
+            job.exception()
         pool.shutdown(wait=True)
         for f in feeds:
             if isinstance(f, _DeviceFeed):
@@ -453,7 +466,7 @@ def map_fastq_to_bam(ref_fa, fq1, out_bam, device: str = "auto", fq2: str = "", 
         index = GpuIndex(ctx, fm_prefix_from_ref(ref_fa), kmer_k=min(kmer_k, params.seed_len), kmer3_k=k3)
     paired = len(str(fq2)) > 0
     dev = torch.device("cuda", ctx.device)
-    stream = torch.cuda.Stream(device=dev)
+    stream = streams.take(dev)
     sh = stream.cuda_stream
     rg = _env(env, "METHYLGRAPHER_RG_ID", "mojo1").encode("ascii")
     d_rg = torch.tensor(list(rg) or [0], dtype=torch.uint8, device=dev)
@@ -549,6 +562,7 @@ def map_fastq_to_bam(ref_fa, fq1, out_bam, device: str = "auto", fq2: str = "", 
         pieces.close()
         stream.synchronize()
         scope.close()
+        streams.give(stream)
         if own_index:
             index.close()
         if own_ctx:

@@ -25,7 +25,7 @@ import ctypes as C
 import os
 from concurrent.futures import ThreadPoolExecutor
 
-from . import pinned
+from . import pinned, streams
 from ._lib import MA_FASTQ_RULES_PAIR_READER, check, lib
 from .fq2bam import mapped_chunks
 from .fqio import ParallelWriter
@@ -63,7 +63,7 @@ def map_fastq_to_sam(ref_fa, fq1, out_sam, device: str = "auto", fq2: str = "", 
         index = GpuIndex(ctx, fm_prefix_from_ref(ref_fa), kmer_k=min(kmer_k, params.seed_len), kmer3_k=k3)
     paired = len(str(fq2)) > 0
     dev = torch.device("cuda", ctx.device)
-    stream = torch.cuda.Stream(device=dev)
+    stream = streams.take(dev)
     sh = stream.cuda_stream
     rg = _env_str("METHYLGRAPHER_RG_ID", "mojo1", env).encode()
     d_rg = torch.tensor(list(rg) or [0], dtype=torch.uint8, device=dev)
@@ -141,6 +141,7 @@ def map_fastq_to_sam(ref_fa, fq1, out_sam, device: str = "auto", fq2: str = "", 
             pinned.give(t)
         stream.synchronize()
         scope.close()
+        streams.give(stream)
         if own_index:
             index.close()
         if own_ctx:
