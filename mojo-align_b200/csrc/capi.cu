@@ -129,8 +129,10 @@ struct ma_ctx {
     static constexpr int NSLOT = 3;  // chunks whose host copies are in flight
     cudaEvent_t h2d_done[NSLOT] = {}, slot_free[NSLOT] = {}, comp_done[NSLOT] = {};
     struct Slot {
-        DevBuf bases, lens, out[12];
-        HostBuf h_lens, h_out[12];  // staging of pageable caller arrays
+        // hits: the 7 hit arrays of a chunk one after the other; debug: the
+        // 5 optional ones.  h_*: staging of pageable caller arrays.
+        DevBuf bases, lens, hits, debug[5];
+        HostBuf h_lens, h_hits, h_debug[5];
     } slot[NSLOT];
     struct Lane {  // a second compute stream with its own work buffers
         DevBuf packed, seed_scratch;
@@ -482,9 +484,11 @@ void ma_ctx_destroy(ma_ctx* ctx) {
     for (auto& sl : ctx->slot) {
         sl.bases.release();
         sl.lens.release();
-        for (DevBuf& b : sl.out) b.release();
+        sl.hits.release();
+        for (DevBuf& b : sl.debug) b.release();
         sl.h_lens.release();
-        for (HostBuf& b : sl.h_out) b.release();
+        sl.h_hits.release();
+        for (HostBuf& b : sl.h_debug) b.release();
     }
     for (auto& ln : ctx->lane) {
         ln.packed.release();
@@ -725,11 +729,20 @@ int ma_map_batch(ma_ctx* ctx, const ma_index* idx, const uint8_t* bases, const u
         const size_t width[12] = {4, 4, 4, 4, 4, 4, 4, 8, 8, 4, 4, 4};
         const bool stage_lens = pageable(lens);
         bool stage_out[12];
-        bool any_stage = stage_lens;
+        bool any_stage = stage_lens, all_hits_staged = true;
         for (int f = 0; f < 12; ++f) {
             stage_out[f] = host_out[f] && pageable(host_out[f]);
             any_stage = any_stage || stage_out[f];
+            if (f < 7) all_hits_staged = all_hits_staged && stage_out[f];
         }
+        // bytes from one hit array of a chunk of c pairs to the next
+        auto stride = [&](uint32_t c) { return (static_cast<size_t>(mates) * c * 4 + 255) & ~static_cast<size_t>(255); };
+        auto dev_out = [&](ma_ctx::Slot& sl, int f, uint32_t c) {
+            return f < 7 ? sl.hits.as<char>() + f * stride(c) : sl.debug[f - 7].as<char>();
+        };
+        auto staged_out = [&](ma_ctx::Slot& sl, int f, uint32_t c) {
+            return f < 7 ? sl.h_hits.as<char>() + f * stride(c) : sl.h_debug[f - 7].as<char>();
+        };
         int k = 0;
         float acc_ms[4] = {0, 0, 0, 0};
         // every slot sized for the largest chunk before any copy starts
@@ -738,10 +751,14 @@ int ma_map_batch(ma_ctx* ctx, const ma_index* idx, const uint8_t* bases, const u
             const int64_t cs = static_cast<int64_t>(std::min(cap, n1)) * mates;
             sl.bases.ensure(static_cast<size_t>(cs) * max_len);
             sl.lens.ensure(cs * 4);
-            for (int f = 0; f < 12; ++f) sl.out[f].ensure(cs * width[f]);
+            sl.hits.ensure(7 * stride(std::min(cap, n1)));
+            for (int f = 7; f < 12; ++f) sl.debug[f - 7].ensure(cs * width[f]);
             if (stage_lens) sl.h_lens.ensure(cs * 4);
-            for (int f = 0; f < 12; ++f)
-                if (stage_out[f]) sl.h_out[f].ensure(cs * width[f]);
+            for (int f = 0; f < 12; ++f) {
+                if (!stage_out[f]) continue;
+                if (f < 7) sl.h_hits.ensure(7 * stride(std::min(cap, n1)));
+                else sl.h_debug[f - 7].ensure(cs * width[f]);
+            }
         }
         // the chunk (first pair, pairs) whose staged outputs slot i holds
         uint32_t pend_a[ma_ctx::NSLOT], pend_c[ma_ctx::NSLOT];
@@ -750,13 +767,13 @@ int ma_map_batch(ma_ctx* ctx, const ma_index* idx, const uint8_t* bases, const u
             if (!pend[si]) return;
             ck(cudaEventSynchronize(ctx->slot_free[si]), "cudaEventSynchronize");
             pend[si] = false;
-            const ma_ctx::Slot& sl = ctx->slot[si];
+            ma_ctx::Slot& sl = ctx->slot[si];
             for (int f = 0; f < 12; ++f) {
                 if (!stage_out[f]) continue;
                 for (int m = 0; m < mates; ++m) {
                     const size_t row0 = static_cast<size_t>(m) * n1 + pend_a[si];
                     std::memcpy(static_cast<char*>(host_out[f]) + row0 * width[f],
-                                sl.h_out[f].as<char>() + static_cast<size_t>(m) * pend_c[si] * width[f],
+                                staged_out(sl, f, pend_c[si]) + static_cast<size_t>(m) * pend_c[si] * width[f],
                                 pend_c[si] * width[f]);
                 }
             }
@@ -783,32 +800,32 @@ int ma_map_batch(ma_ctx* ctx, const ma_index* idx, const uint8_t* bases, const u
             // (on the host too when its staging buffers are reused)
             drain(si);
             ck(cudaStreamWaitEvent(ctx->copy_stream, ctx->slot_free[si], 0), "cudaStreamWaitEvent");
-            for (int m = 0; m < mates; ++m) {
+            // the mates of a whole batch lie next to one another: one copy
+            const int parts = c == n1 ? 1 : mates;
+            const size_t rows = static_cast<size_t>(c) * mates / parts;
+            for (int m = 0; m < parts; ++m) {
                 const size_t row0 = static_cast<size_t>(m) * n1 + a;
-                ck(cudaMemcpyAsync(sl.bases.as<uint8_t>() + static_cast<size_t>(m) * c * max_len,
-                                   bases + row0 * max_len, static_cast<size_t>(c) * max_len, cudaMemcpyHostToDevice,
-                                   ctx->copy_stream), "H2D bases");
-                const uint32_t* lsrc = lens + row0;
-                if (stage_lens) {
-                    uint32_t* h = sl.h_lens.as<uint32_t>() + static_cast<size_t>(m) * c;
-                    std::memcpy(h, lsrc, c * 4);
-                    lsrc = h;
-                }
-                ck(cudaMemcpyAsync(sl.lens.as<uint32_t>() + static_cast<size_t>(m) * c, lsrc, c * 4,
-                                   cudaMemcpyHostToDevice, ctx->copy_stream), "H2D lens");
+                ck(cudaMemcpyAsync(sl.bases.as<uint8_t>() + m * rows * max_len, bases + row0 * max_len,
+                                   rows * max_len, cudaMemcpyHostToDevice, ctx->copy_stream), "H2D bases");
+                uint32_t* d = sl.lens.as<uint32_t>() + m * rows;
+                if (stage_lens) std::memcpy(sl.h_lens.as<uint32_t>() + m * rows, lens + row0, rows * 4);
+                else ck(cudaMemcpyAsync(d, lens + row0, rows * 4, cudaMemcpyHostToDevice, ctx->copy_stream), "H2D lens");
             }
+            if (stage_lens)
+                ck(cudaMemcpyAsync(sl.lens.p, sl.h_lens.p, static_cast<size_t>(c) * mates * 4, cudaMemcpyHostToDevice,
+                                   ctx->copy_stream), "H2D lens");
             ck(cudaEventRecord(ctx->h2d_done[si], ctx->copy_stream), "cudaEventRecord");
             // compute the chunk, then read it back on the compute stream
             ck(cudaStreamWaitEvent(cst, ctx->h2d_done[si], 0), "cudaStreamWaitEvent");
-            DevOut o{sl.out[0].as<int32_t>(), sl.out[1].as<uint32_t>(), sl.out[2].as<uint32_t>(),
-                     sl.out[3].as<int32_t>(), sl.out[4].as<uint32_t>(), sl.out[5].as<uint32_t>(),
-                     sl.out[6].as<uint32_t>(), nullptr, nullptr, nullptr, nullptr, nullptr};
+            auto hit = [&](int f) { return reinterpret_cast<uint32_t*>(dev_out(sl, f, c)); };
+            DevOut o{reinterpret_cast<int32_t*>(hit(0)), hit(1), hit(2), reinterpret_cast<int32_t*>(hit(3)), hit(4),
+                     hit(5), hit(6), nullptr, nullptr, nullptr, nullptr, nullptr};
             if (want_dbg) {
-                o.uk = sl.out[7].as<uint64_t>();
-                o.ul = sl.out[8].as<uint64_t>();
-                o.us = sl.out[9].as<int32_t>();
-                o.e = sl.out[10].as<int32_t>();
-                o.score = sl.out[11].as<int32_t>();
+                o.uk = sl.debug[0].as<uint64_t>();
+                o.ul = sl.debug[1].as<uint64_t>();
+                o.us = sl.debug[2].as<int32_t>();
+                o.e = sl.debug[3].as<int32_t>();
+                o.score = sl.debug[4].as<int32_t>();
             }
             enqueue_map(ctx, idx, sl.bases.as<uint8_t>(), sl.lens.as<uint32_t>(), c, paired, max_len, bs_r1, bs_r2,
                         p, o, cst, false, two ? &ln.packed : nullptr, two ? &ln.seed_scratch : nullptr);
@@ -824,17 +841,21 @@ int ma_map_batch(ma_ctx* ctx, const ma_index* idx, const uint8_t* bases, const u
             }
             ck(cudaEventRecord(ctx->comp_done[si], cst), "cudaEventRecord");
             ck(cudaStreamWaitEvent(ctx->d2h_stream, ctx->comp_done[si], 0), "cudaStreamWaitEvent");
-            for (int f = 0; f < 12; ++f) {
+            if (all_hits_staged)  // the 7 arrays in one copy
+                ck(cudaMemcpyAsync(sl.h_hits.p, sl.hits.p, 7 * stride(c), cudaMemcpyDeviceToHost, ctx->d2h_stream),
+                   "D2H");
+            for (int f = all_hits_staged ? 7 : 0; f < 12; ++f) {
                 if (!host_out[f]) continue;
                 if (stage_out[f]) {  // one copy of the chunk into the staging buffer
-                    ck(cudaMemcpyAsync(sl.h_out[f].p, sl.out[f].p, static_cast<size_t>(mates) * c * width[f],
-                                       cudaMemcpyDeviceToHost, ctx->d2h_stream), "D2H");
+                    ck(cudaMemcpyAsync(staged_out(sl, f, c), dev_out(sl, f, c),
+                                       static_cast<size_t>(mates) * c * width[f], cudaMemcpyDeviceToHost,
+                                       ctx->d2h_stream), "D2H");
                     continue;
                 }
                 for (int m = 0; m < mates; ++m) {
                     const size_t row0 = static_cast<size_t>(m) * n1 + a;
                     ck(cudaMemcpyAsync(static_cast<char*>(host_out[f]) + row0 * width[f],
-                                       sl.out[f].as<char>() + static_cast<size_t>(m) * c * width[f], c * width[f],
+                                       dev_out(sl, f, c) + static_cast<size_t>(m) * c * width[f], c * width[f],
                                        cudaMemcpyDeviceToHost, ctx->d2h_stream), "D2H");
                 }
             }

@@ -369,3 +369,27 @@ def test_packed_rows_at_block_edges(ctx, small_ref, max_len, n1, skew):
     for f in MapResult.FIELDS:
         got = out[f].cpu().numpy().view(o[f].dtype)
         assert np.array_equal(got, o[f]), f
+
+
+@pytest.mark.parametrize("pinned", [("rid",), ("pos", "nm"), ("rid", "pos", "mapq", "flag", "sl", "sr")])
+@pytest.mark.parametrize("n1,paired,chunk", [(1, True, 0), (33, False, 0), (65, True, 7)])
+def test_host_batch_with_some_outputs_page_locked(ctx, small_ref, pinned, n1, paired, chunk):
+    """The hit arrays share one copy back only when all of them are staged."""
+    torch = pytest.importorskip("torch")
+    from mojoalign_b200 import MapResult
+
+    fa, prefix = small_ref
+    gi = gpu_index(ctx, prefix, 12, 12)
+    rb = sim(fa, n1, paired, seed=n1)
+    o = oracle.OracleIndex(prefix).map(rb.bases, rb.lens, n1, paired, 150, 1, 2, BENCH_PARAMS.as_list())
+    res = MapResult.empty(rb.n_seq, False)
+    for f in pinned:
+        a = getattr(res, f)
+        setattr(res, f, torch.empty(a.size, dtype=torch.int32, pin_memory=True).numpy().view(a.dtype))
+    ctx.set_pipeline(chunk, 0, chunk, 2)
+    try:
+        got = map_batch(ctx, gi, rb.bases, rb.lens, n1, paired, 150, "C2T", "G2A", BENCH_PARAMS, out=res)
+    finally:
+        ctx.set_pipeline()
+    for f in MapResult.FIELDS:
+        assert np.array_equal(getattr(got, f), o[f]), f
