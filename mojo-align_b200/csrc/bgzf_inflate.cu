@@ -32,7 +32,7 @@
 // about 80 k cycles (segments of equal code lengths fall into step late), the
 // write pass 25 k, the resolve 54 k, the CRC 11 k; the next member's header and
 // tables (82 k by one warp) are read meanwhile.  128 MB in 1961 members (zlib
-// level 6): 1.45 ms; segments of 96 bits 1.87, of 160 or 288 bits 1.46 and
+// level 6): 1.42 ms, 1.45 with one literal per table entry; segments of 96 bits 1.87, of 160 or 288 bits 1.46 and
 // 1.49 ms, 3 to 5 checkpoints per segment that stop a second decode early 1.74
 // ms; one warp per member, decoded by one lane throughout, took 6.2 ms.
 #include <string>
@@ -161,7 +161,9 @@ static_assert(THREADS * CRC_BYTES >= MAX_BYTES, "the CRC covers a member");
 constexpr int STRIP = 4 * THREADS;
 
 // Decoding table entries: bits 0-3 code length, 4-5 kind, 6-9 extra bits,
-// 16-31 value (byte, or the length's or distance's base).
+// 16-31 value (the length's or distance's base).  Of a literal: 7-10 its code
+// length, 16-23 the byte; where the table's bits hold another literal after it
+// bit 6 is set, 24-31 are that byte, and 0-3 the length of both codes.
 enum : uint32_t { K_LITERAL = 0, K_COPY = 1, K_END = 2, K_OTHER = 3 };  // K_OTHER: longer than the table's bits, or no code
 
 // The canonical codes of an alphabet: of length l, `count` codes from `first`
@@ -298,7 +300,7 @@ __device__ __forceinline__ int canon_find(const Canon& c, uint32_t v, int from, 
 
 __device__ __forceinline__ uint32_t lit_entry(int sym, uint32_t bits) {
     if (sym < 0 || sym > 285) return K_OTHER << 4;
-    if (sym < 256) return bits | static_cast<uint32_t>(sym) << 16;
+    if (sym < 256) return bits | bits << 7 | static_cast<uint32_t>(sym) << 16;
     if (sym == 256) return bits | K_END << 4;
     const int i = sym - 257;
     return bits | K_COPY << 4 | static_cast<uint32_t>(inflate::len_extra(i)) << 6 | inflate::len_base(i) << 16;
@@ -342,8 +344,17 @@ __device__ __forceinline__ uint32_t decode_bits(Smem& S, const Head& H, bool on,
             const Window w(S.in, pos);
             const uint32_t e = entry_at<LIT_BITS>(w.lo, H.lit, H.cl, lit_entry);
             const uint32_t kind = (e >> 4) & 3;
-            uint32_t used = e & 15, v = 0xff00u | (e >> 16), len = 1, dist = 1;
-            if (kind == K_COPY) {
+            uint32_t used = e & 15, v = 0xff00u | ((e >> 16) & 0xff), len = 1, dist = 1;
+            bool two = false;
+            if (kind == K_LITERAL) {
+                // a second literal that starts past the limit is the next
+                // segment's: where a segment ends must not depend on how its
+                // literals fall into pairs, or starts would take longer to settle
+                const uint32_t b1 = (e >> 7) & 15;
+                two = (e & 64) && pos + b1 < limit;
+                if (two) len = 2;
+                else used = b1;
+            } else if (kind == K_COPY) {
                 const uint32_t eb = (e >> 6) & 15;
                 len = (e >> 16) + low_bits(w.lo >> used, eb);
                 used += eb;  // at most 20
@@ -354,12 +365,17 @@ __device__ __forceinline__ uint32_t decode_bits(Smem& S, const Head& H, bool on,
                 used += db + deb;
                 if (((d >> 4) & 3) == K_OTHER || (WRITE && dist > o)) flag = F_BAD;
                 v = o - dist;
-            } else if (kind != K_LITERAL) {
+            } else {
                 flag = kind == K_END ? F_END : F_BAD;
             }
             pos += used;
             if (flag == F_NONE) {
-                if (WRITE) {
+                if (WRITE && two) {
+                    S.u.cell[o] = static_cast<uint16_t>(v);
+                    S.u.cell[o + 1] = static_cast<uint16_t>(0xff00u | (e >> 24));
+                    atomicOr(S.starts + (o >> 5), 3u << (o & 31));
+                    if ((o & 31) == 31) atomicOr(S.starts + (o >> 5) + 1, 1u);
+                } else if (WRITE) {
                     // a copy that overlaps itself in pieces of dist, 2 dist,
                     // 4 dist ... bytes, each of which copies from v on, where
                     // the pieces before it have put as many
@@ -495,10 +511,23 @@ __device__ void read_head(Head& H, const uint8_t* in, uint32_t n, uint32_t pos, 
     __syncwarp();
 }
 
-__device__ __forceinline__ void fill_tables(Head& H, uint32_t t, uint32_t threads) {
+// The tables of H by `threads` threads that `sync` waits for.  The entries of
+// two literals come from the single ones in place: one that is paired already
+// still tells its first literal.
+template <typename F>
+__device__ __forceinline__ void fill_tables(Head& H, uint32_t t, uint32_t threads, F sync) {
     if (!H.ok || H.type == 0) return;
     fill_table<LIT_BITS>(H.lit, H.cl, t, threads, lit_entry);
     fill_table<DIST_BITS>(H.dist, H.cd, t, threads, dist_entry);
+    sync();
+    volatile uint32_t* lit = H.lit;
+    for (uint32_t i = t; i < (1u << LIT_BITS); i += threads) {
+        const uint32_t e = lit[i], b1 = (e >> 7) & 15;
+        if (((e >> 4) & 3) != K_LITERAL) continue;
+        const uint32_t d = lit[i >> b1], b2 = (d >> 7) & 15;
+        if (((d >> 4) & 3) == K_LITERAL && b1 + b2 <= LIT_BITS)
+            lit[i] = (b1 + b2) | 64u | b1 << 7 | (e & 0xff0000u) | (d & 0xff0000u) << 8;
+    }
 }
 
 // Whether member m's spans lie in their buffers.
@@ -587,7 +616,7 @@ __device__ bool cta_member(const bgzf_inflate::Job& j, uint32_t m, Smem& S, Head
         work_sync();  // the block's tables are done with
         if (warp == 0) read_head(H, in, n, pos, static_cast<int>(lane));
         work_sync();
-        fill_tables(H, t, THREADS);
+        fill_tables(H, t, THREADS, [] { work_sync(); });
         work_sync();
     }
     if (made != isz) return false;
@@ -699,7 +728,7 @@ __global__ void __launch_bounds__(CTA_THREADS, 1) bgzf_inflate_kernel(bgzf_infla
     auto header_of = [&](uint32_t m, Head& H) {
         if (m >= j.n || !member_spans(j, m) || !member_fits(j, m)) return;
         read_head(H, j.in + j.src_off[m], j.src_len[m], 0, static_cast<int>(t - THREADS));
-        fill_tables(H, t - THREADS, 32);
+        fill_tables(H, t - THREADS, 32, [] { __syncwarp(); });
     };
     if (t >= THREADS) header_of(blockIdx.x, S.head[0]);
     __syncthreads();

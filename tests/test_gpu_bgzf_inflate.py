@@ -186,3 +186,22 @@ def test_damaged_members_end_as_on_the_host(ctx, tmp_path_factory):
             want.append(rc if rc else 8 if len(b) != n else 0 if zlib.crc32(b) == c else 9)
     status, _, _, _ = _inflate_raw(ctx, members)
     np.testing.assert_array_equal(status, want)
+
+
+@pytest.mark.parametrize("symbols", [1, 2, 3, 5, 16, 64, 65, 200, 256])
+def test_literals_in_pairs(ctx, symbols):
+    """Members of literals alone, of 1 to 15 bits: pairs that fill the table's
+    bits or just miss them, that straddle a segment's end, a word of the start
+    marks and the member's last byte."""
+    import zlib
+
+    rng = np.random.default_rng(symbols)
+    cases = []
+    for n in (4, 5, 31, 32, 33, 64, 65, 2047, 30_001, 65_279, 65_280):
+        for p in (np.full(symbols, 1 / symbols), np.geomspace(1, 1e-4, symbols)):
+            data = rng.choice(symbols, n, p=p / p.sum()).astype(np.uint8).tobytes()
+            c = zlib.compressobj(6, zlib.DEFLATED, -15, 8, zlib.Z_HUFFMAN_ONLY)
+            cases.append((c.compress(data) + c.flush(), data))
+    status, got, _, _ = _inflate_raw(ctx, [(p, len(d), zlib.crc32(d)) for p, d in cases])
+    for i, ((_, data), s, g) in enumerate(zip(cases, status, got)):
+        assert s == 0 and g == data, i
