@@ -38,10 +38,12 @@ namespace {
 // counters[]
 constexpr int C_ACTIVE = 0;    // reads active in the current round
 constexpr int C_NEXT = 1;      // reads appended to the next round's list
-constexpr int C_LOCI = 4;      // loci appended in the current round: a u64 in counters[4..5]
+constexpr int C_LOCI = 32;     // loci appended in the current round: a u64 in counters[32..33]
 constexpr int C_ROUNDS = 3;    // read-rounds processed (tally)
 constexpr int C_HANDOFF = 8;   // [8] reads for stage 2, [9] its work cursor
-constexpr int N_COUNTERS = 16;
+constexpr int C_SEARCH = 64;   // deals of the round's items and loci beyond the
+constexpr int C_EVAL = 96;     // warps' first ones: u64 each
+constexpr int N_COUNTERS = 128;  // what whole grids add to lies 128 bytes apart
 
 // Round keys: nm << (27 + ib) | ordinal << ib | locus index, ib bits of
 // index: what the largest nm of the call leaves of the 64 bits, at most 31.
@@ -86,6 +88,46 @@ size_t align256(size_t b) { return (b + 255) & ~static_cast<size_t>(255); }
 __device__ __forceinline__ unsigned long long* loci_count(const Wave& w) {
     return reinterpret_cast<unsigned long long*>(w.counters + C_LOCI);
 }
+
+// The round's items or loci in groups of 32, dealt to the warps a few groups at
+// a time: a warp's first ones by its place in the grid, later ones from a
+// counter, asked for ahead.  Dealt by place alone, the warps whose groups held
+// the long searches and the repeats kept the rest waiting (eval ran with 40 %
+// of an SM's warps on average where 50 % fit).  A warp that is to come back
+// more than DEALS times takes several groups at once and the counters lie in
+// lines of their own: one group at a time, in the line of the loci's count,
+// the 4 M additions for 2 M reads' items took 12 ms on some cards.  Loci of
+// one read lie together, so eval takes two groups at most.  2 M uneven reads:
+// search 8.2 -> 7.3 ms, eval 6.6 -> 6.0 (6.45 with up to 8 groups); 800 k reads
+// of 250 bases 2.04 -> 1.95 and 1.47 -> 1.47.
+constexpr uint32_t DEALS = 4, SEARCH_DEAL = 8, EVAL_DEAL = 2;
+struct Groups {
+    unsigned long long* counter;
+    uint64_t base, ticket;  // base: first item of the group in hand
+    uint32_t per, left;     // groups of a deal; of this one from the group in hand on
+    __device__ __forceinline__ Groups(uint32_t* counters, int c, uint64_t n_items, uint32_t most)
+        : counter(reinterpret_cast<unsigned long long*>(counters + c)), ticket(0) {
+        const uint64_t threads = static_cast<uint64_t>(gridDim.x) * blockDim.x;
+        per = 1;
+        while (per < most && 2 * per * DEALS * threads <= n_items) per *= 2;
+        left = per;
+        base = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + (threadIdx.x & ~31u)) * per;
+    }
+    // The group in hand, one of the round's, is taken up (an empty round asks
+    // for nothing) ...
+    __device__ __forceinline__ void take() {
+        if (--left == 0 && (threadIdx.x & 31) == 0) ticket = atomicAdd(counter, 1ull);
+    }
+    // ... and worked through: the following one.
+    __device__ __forceinline__ void next() {
+        if (left) {
+            base += 32;
+        } else {
+            left = per;
+            base = 32 * per * (__shfl_sync(0xFFFFFFFFu, ticket, 0) + gridDim.x * (blockDim.x >> 5));
+        }
+    }
+};
 
 // Carves the scratch; returns the bytes used (layout only when p != null).
 size_t wave_layout(char* p, int64_t n_seq, uint64_t locus_cap, Wave* w) {
@@ -150,6 +192,7 @@ __global__ void wf_round_begin_kernel(Wave w) {
     w.counters[C_ACTIVE] = w.counters[C_NEXT];
     w.counters[C_NEXT] = 0;
     *loci_count(w) = 0;
+    for (int i = 0; i < 2; ++i) w.counters[C_SEARCH + i] = w.counters[C_EVAL + i] = 0;
 }
 
 // A read's memo (MEMO1 loci, 64 bytes), all of it in flight at once; entries
@@ -187,9 +230,9 @@ struct MemoRow {
 //           leave their slot dead.
 // Which pass finds a seed does not change the round's result: the eval keys
 // carry the candidate order.
-// 2 M uneven reads on 250 Mbp (62 M lookups, 56 M steps, 103 M rows): 8.1 ms,
-// 10.1 ms with a thread per item through all three; 800 k reads of 250 bases
-// 2.05 and 2.7 ms.  Bound by the latency of the gathers.
+// 2 M uneven reads on 250 Mbp (62 M lookups, 56 M steps, 103 M rows): 7.3 ms;
+// with a thread per item through all three the pass took a quarter longer.
+// Bound by the latency of the gathers.
 constexpr int SEARCH_WARPS = 8;   // 256 threads
 constexpr int SEARCH_LIST = 64;   // searches under way per warp
 constexpr int SEED_STAGE = 64;    // seeds waiting per warp
@@ -232,9 +275,7 @@ __global__ void __launch_bounds__(256, MINB) wf_search_kernel(DevIndex ix, DevRe
     const unsigned lt_mask = (1u << lane) - 1;
     const bool can_predict = ix.summary && ix.kmer3_k > 0 && ix.kmer3_k <= P.seed_len;
     SearchLists& q = s_lists[threadIdx.x >> 5];
-    // the warp's items: 32 at a time, warp g takes groups g, g + n_warps, ...
-    const uint64_t group_stride = static_cast<uint64_t>(gridDim.x) * (SEARCH_WARPS * 32);
-    uint64_t base = (static_cast<uint64_t>(blockIdx.x) * SEARCH_WARPS + (threadIdx.x >> 5)) * 32;
+    Groups groups(w.counters, C_SEARCH, n_items, SEARCH_DEAL);
     int n_search = 0, n_seeds = 0;  // entries of the lists (warp-uniform)
     uint32_t n_rows = 0;
     // pushes the seeds of the lanes that found one
@@ -271,7 +312,7 @@ __global__ void __launch_bounds__(256, MINB) wf_search_kernel(DevIndex ix, DevRe
         n_search += __popc(ob);
     };
     for (;;) {
-        const bool more = base < n_items;
+        const bool more = groups.base < n_items;
         const bool look = more && n_search <= SEARCH_LIST - 32;
         if (n_seeds > SEED_STAGE - 32 || (!more && n_search == 0)) {
             // ---- rows ----
@@ -326,8 +367,8 @@ __global__ void __launch_bounds__(256, MINB) wf_search_kernel(DevIndex ix, DevRe
             n_rows = 0;
         } else if (look) {
             // ---- lookup ----
-            const uint64_t item = base + lane;
-            base += group_stride;
+            const uint64_t item = groups.base + lane;
+            groups.take();
             Seed sd{0, 0, -1, false};
             SeedSearch c{};
             bool go_on = false;
@@ -357,6 +398,7 @@ __global__ void __launch_bounds__(256, MINB) wf_search_kernel(DevIndex ix, DevRe
             }
             push_search(go_on, c, r, e, ei);
             push_seeds(sd, r, e, ei);
+            groups.next();
             __syncwarp();
         } else {
             // ---- step ----
@@ -408,7 +450,8 @@ __global__ void __launch_bounds__(256, MINB) wf_search_kernel(DevIndex ix, DevRe
 // the shift, the rare long ones kept the warp at 16 lanes of 32.  Candidates
 // are pruned against the read's best from earlier rounds; the round's minimum
 // key per read is an atomicMin of (nm, ordinal, locus index) packed in 64 bits.
-// 102 M loci, 31 M live shifts of 2 M uneven reads: 6.7 ms, 8.0 ms before.
+// 102 M loci, 31 M live shifts of 2 M uneven reads: 6.0 ms; with a lane for all
+// parts of a shift the pass took a fifth longer.
 constexpr int EVAL_THREADS = 256;
 constexpr int SHIFT_LIST = 64;  // entries per list and warp: locus index << 5 | shift
 enum : int { L_CORE = 0, L_FULL = SHIFT_FULL, L_DELETION = SHIFT_DELETION, L_OFFSETS = SHIFT_OFFSETS };
@@ -433,10 +476,9 @@ __global__ void __launch_bounds__(EVAL_THREADS, MINB) wf_eval_kernel(DevIndex ix
     uint64_t(*list)[SHIFT_LIST] = s_list[threadIdx.x >> 5];
     int n[4] = {0, 0, 0, 0};  // entries of each list (warp-uniform)
     uint32_t rem = 0, li = 0;  // the lane's locus and its live shifts not yet listed
-    const uint32_t stride = gridDim.x * blockDim.x;
-    uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u);
+    Groups groups(w.counters, C_EVAL, n_loci, EVAL_DEAL);
     for (;;) {
-        const bool have = base < n_loci, pending = __any_sync(FULL, rem != 0);
+        const bool have = groups.base < n_loci, pending = __any_sync(FULL, rem != 0);
         // a full list first, the last part's before the others; then the shifts
         // waiting, the next loci, and in the end what the lists still hold
         int part = -1;
@@ -504,8 +546,8 @@ __global__ void __launch_bounds__(EVAL_THREADS, MINB) wf_eval_kernel(DevIndex ix
             const int total = n[L_CORE] + __shfl_sync(FULL, incl, 31);
             n[L_CORE] = total < SHIFT_LIST ? total : SHIFT_LIST;
         } else {
-            li = base + lane;
-            base += stride;
+            li = static_cast<uint32_t>(groups.base) + lane;
+            groups.take();
             if (li < n_loci) {
                 const WLocus L = w.loci[li];
                 if (L.read != DEAD_LOCUS && !w.overflow[L.read]) {
@@ -514,6 +556,7 @@ __global__ void __launch_bounds__(EVAL_THREADS, MINB) wf_eval_kernel(DevIndex ix
                     rem = live_shifts<S>(ix, rd, L.b0, L.rev, adj_cap, cl.budget, cl.clip_cap, prune_of(w, L.read), t);
                 }
             }
+            groups.next();
         }
     }
     flush_tally<S>(t, tally_out);
