@@ -50,10 +50,11 @@ METRIC = "reads/s seed+extend"
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of the seed
 # kernels (wf_init through seed_stage2, pack excluded) per read of one timed
 # step of the default genome workload (3100 Mbp, 50 M uneven single-end
-# reads), from a one-pass ncu capture of that step on this build with the
-# tuning below; roofline.traffic reports it for runs of that workload and
-# tuning, and null otherwise.
-GENOME_SEED_DRAM_BYTES_PER_READ = 24660
+# reads), from a one-pass ncu capture of that step with the tuning below;
+# roofline.traffic reports it for runs of that workload and tuning, and null
+# otherwise.  None: the capture (24660) is of the search and eval kernels
+# before they ran from lists per warp.
+GENOME_SEED_DRAM_BYTES_PER_READ = None
 GENOME_SEED_DRAM_TUNING = (4, 2, 0, 1, 1, 1, 8, 32, 0, 1)
 GENOME_SEED_DRAM_AT_K = 28  # the capture's A/T window table (0: none)
 # The workload parameters: the reference defaults with seed_len 19 and
@@ -65,12 +66,8 @@ BENCH_PARAM_VALUES = {"seed_len": 19, "seed_stride": 2, "max_occ": 500, "max_dif
 SEED_KERNELS = {
     0: "seed/extend: seed_stage1_kernel over every endpoint (one thread per read)",
     1: "seed/extend: seed_stage1_kernel + seed_stage2_kernel (thread per read, then warp per read)",
-    2: "seed/extend: wavefront rounds (wf_search_kernel + wf_eval_kernel + wf_finalize_kernel per round, "
-       "seed_stage2_kernel for reads left over)",
-    3: "seed/extend: wavefront rounds with lane refill (wf_search_refill_kernel + wf_eval_staged_kernel + "
-       "wf_finalize_kernel per round, seed_stage2_kernel for reads left over)",
-    4: "seed/extend: wavefront rounds with staged eval (wf_search_kernel + wf_eval_staged_kernel + "
-       "wf_finalize_kernel per round, seed_stage2_kernel for reads left over)",
+    **dict.fromkeys((2, 3, 4), "seed/extend: wavefront rounds (wf_search_kernel + wf_eval_kernel + "
+                    "wf_finalize_kernel per round, seed_stage2_kernel for reads left over)"),
 }
 READ_LEN = 150
 
@@ -757,7 +754,7 @@ def run_fq2bam_stage(args, ctx, gi, rb, local, params):
                            "phases_s": gz_phases, "input_bytes": gz_bytes,
                            "e2e": {"h2d_bytes_per_step": int(gz_phases.get("fastq_h2d_bytes", gz_bytes)),
                                    "d2h_bytes_per_step": out_gz.stat().st_size},
-                           "inflate": "BGZF members copied to the device and inflated there (one warp per member)",
+                           "inflate": "BGZF members copied to the device and inflated there (one CTA per member)",
                            "parity": {"bam_content_equals_plain_input": bool(gz_same)}},
         }
     finally:
@@ -1047,8 +1044,7 @@ def seeding_roofline(tally, wave, tally2=None, n_seq=0, seed_kernel=2) -> dict:
     tally2 = tally2 or [0] * 12
     search_ms = statistics.mean(w[0] for w in wave)
     seed_bytes = 32 * sum(tally[i] - tally2[i] for i in range(3))
-    name = "wf_search_refill_kernel" if seed_kernel == 3 else "wf_search_kernel"
-    out = {"seeding": {"kernel": f"{name} (all rounds)", "ms": round(search_ms, 3),
+    out = {"seeding": {"kernel": "wf_search_kernel (all rounds)", "ms": round(search_ms, 3),
                        "eval_ms": round(statistics.mean(w[1] for w in wave), 3),
                        "finalize_ms": round(statistics.mean(w[2] for w in wave), 3),
                        "alg_bytes": int(seed_bytes),
