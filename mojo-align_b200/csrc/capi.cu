@@ -25,10 +25,10 @@ int launch_seed_extend(const DevIndex& ix, const DevReads& R, const DevParams& P
                        unsigned long long* d_tally, int level, cudaStream_t st);
 double run_gather_bench(uint64_t buffer_bytes, int line_bytes, uint64_t n_loads, int sm_count, cudaStream_t st);
 size_t two_stage_scratch_bytes(int64_t n_seq);
-size_t wavefront_scratch_bytes(int64_t n_seq, int loci_per_read);
-ma_tuning wave_tuning(const ma_tuning& asked, int64_t n_seq, int max_len, const DevParams& P);
+size_t wavefront_scratch_bytes(int64_t n_seq, uint64_t loci);
+WavePlan wave_plan(const ma_tuning& asked, int64_t n_seq, int max_len, const DevParams& P);
 int launch_seed_wavefront(const DevIndex& ix, const DevReads& R, const DevParams& P, const DevOut& out, int max_len,
-                          const ma_tuning& t, int stage2_blocks, void* scratch, int sm_count, int* d_err,
+                          const WavePlan& plan, int stage2_blocks, void* scratch, int sm_count, int* d_err,
                           unsigned long long* d_tally, WaveTimer* timer, cudaStream_t st);
 int launch_seed_two_stage(const DevIndex& ix, const DevReads& R, const DevParams& P, const DevOut& out,
                           int stage1_endpoints, int stage1_max_rows, int stage2_blocks, int level,
@@ -284,11 +284,11 @@ void enqueue_map(ma_ctx* ctx, const ma_index* idx, const uint8_t* d_bases, const
     if (ctx->tuning.seed_kernel == 0) {
         launches += launch_seed_extend(idx->dix, R, P, out, d_tally, level, st);
     } else if (ctx->tuning.seed_kernel >= 2) {
-        const ma_tuning t = wave_tuning(ctx->tuning, n_seq, static_cast<int>(max_len), P);
-        seed_scratch->ensure(wavefront_scratch_bytes(n_seq, t.wave_loci_per_read));
+        const WavePlan plan = wave_plan(ctx->tuning, n_seq, static_cast<int>(max_len), P);
+        seed_scratch->ensure(wavefront_scratch_bytes(n_seq, plan.loci));
         const int bps = ctx->tuning.stage2_blocks_per_sm > 0 ? ctx->tuning.stage2_blocks_per_sm
                                                              : stage2_blocks_per_sm(level, d_tally != nullptr);
-        launches += launch_seed_wavefront(idx->dix, R, P, out, static_cast<int>(max_len), t,
+        launches += launch_seed_wavefront(idx->dix, R, P, out, static_cast<int>(max_len), plan,
                                           bps * ctx->sm_count, seed_scratch->p, ctx->sm_count,
                                           ctx->err_flag.as<int>(), d_tally, timed ? &ctx->wave_timer : nullptr, st);
     } else {

@@ -89,6 +89,13 @@ struct WaveTimer {
     bool complete = true;
 };
 
+// How the wavefront form runs a call: its round widths (the wave fields of a
+// tuning) and the entries of its locus list.
+struct WavePlan {
+    ma_tuning tuning;
+    uint64_t loci;
+};
+
 void build_index(const std::string& fasta, const std::string& out_prefix, bool bwameth_c2t,
                  int sa_intv, int device, uint64_t batch_limit = 0);
 

@@ -42,9 +42,10 @@ int pack_rows_per_block(int max_len, int words);
 int launch_seed_extend(const DevIndex& ix, const DevReads& R, const DevParams& P, const DevOut& out,
                        unsigned long long* d_tally, int level, cudaStream_t st);
 size_t two_stage_scratch_bytes(int64_t n_seq);
-size_t wavefront_scratch_bytes(int64_t n_seq, int loci_per_read);
+size_t wavefront_scratch_bytes(int64_t n_seq, uint64_t loci);
+WavePlan wave_plan_asked(const ma_tuning& asked, int64_t n_seq);
 int launch_seed_wavefront(const DevIndex& ix, const DevReads& R, const DevParams& P, const DevOut& out, int max_len,
-                          const ma_tuning& t, int stage2_blocks, void* scratch, int sm_count, int* d_err,
+                          const WavePlan& plan, int stage2_blocks, void* scratch, int sm_count, int* d_err,
                           unsigned long long* d_tally, WaveTimer* timer, cudaStream_t st);
 int launch_seed_two_stage(const DevIndex& ix, const DevReads& R, const DevParams& P, const DevOut& out,
                           int stage1_endpoints, int stage1_max_rows, int stage2_blocks, int level,
@@ -138,7 +139,8 @@ GroupLayout layout_for(uint32_t n1, bool paired, int words, uint64_t stage_bytes
     o += OffsetArena::kAlign;
     L.scratch = o;
     if (seed_kernel == 1) o += rnd(two_stage_scratch_bytes(static_cast<int64_t>(n_seq)));
-    if (seed_kernel >= 2) o += rnd(wavefront_scratch_bytes(static_cast<int64_t>(n_seq), t.wave_loci_per_read));
+    const int64_t n = static_cast<int64_t>(n_seq);
+    if (seed_kernel >= 2) o += rnd(wavefront_scratch_bytes(n, wave_plan_asked(t, n).loci));
     L.total = o;
     return L;
 }
@@ -355,8 +357,8 @@ void issue_group(ma_server* s, Group& g) {
         launch_seed_two_stage(*s->dix, R, P, o, t.stage1_endpoints, t.stage1_max_rows, bps * s->sm_count, t.reg_level,
                               t.stage2_first_wave, dev + g.L.scratch, nullptr, nullptr, st);
     } else if (s->seed_kernel() >= 2) {
-        launch_seed_wavefront(*s->dix, R, P, o, 32 * g.words, t, bps * s->sm_count, dev + g.L.scratch, s->sm_count,
-                              d_err, nullptr, nullptr, st);
+        launch_seed_wavefront(*s->dix, R, P, o, 32 * g.words, wave_plan_asked(t, n_seq), bps * s->sm_count,
+                              dev + g.L.scratch, s->sm_count, d_err, nullptr, nullptr, st);
     } else {
         launch_seed_extend(*s->dix, R, P, o, nullptr, t.reg_level, st);
     }

@@ -157,10 +157,9 @@ size_t wave_layout(char* p, int64_t n_seq, uint64_t locus_cap, Wave* w) {
     return o;
 }
 
-uint64_t locus_capacity(int64_t n_seq, int per_read) {
-    uint64_t c = static_cast<uint64_t>(per_read) * static_cast<uint64_t>(n_seq);
-    if (c < 1024) c = 1024;
-    return c < MAX_LOCI ? c : MAX_LOCI;
+uint64_t locus_capacity(uint64_t entries) {
+    if (entries < 1024) entries = 1024;
+    return entries < MAX_LOCI ? entries : MAX_LOCI;
 }
 
 __global__ void __launch_bounds__(256) wf_init_kernel(Wave w, DevOut out, const uint32_t* __restrict__ lens,
@@ -653,7 +652,7 @@ __global__ void __launch_bounds__(256, 4) wf_finalize_kernel(DevIndex ix, DevRea
     flush_tally<S>(t, tally_out);
 }
 
-// See wave_tuning below.
+// See wave_plan below.
 constexpr int64_t WAVE_ONE = 131072, WAVE_ITEMS = 4 << 20, WAVE_LOCI = 2 << 20, WAVE_LOCI_MOST = 16 << 20;
 
 int endpoint_count_host(const DevParams& P, int qlen) {
@@ -726,8 +725,13 @@ int launch_rounds(const DevIndex& ix, const DevReads& R, const DevParams& P, con
 
 }  // namespace
 
-size_t wavefront_scratch_bytes(int64_t n_seq, int loci_per_read) {
-    return wave_layout(nullptr, n_seq, locus_capacity(n_seq, loci_per_read), nullptr);
+size_t wavefront_scratch_bytes(int64_t n_seq, uint64_t loci) {
+    return wave_layout(nullptr, n_seq, locus_capacity(loci), nullptr);
+}
+
+// The plan that takes a tuning as it is.
+WavePlan wave_plan_asked(const ma_tuning& asked, int64_t n_seq) {
+    return WavePlan{asked, static_cast<uint64_t>(asked.wave_loci_per_read) * static_cast<uint64_t>(n_seq)};
 }
 
 // The round widths and the locus list of a call under the default tuning,
@@ -742,15 +746,17 @@ size_t wavefront_scratch_bytes(int64_t n_seq, int loci_per_read) {
 //   400 k 2x250  4.6 (8 endpoints, doubling) and 5.2 ms (16 endpoints)
 // So a batch of up to WAVE_ONE items (reads x endpoints) takes one round, and
 // a later round covers up to WAVE_ITEMS items.  Wide rounds need longer locus
-// lists: up to 256 entries per read while the list stays below 2 M entries (64
-// MB), 8 while it stays below 16 M (512 MB): 800 k reads of 250 bases take 4.3
-// ms with 8 entries and 4.9 with 4, whose list fills up.
-
-ma_tuning wave_tuning(const ma_tuning& asked, int64_t n_seq, int max_len, const DevParams& P) {
-    ma_tuning t = asked;
+// lists: 256 entries per read up to 2 M entries (64 MB) in all, 8 up to 16 M (512
+// MB): 800 k reads of 250 bases take 4.3 ms with 8 entries and 4.9 with 4, whose
+// list fills up.  The list never gets shorter as the reads of a call grow in
+// number, so that a call with fewer reads than one before it finds its scratch
+// there: it allocates nothing, and no captured graph is dropped for it.
+WavePlan wave_plan(const ma_tuning& asked, int64_t n_seq, int max_len, const DevParams& P) {
+    WavePlan plan = wave_plan_asked(asked, n_seq);
+    ma_tuning& t = plan.tuning;
     if (t.stage1_endpoints != 1 || t.wave_endpoints != 8 || t.wave_loci_per_read != 4 || t.wave_max_rounds != 0 ||
         t.wave_growth != 1 || n_seq < 1)
-        return t;
+        return plan;
     const int64_t n_end = endpoint_count_host(P, max_len);
     if (n_seq * n_end <= WAVE_ONE) {
         t.stage1_endpoints = static_cast<int32_t>(n_end > 1 ? n_end : 1);
@@ -758,20 +764,21 @@ ma_tuning wave_tuning(const ma_tuning& asked, int64_t n_seq, int max_len, const 
         t.stage1_endpoints = 2;
         t.wave_endpoints = static_cast<int32_t>(WAVE_ITEMS / n_seq < n_end ? WAVE_ITEMS / n_seq : n_end);
     }
-    int64_t loci = WAVE_LOCI / n_seq < 256 ? WAVE_LOCI / n_seq : 256;
-    if (loci < 8 && n_seq * 8 <= WAVE_LOCI_MOST) loci = 8;
-    if (loci > t.wave_loci_per_read) t.wave_loci_per_read = static_cast<int32_t>(loci);
-    return t;
+    const auto at_most = [](int64_t a, int64_t b) { return static_cast<uint64_t>(a < b ? a : b); };
+    for (const uint64_t c : {at_most(256 * n_seq, WAVE_LOCI), at_most(8 * n_seq, WAVE_LOCI_MOST)})
+        if (c > plan.loci) plan.loci = c;
+    return plan;
 }
 
 // The wavefront form; `scratch` holds wavefront_scratch_bytes(n_seq,
-// t.wave_loci_per_read) bytes, d_err is the batch's error word.  Returns
-// the number of kernel launches.
+// plan.loci) bytes, d_err is the batch's error word.  Returns the number of
+// kernel launches.
 int launch_seed_wavefront(const DevIndex& ix, const DevReads& R, const DevParams& P, const DevOut& out, int max_len,
-                          const ma_tuning& t, int stage2_blocks, void* scratch, int sm_count, int* d_err,
+                          const WavePlan& plan, int stage2_blocks, void* scratch, int sm_count, int* d_err,
                           unsigned long long* d_tally, WaveTimer* timer, cudaStream_t st) {
+    const ma_tuning& t = plan.tuning;
     Wave w;
-    wave_layout(static_cast<char*>(scratch), R.n_seq, locus_capacity(R.n_seq, t.wave_loci_per_read), &w);
+    wave_layout(static_cast<char*>(scratch), R.n_seq, locus_capacity(plan.loci), &w);
     // an accepted candidate has nm <= its read's budget <= max(2, max_diff)
     // (and <= 512): the round keys give the rest to the locus index
     const int max_nm = P.max_diff < 2 ? 2 : (P.max_diff > 512 ? 512 : P.max_diff);

@@ -64,3 +64,35 @@ def test_graph_replay_equals_plain_calls(small_ref):
     torch.cuda.set_stream(torch.cuda.default_stream(dev))
     gi.close()
     ctx.close()
+
+
+@pytest.mark.parametrize("larger,smaller", [(150_000, 139_810), (2_200_000, 2_000_000)])
+def test_a_smaller_call_allocates_nothing(small_ref, larger, smaller):
+    """The work buffers of a call hold any call with fewer reads: none of them
+    grows, so no graph captured with them is dropped."""
+    torch = pytest.importorskip("torch")
+    fa, prefix = small_ref
+    ctx = GpuContext(0)
+    gi = GpuIndex(ctx, prefix, kmer_k=12, kmer3_k=12)
+    dev = torch.device("cuda:0")
+    rb = synth.simulate_reads(fa, synth.ReadModel(len_fixed=36, len_min=36, len_max=36), 5000, False, 36, seed=5)
+    d_b = torch.from_numpy(rb.bases).to(dev).repeat(larger // 5000 + 1, 1)[:larger].contiguous()
+    d_l = torch.full((larger,), 36, dtype=torch.int32, device=dev)
+    out = {f: torch.full((larger,), -9, dtype=torch.int32, device=dev) for f in MapResult.FIELDS}
+    ptrs = {f: x.data_ptr() for f, x in out.items()}
+    torch.cuda.synchronize()
+    free = want = None
+    for n in (larger, smaller, smaller // 2, smaller // 16, 1):
+        for x in out.values():
+            x.fill_(-9)
+        torch.cuda.synchronize()
+        map_batch_device(ctx, gi, d_b.data_ptr(), d_l.data_ptr(), n, False, 36, ptrs, "C2T", "G2A", BENCH_PARAMS)
+        torch.cuda.synchronize()
+        got = {f: x.cpu().numpy() for f, x in out.items()}  # nothing of torch's on the device either
+        if free is None:
+            free, want = torch.cuda.mem_get_info(dev)[0], got
+        assert torch.cuda.mem_get_info(dev)[0] == free, n
+        for f, x in got.items():
+            assert np.array_equal(x[:n], want[f][:n]) and (x[n:] == -9).all(), (n, f)
+    gi.close()
+    ctx.close()
