@@ -235,3 +235,45 @@ def test_lines_at_the_edges_of_the_lanes_the_slots_and_the_stage(ctx, rg, paired
     want = oracle.emit_sam(hits, n1, paired, oracle_arena(arena), names, rg)
     got = emit_sam_from_batch(ctx, hits, n1, paired, arena, SamContigs.from_names(names), rg)
     assert got == want
+
+
+def test_long_contig_names_cost_little(ctx):
+    """Names of 150 bytes, most pairs on two contigs: the warp copies the names,
+    so a call takes little more than with short ones (1.3 times; 6 times when
+    the lane that formats a line's fields copied them)."""
+    import torch
+
+    dev = torch.device("cuda", 0)
+    n1, took = 50_000, []
+    hits, arena, _ = random_sam_batch(41, n1, True, odd_text=0.0)
+    rid = np.random.default_rng(41).integers(0, 6, 2 * n1).astype(np.int32)
+    hits = dict(hits, rid=np.where(hits["rid"] < 0, hits["rid"], rid).astype(np.int32))
+    d_h = {k: _dev(np.asarray(hits[k], dt), dev) for k, dt in HIT_FIELDS}
+    hc = _lib.ma_hits(*[d_h[k].data_ptr() for k, _ in HIT_FIELDS])
+    d_a = {k: _dev(getattr(arena, k), dev) for k in ("data", "name_off", "name_len", "orig_off", "orig_len",
+                                                     "qual_off", "qual_len")}
+    ac = _lib.ma_fastq_arena(d_a["data"].data_ptr(), int(arena.data.size), d_a["name_off"].data_ptr(),
+                             d_a["name_len"].data_ptr(), d_a["orig_off"].data_ptr(), d_a["orig_len"].data_ptr(),
+                             d_a["qual_off"].data_ptr(), d_a["qual_len"].data_ptr())
+    for width in (5, 150):
+        names = [(s + b"%d" % (k // 2)).ljust(width, b"n") for k, s in enumerate([b"f", b"r"] * 3)]
+        want, want_mapped = oracle.emit_sam(hits, n1, True, oracle_arena(arena), names, b"grp")
+        contigs = SamContigs.from_names(names).to_device(torch, dev)
+        d_rg = torch.frombuffer(bytearray(b"grp"), dtype=torch.uint8).to(dev)
+        d_out = torch.zeros(len(want), dtype=torch.uint8, device=dev)
+        d_status = torch.zeros(3, dtype=torch.int64, device=dev)
+        stream = torch.cuda.Stream(dev)
+        torch.cuda.synchronize()
+        times = []
+        for _ in range(9):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record(stream)
+            emit_sam_device(ctx, hc, n1, True, ac, contigs, d_rg.data_ptr(), 3, d_out.data_ptr(), len(want),
+                            d_status.data_ptr(), stream.cuda_stream)
+            b.record(stream)
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+        took.append(float(np.median(times[2:])))
+        assert d_status.tolist() == [len(want), want_mapped, 0]
+        assert d_out.cpu().numpy().tobytes() == want
+    assert took[1] < 3 * took[0], took
