@@ -765,7 +765,7 @@ uint64_t ma_bgzf_bound(uint64_t n);
 
 /*
  * Inflates the members of a BGZF file (compressed FASTQ as bgzip writes it)
- * on the device, one member per CTA: the deflate payload of member m is
+ * on the device, a CTA or a warp per member: the deflate payload of member m is
  * in[src_off[m], + src_len[m]) and its isize[m] bytes go to
  * out[dst_off[m], ...); each member's size and CRC-32 (crc[m]) are checked.
  * The member table comes from the gzip headers (BSIZE of the "BC" extra

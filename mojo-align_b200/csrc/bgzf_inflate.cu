@@ -1,5 +1,6 @@
 // bgzf_inflate.cu - BGZF members inflated on the device (bgzf_inflate.cuh), one
-// CTA per member, a grid-stride loop over the members.
+// CTA per member, a grid-stride loop over the members, and one warp per member
+// for those that the CTAs leave.
 //
 // A deflate stream is serial: where a code starts is known once the codes
 // before it are read.  But a decoder that starts in mid-stream falls into step
@@ -23,18 +24,21 @@
 //            output from here;
 //   CRC-32   66 bytes per thread, counted from the member's end (zero bytes
 //            in front leave a CRC register of zero as it is), combined in GF(2).
-// Members that this form does not hold (more than 0xff00 bytes, many blocks)
-// and members with anything invalid in them go to warp_member, where lane 0
-// decodes the stream code by code (inflate.cuh) and gives the status.
+// A second kernel, one warp per member (left_kernel: lane 0 decodes the stream
+// code by code, inflate.cuh, the warp writes its bytes), takes what the first
+// leaves: members that this form does not hold (more than 0xff00 bytes, as some
+// writers fill them, or many blocks), members with anything invalid in them (it
+// gives their status), and those that many warps finish sooner than the CTAs
+// (cta_takes, Rounds).
 // Every code's reads stay in the staged input and every cell in the member:
 // sizes are checked before they are used.
 // Bound by latency: per member of 65280 bytes of FASTQ the sync rounds take
 // about 80 k cycles (segments of equal code lengths fall into step late), the
 // write pass 25 k, the resolve 54 k, the CRC 11 k; the next member's header and
 // tables (82 k by one warp) are read meanwhile.  128 MB in 1961 members (zlib
-// level 6): 1.42 ms, 1.45 with one literal per table entry; segments of 96 bits 1.87, of 160 or 288 bits 1.46 and
-// 1.49 ms, 3 to 5 checkpoints per segment that stop a second decode early 1.74
-// ms; one warp per member, decoded by one lane throughout, took 6.2 ms.
+// level 6): 1.42 ms, 1.45 with one literal per table entry; segments of 96 bits
+// 1.87, of 160 or 288 bits 1.46 and 1.49 ms, 3 to 5 checkpoints per segment that
+// stop a second decode early 1.74 ms; all members in left_kernel 6.2 ms.
 #include <string>
 
 #include "bgzf_inflate.cuh"
@@ -46,6 +50,8 @@ namespace {
 constexpr int THREADS = 992;              // that work on a member; one more warp reads the next member's header
 constexpr int WARPS = THREADS / 32;
 constexpr int CTA_THREADS = THREADS + 32;
+constexpr int LEFT_WARPS = 4;             // per block of left_kernel
+constexpr uint32_t S_LEFT = 0xffffffffu;  // the status of a member that is left to it
 constexpr uint32_t CRC_POLY = 0xEDB88320u;
 
 struct __align__(16) WarpSmem {
@@ -102,16 +108,14 @@ __device__ uint32_t warp_crc(const uint8_t* out, uint32_t n, const uint32_t* crc
     return r;
 }
 
-// Member m by the warp; returns its status (valid in lane 0).
+// Member m by the warp, its spans checked; returns its status (valid in lane 0).
 __device__ uint32_t warp_member(const bgzf_inflate::Job& j, uint32_t m, WarpSmem& S, const uint32_t* crc_tab,
                                 int lane) {
-    const uint64_t so = j.src_off[m], sl = j.src_len[m], dof = j.dst_off[m], isz = j.isize[m];
-    if (so > j.in_bytes || sl > j.in_bytes - so || dof > j.out_bytes || isz > j.out_bytes - dof)
-        return bgzf_inflate::S_SPAN;
-    const uint8_t* in = j.in + so;
-    uint8_t* out = j.out + dof;
+    const uint8_t* in = j.in + j.src_off[m];
+    uint8_t* out = j.out + j.dst_off[m];
+    const uint32_t isz = j.isize[m];
     inflate::Stream st;  // lane 0's decoder state
-    if (lane == 0) inflate::stream_init(st, in, static_cast<uint32_t>(sl), static_cast<uint32_t>(isz));
+    if (lane == 0) inflate::stream_init(st, in, j.src_len[m], isz);
     for (;;) {
         if (lane == 0) {
             S.o0 = st.o;
@@ -149,6 +153,23 @@ __device__ uint32_t warp_member(const bgzf_inflate::Job& j, uint32_t m, WarpSmem
     return c == j.crc[m] ? 0u : bgzf_inflate::S_CRC;
 }
 
+// The members that the CTAs left.
+__global__ void __launch_bounds__(LEFT_WARPS * 32) left_kernel(bgzf_inflate::Job j) {
+    __shared__ WarpSmem smem[LEFT_WARPS];
+    __shared__ uint32_t crc_tab[256];
+    bgzf_inflate::crc_table(crc_tab, static_cast<int>(threadIdx.x), LEFT_WARPS * 32);
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t n_warps = static_cast<uint64_t>(gridDim.x) * LEFT_WARPS;
+    for (uint64_t m = static_cast<uint64_t>(blockIdx.x) * LEFT_WARPS + warp; m < j.n; m += n_warps) {
+        if (j.status[m] != S_LEFT) continue;
+        __syncwarp();
+        const uint32_t s = warp_member(j, static_cast<uint32_t>(m), smem[warp], crc_tab, lane);
+        if (lane == 0) j.status[m] = s;
+        __syncwarp();
+    }
+}
+
 constexpr uint32_t MAX_BYTES = 0xff00;   // output bytes of a member in cells
 constexpr uint32_t SEG_WORDS = 7;        // bits per thread: an odd number of words, so the threads' reads spread over the banks
 constexpr uint32_t SEG_BITS = 32 * SEG_WORDS;
@@ -181,13 +202,11 @@ struct Head {
     uint32_t in[HEAD_WORDS + 2];
     uint32_t pos;   // bit of the stream after the header
     uint32_t type, last, nlit, ndist, ok;
+    uint32_t flat;  // all but an eighth of the literal codes are of one length
 };
 
 struct __align__(16) Smem {
-    union {
-        uint16_t cell[MAX_BYTES];
-        WarpSmem warp;  // warp_member's
-    } u;
+    uint16_t cell[MAX_BYTES];
     Head head[2];  // the member's, and the next one's
     uint32_t in[IN_WORDS];
     uint32_t starts[(MAX_BYTES + 31) / 32];  // a code's output (or a piece of it) starts at this byte
@@ -197,6 +216,8 @@ struct __align__(16) Smem {
     uint32_t part[32];
     uint32_t carry_at, carry_cell;  // the code that a strip begins in
     uint32_t first_flag;
+    uint32_t mine[CTA_THREADS / 32];  // which of the CTA's next members it takes
+    uint32_t stopped;                 // it takes no more of them
 };
 
 // Barriers of the THREADS that work on a member (the header warp takes none).
@@ -371,8 +392,8 @@ __device__ __forceinline__ uint32_t decode_bits(Smem& S, const Head& H, bool on,
             pos += used;
             if (flag == F_NONE) {
                 if (WRITE && two) {
-                    S.u.cell[o] = static_cast<uint16_t>(v);
-                    S.u.cell[o + 1] = static_cast<uint16_t>(0xff00u | (e >> 24));
+                    S.cell[o] = static_cast<uint16_t>(v);
+                    S.cell[o + 1] = static_cast<uint16_t>(0xff00u | (e >> 24));
                     atomicOr(S.starts + (o >> 5), 3u << (o & 31));
                     if ((o & 31) == 31) atomicOr(S.starts + (o >> 5) + 1, 1u);
                 } else if (WRITE) {
@@ -380,7 +401,7 @@ __device__ __forceinline__ uint32_t decode_bits(Smem& S, const Head& H, bool on,
                     // 4 dist ... bytes, each of which copies from v on, where
                     // the pieces before it have put as many
                     for (;;) {
-                        S.u.cell[o] = static_cast<uint16_t>(v);
+                        S.cell[o] = static_cast<uint16_t>(v);
                         atomicOr(S.starts + (o >> 5), 1u << (o & 31));
                         if (len <= dist) break;
                         o += dist;
@@ -502,7 +523,10 @@ __device__ void read_head(Head& H, const uint8_t* in, uint32_t n, uint32_t pos, 
         ok = canon_build(H.cl, H.lens, static_cast<int>(nlit), 1, lane);
         ok = ok && canon_build(H.cd, H.lens + nlit, static_cast<int>(ndist), 1, lane);
     }
+    const uint32_t of_length = ok && type == 2 && lane >= 1 && lane < 16 ? H.cl.count[lane] << (15 - lane) : 0;
+    const uint32_t flat = __any_sync(0xffffffffu, of_length > (7u << 12));
     if (lane == 0) {
+        H.flat = flat;
         H.pos = 8 * base + at;
         H.type = type;
         H.last = w.lo & 1;
@@ -536,31 +560,64 @@ __device__ __forceinline__ bool member_spans(const bgzf_inflate::Job& j, uint32_
     return !(so > j.in_bytes || sl > j.in_bytes - so || dof > j.out_bytes || isz > j.out_bytes - dof);
 }
 
-// Whether it is of a size that cta_member takes.
-__device__ __forceinline__ bool member_fits(const bgzf_inflate::Job& j, uint32_t m) {
-    return j.isize[m] >= 4 && j.isize[m] <= MAX_BYTES && j.src_len[m] >= 1 && j.src_len[m] <= (1u << 26);
+// Whether a CTA takes member m of a call of j.n; its spans are checked.  A CTA
+// decodes a large member up to 40 times as fast as a warp, but 148 members are in
+// CTAs at a time and 9472 in warps, and a small member's time is the CTA's own.
+// So: the CTAs' turns at members like this one against one member's time in a
+// warp, and an SM's time for a member either way, in nanoseconds by the kind of
+// its first block (fitted to members of 512 .. 65280 bytes: FASTQ at level 6,
+// zeros, base-64 text, fixed codes, whose segments fall into step late, and stored
+// noise).  16000 members of 512 bytes of FASTQ: 1.5 ms in warps, 5.3 in CTAs;
+// 2368 of 4096 bytes 0.82 and 0.95, of 16384 bytes 2.5 and 1.15.  8000 members of
+// 65280 bytes of zeros 2.1 and 6.8 ms, of stored noise 2.2 and 3.5, 2000 of
+// FASTQ in fixed codes 9.8 and 18.3.
+__device__ __forceinline__ bool cta_takes(const bgzf_inflate::Job& j, uint32_t m) {
+    const uint64_t isz = j.isize[m], src = j.src_len[m];
+    if (isz < 4 || isz > MAX_BYTES || src < 1 || src > (1u << 26)) return false;
+    const uint32_t type = j.in[j.src_off[m]] >> 1 & 3;
+    const uint64_t cta = type == 0 ? 17000 + isz * 3 / 4 : type == 1 ? 45000 + src * 45 : 50000 + isz * 9 / 10;  // a turn
+    const uint64_t warp = type == 0 ? 10000 + isz * 8 : 130000 + src * 260 + isz * 6;  // the first members in warps
+    const uint64_t sm = type == 0 ? 4000 + isz * 9 / 16 : 9000 + src * 17 + isz / 2;   // one more, all warps at work
+    return j.n * cta <= gridDim.x * warp || cta <= sm;
 }
 
-// Member m by THREADS threads, from its first block's header H on; false:
-// nothing written, warp_member has to do it.  status: the CRC's outcome.
-__device__ bool cta_member(const bgzf_inflate::Job& j, uint32_t m, Smem& S, Head& H, uint32_t t, uint32_t& status) {
+// Codes that fall into step late, beyond four turns of the CTAs: there a member
+// whose literal codes are all but an eighth of one length (base-64, hexadecimal
+// text; FASTQ's are up to 0.8) is left, and so is one whose sync rounds go past
+// USUAL (FASTQ takes 3 to 12) and what is left of the CTA's SPARE.  A CTA that
+// left one leaves its later ones too: beside it in other warps they cost nothing.
+// 2000 members of base-64 text take 17 ms in warps, up to 51 in CTAs (850 rounds).
+struct Rounds {
+    static constexpr int USUAL = 32, SPARE = 64;
+    bool limited, out;  // out: the CTA leaves the rest
+    int over;           // spent beyond USUAL
+    __device__ __forceinline__ int limit() const { return limited ? USUAL + max(0, SPARE - over) : THREADS + 1; }
+};
+
+// Member m by THREADS threads, from its first block's header H on; returns its
+// status (valid in thread 0), S_LEFT: nothing written.
+__device__ uint32_t cta_member(const bgzf_inflate::Job& j, uint32_t m, Smem& S, Head& H, uint32_t t, Rounds& rounds) {
     const uint8_t* in = j.in + j.src_off[m];
     uint8_t* out = j.out + j.dst_off[m];
     const uint32_t n = j.src_len[m], isz = j.isize[m], lane = t & 31, warp = t >> 5;
+    if (rounds.limited && H.flat) {
+        rounds.out = true;
+        return S_LEFT;
+    }
     for (uint32_t i = t; i < (MAX_BYTES + 31) / 32; i += THREADS) S.starts[i] = 0;
     work_sync();
     uint32_t made = 0;  // bytes whose cells are written
     for (int blocks = 0;; ++blocks) {
-        if (!H.ok || blocks == MAX_BLOCKS) return false;
+        if (!H.ok || blocks == MAX_BLOCKS) return S_LEFT;
         const bool last = H.last;
         uint32_t pos = H.pos;  // bit of the stream
         if (H.type == 0) {
             const uint32_t p = (pos + 7) >> 3;  // LEN, NLEN, the bytes
-            if (p + 4 > n) return false;
+            if (p + 4 > n) return S_LEFT;
             const uint32_t len = in[p] | in[p + 1] << 8, nlen = in[p + 2] | in[p + 3] << 8;
-            if (len != (~nlen & 0xffffu) || len > n - p - 4 || len > isz - made) return false;
+            if (len != (~nlen & 0xffffu) || len > n - p - 4 || len > isz - made) return S_LEFT;
             for (uint32_t i = t; i < len; i += THREADS) {
-                S.u.cell[made + i] = static_cast<uint16_t>(0xff00u | in[p + 4 + i]);
+                S.cell[made + i] = static_cast<uint16_t>(0xff00u | in[p + 4 + i]);
                 atomicOr(S.starts + ((made + i) >> 5), 1u << ((made + i) & 31));
             }
             made += len;
@@ -568,7 +625,7 @@ __device__ bool cta_member(const bgzf_inflate::Job& j, uint32_t m, Smem& S, Head
         } else {
             // the block's codes, THREADS segments at a time
             for (bool ended = false; !ended;) {
-                if (pos >= 8 * n) return false;
+                if (pos >= 8 * n) return S_LEFT;
                 const uint32_t base = (pos >> 3) & ~3u, at = pos - 8 * base;  // `at`: bit of the staged input
                 stage_input(S.in, IN_WORDS, in, n, base, t, THREADS);
                 work_sync();
@@ -577,8 +634,9 @@ __device__ bool cta_member(const bgzf_inflate::Job& j, uint32_t m, Smem& S, Head
                 uint32_t start = at + t * SEG_BITS, end = 0, bytes = 0;
                 uint32_t flag = decode_bits<false>(S, H, true, start, limit, n_bits, end, bytes);
                 uint32_t f = THREADS;  // the first thread that met an end or no code
-                bool settled = false;  // after at most one round per thread
-                for (int round = 0; round <= THREADS && !settled; ++round) {
+                bool settled = false;  // after at most one round per thread, if it may spend them
+                int round = 0;
+                for (const int most = rounds.limit(); round < most && !settled; ++round) {
                     if (t == 0) S.first_flag = THREADS - 1;
                     S.end[t] = end;
                     work_sync();
@@ -597,33 +655,35 @@ __device__ bool cta_member(const bgzf_inflate::Job& j, uint32_t m, Smem& S, Head
                     }
                     settled = !work_or(again);
                 }
+                rounds.over += max(0, round - Rounds::USUAL);
+                if (!settled) rounds.out = rounds.limited;
                 if (t > f) bytes = 0;
                 const bool bad = work_or(t == f && flag == F_BAD);
                 ended = work_or(t == f && flag == F_END);
-                if (bad || !settled) return false;
+                if (bad || !settled) return S_LEFT;
                 uint32_t total;
                 uint32_t o = made + block_scan(S, bytes, t, total);
                 const uint32_t reached = S.end[f];
-                if (reached > n_bits || total > isz - made) return false;
+                if (reached > n_bits || total > isz - made) return S_LEFT;
                 const uint32_t f2 = decode_bits<true>(S, H, t <= f, start, limit, n_bits, end, o);
-                if (work_or(t <= f && f2 == F_BAD)) return false;
+                if (work_or(t <= f && f2 == F_BAD)) return S_LEFT;
                 made += total;
                 pos = 8 * base + reached;
             }
         }
         if (last) break;
-        if (pos >= 8 * n) return false;
+        if (pos >= 8 * n) return S_LEFT;
         work_sync();  // the block's tables are done with
         if (warp == 0) read_head(H, in, n, pos, static_cast<int>(lane));
         work_sync();
         fill_tables(H, t, THREADS, [] { work_sync(); });
         work_sync();
     }
-    if (made != isz) return false;
+    if (made != isz) return S_LEFT;
     work_sync();
     // resolve, a strip at a time, four bytes per thread
-    volatile uint16_t* cell = S.u.cell;
-    volatile uint64_t* cell4 = reinterpret_cast<volatile uint64_t*>(S.u.cell);
+    volatile uint16_t* cell = S.cell;
+    volatile uint64_t* cell4 = reinterpret_cast<volatile uint64_t*>(S.cell);
     const bool aligned = (reinterpret_cast<uintptr_t>(out) & 3) == 0;
     if (t == 0) S.carry_at = S.carry_cell = 0;
     for (uint32_t strip = 0; strip < isz; strip += STRIP) {
@@ -699,52 +759,82 @@ __device__ bool cta_member(const bgzf_inflate::Job& j, uint32_t m, Smem& S, Head
         c = lane ? S.part[lane - 1] : 0;
         for (int k = 0; k < 5; ++k) c = gf2_mul(c, S.xpow[5 + k]) ^ __shfl_down_sync(0xffffffffu, c, 1 << k);
     }
-    status = ~c == j.crc[m] ? 0u : bgzf_inflate::S_CRC;
-    return true;
+    return ~c == j.crc[m] ? 0u : bgzf_inflate::S_CRC;
 }
 
 __global__ void __launch_bounds__(CTA_THREADS, 1) bgzf_inflate_kernel(bgzf_inflate::Job j) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
     Smem& S = *reinterpret_cast<Smem*>(smem_raw);
     const uint32_t t = threadIdx.x;
-    bgzf_inflate::crc_table(S.crc[0], static_cast<int>(t), CTA_THREADS);
-    if (t == 0) {
-        uint32_t x = gf2_xpow(8ull * CRC_BYTES);
-        for (int k = 0; k < 10; ++k) {
-            S.xpow[k] = x;
-            x = gf2_mul(x, x);
-        }
-    }
-    __syncthreads();
-    if (t < 256) {
-        uint32_t c = S.crc[0][t];
-        for (int k = 1; k < 4; ++k) {
-            c = (c >> 8) ^ S.crc[0][c & 255];
-            S.crc[k][t] = c;
-        }
-    }
-    // the last warp reads the first header of member m + gridDim.x while the
-    // others work on member m
-    auto header_of = [&](uint32_t m, Head& H) {
-        if (m >= j.n || !member_spans(j, m) || !member_fits(j, m)) return;
-        read_head(H, j.in + j.src_off[m], j.src_len[m], 0, static_cast<int>(t - THREADS));
-        fill_tables(H, t - THREADS, 32, [] { __syncwarp(); });
-    };
-    if (t >= THREADS) header_of(blockIdx.x, S.head[0]);
-    __syncthreads();
-    uint32_t which = 0;
-    for (uint32_t m = blockIdx.x; m < j.n; m += gridDim.x, which ^= 1) {
-        if (t >= THREADS) {
-            if (j.n - m > gridDim.x) header_of(m + gridDim.x, S.head[which ^ 1]);
-        } else {
-            uint32_t status = bgzf_inflate::S_SPAN;
-            if (member_spans(j, m) && !(member_fits(j, m) && cta_member(j, m, S, S.head[which], t, status))) {
-                work_sync();
-                if (t < 32) status = warp_member(j, m, S.u.warp, S.crc[0], static_cast<int>(t));
+    bool tables = false;
+    auto make_tables = [&] {  // for the first member that the CTA takes
+        bgzf_inflate::crc_table(S.crc[0], static_cast<int>(t), CTA_THREADS);
+        if (t == 0) {
+            uint32_t x = gf2_xpow(8ull * CRC_BYTES);
+            for (int k = 0; k < 10; ++k) {
+                S.xpow[k] = x;
+                x = gf2_mul(x, x);
             }
-            if (t == 0) j.status[m] = status;
         }
         __syncthreads();
+        if (t < 256) {
+            uint32_t c = S.crc[0][t];
+            for (int k = 1; k < 4; ++k) {
+                c = (c >> 8) ^ S.crc[0][c & 255];
+                S.crc[k][t] = c;
+            }
+        }
+        tables = true;
+    };
+    if (t == 0) S.stopped = 0;
+    Rounds rounds{j.n > 4 * static_cast<uint64_t>(gridDim.x), false, 0};
+    // the CTA's members are blockIdx.x + i * gridDim.x; which of the next
+    // CTA_THREADS it takes is looked up for all of them at once
+    for (uint64_t base = 0; blockIdx.x + base * gridDim.x < j.n; base += CTA_THREADS) {
+        auto member = [&](int i) { return static_cast<uint32_t>(blockIdx.x + (base + i) * gridDim.x); };
+        bool take = false;
+        if (blockIdx.x + (base + t) * gridDim.x < j.n) {
+            const uint32_t m = member(static_cast<int>(t));
+            const bool spans = member_spans(j, m);
+            take = spans && cta_takes(j, m);
+            if (!take) j.status[m] = spans ? S_LEFT : bgzf_inflate::S_SPAN;
+        }
+        const uint32_t word = __ballot_sync(0xffffffffu, take);
+        if ((t & 31) == 0) S.mine[t >> 5] = word;
+        __syncthreads();
+        auto after = [&](int i) {  // the first one taken after i, -1: none
+            for (int w = ++i >> 5; w < CTA_THREADS / 32; ++w, i = 0) {
+                const uint32_t x = S.mine[w] >> (i & 31) << (i & 31);
+                if (x) return 32 * w + __ffs(static_cast<int>(x)) - 1;
+            }
+            return -1;
+        };
+        // the last warp reads the next member's first header while the others
+        // work on this one
+        auto header_of = [&](int i, Head& H) {
+            if (i < 0 || S.stopped) return;
+            const uint32_t m = member(i);
+            read_head(H, j.in + j.src_off[m], j.src_len[m], 0, static_cast<int>(t - THREADS));
+            fill_tables(H, t - THREADS, 32, [] { __syncwarp(); });
+        };
+        int i = after(-1);
+        if (i >= 0 && !tables) make_tables();
+        if (t >= THREADS) header_of(i, S.head[0]);
+        __syncthreads();
+        for (uint32_t which = 0; i >= 0; which ^= 1) {
+            const int next = after(i);
+            if (t >= THREADS) {
+                header_of(next, S.head[which ^ 1]);
+            } else {
+                const uint32_t m = member(i);
+                const uint32_t status = S.stopped ? S_LEFT : cta_member(j, m, S, S.head[which], t, rounds);
+                if (t == 0) j.status[m] = status;
+            }
+            __syncthreads();
+            if (t == 0 && rounds.out) S.stopped = 1;
+            __syncthreads();
+            i = next;
+        }
     }
 }
 
@@ -762,7 +852,10 @@ int bgzf_inflate_enqueue(const bgzf_inflate::Job& j, int sm_count, cudaStream_t 
                  "inflate smem");
     bgzf_inflate_kernel<<<j.n < sms ? j.n : sms, CTA_THREADS, sizeof(Smem), st>>>(j);
     check_launch(cudaGetLastError(), "bgzf_inflate_kernel");
-    return 1;
+    const uint32_t want = (j.n + LEFT_WARPS - 1) / LEFT_WARPS;
+    left_kernel<<<want < sms * 16 ? want : sms * 16, LEFT_WARPS * 32, 0, st>>>(j);
+    check_launch(cudaGetLastError(), "left_kernel");
+    return 2;
 }
 
 }  // namespace ma

@@ -120,8 +120,8 @@ class _DeviceFeed:
     """Uncompressed bytes of one BGZF FASTQ file in HBM, inflated on the
     device: fill() reads whole members (their compressed bytes only cross
     PCIe) into a pinned buffer, copies them to the device and inflates them
-    behind the bytes left from the last piece (ma_bgzf_inflate_device, one
-    CTA per member); consume(n) drops the first n bytes, moving the rest to
+    behind the bytes left from the last piece (ma_bgzf_inflate_device, a
+    CTA or a warp per member); consume(n) drops the first n bytes, moving the rest to
     the front on the device.  Same interface as _Feed, with `dev` in place
     of `pin`.  A member that is not BGZF (an appended plain gzip member) is
     inflated on the host and copied in."""

@@ -205,3 +205,70 @@ def test_literals_in_pairs(ctx, symbols):
     status, got, _, _ = _inflate_raw(ctx, [(p, len(d), zlib.crc32(d)) for p, d in cases])
     for i, ((_, data), s, g) in enumerate(zip(cases, status, got)):
         assert s == 0 and g == data, i
+
+
+def _members(kind):
+    """One to eight deflate payloads of a kind of member and their bytes."""
+    import base64
+    import zlib
+
+    rng = np.random.default_rng(12)
+    text = random_fastq(13, 6000)
+    noise = rng.integers(0, 256, 8 * 65280, dtype=np.uint8).tobytes()
+    size, data, level, strategy = {
+        "small": (512, text, 6, zlib.Z_DEFAULT_STRATEGY), "whole": (65536, text, 6, zlib.Z_DEFAULT_STRATEGY),
+        "zeros": (65280, bytes(65280), 6, zlib.Z_DEFAULT_STRATEGY), "stored": (4096, noise, 0, zlib.Z_DEFAULT_STRATEGY),
+        "fixed": (65280, text, 6, zlib.Z_FIXED), "base64": (65280, base64.b64encode(noise), 6, zlib.Z_HUFFMAN_ONLY)}[kind]
+    made = []
+    for a in range(0, min(len(data), 8 * size) - size + 1, size):
+        c = zlib.compressobj(level, zlib.DEFLATED, -15, 8, strategy)
+        made.append((c.compress(data[a:a + size]) + c.flush(), data[a:a + size]))
+    return made
+
+
+@pytest.mark.parametrize("kind,many,most", [("whole", 2368, 4), ("small", 2368, 4.5), ("stored", 8000, 10),
+                                            ("zeros", 2368, 8), ("fixed", 2368, 11), ("base64", 2368, 8)])
+def test_many_members_of_any_kind_run_side_by_side(ctx, kind, many, most):
+    """Members that a CTA does not hold, that it is slow at, or that are mostly
+    its own overhead: a call of 16 members an SM (54 stored ones) takes at most
+    `most` times one of a member an SM, 16 (54) times where each had an SM to
+    itself.  The measured factors are 1.4, 2.3, 5.5, 4.8, 7 and 4.6."""
+    import torch
+    import zlib
+
+    made = _members(kind)
+    took = []
+    for n in (148, many):
+        src, so, sl = bytearray(), [], []
+        for p, _ in made:
+            so.append(len(src))
+            sl.append(len(p))
+            src += p
+        i = np.arange(n) % len(made)
+        size = len(made[0][1])
+        put = lambda v, t: torch.from_numpy(np.asarray(v).astype(t)).cuda()  # noqa: E731
+        cols = [put(np.array(so)[i], np.int64), put(np.array(sl)[i], np.int32), put(np.arange(n) * size, np.int64),
+                put(np.full(n, size), np.int32),
+                put(np.array([zlib.crc32(d) for _, d in made], np.uint32).view(np.int32)[i], np.int32)]
+        d_in = torch.frombuffer(src, dtype=torch.uint8).cuda()
+        d_out = torch.zeros(n * size, dtype=torch.uint8, device="cuda")
+        status = torch.full((n,), 77, dtype=torch.int32, device="cuda")
+        stream = torch.cuda.Stream()
+        torch.cuda.synchronize()
+        times = []
+        for _ in range(7):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record(stream)
+            _lib.check(_lib.lib.ma_bgzf_inflate_device(ctx.handle, d_in.data_ptr(), len(src),
+                                                       *[c.data_ptr() for c in cols], n, d_out.data_ptr(), n * size,
+                                                       status.data_ptr(), stream.cuda_stream), ctx.handle)
+            b.record(stream)
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+        took.append(float(np.median(times[2:])))
+        assert not status.any()
+        want = torch.frombuffer(bytearray(b"".join(d for _, d in made)), dtype=torch.uint8).cuda()
+        whole = n // len(made) * len(made) * size
+        assert torch.equal(d_out[:whole].view(-1, want.numel()), want.expand(whole // want.numel(), -1))
+        assert torch.equal(d_out[whole:], want[:n * size - whole])
+    assert took[1] < most * took[0], took
