@@ -272,3 +272,44 @@ def test_many_members_of_any_kind_run_side_by_side(ctx, kind, many, most):
         assert torch.equal(d_out[:whole].view(-1, want.numel()), want.expand(whole // want.numel(), -1))
         assert torch.equal(d_out[whole:], want[:n * size - whole])
     assert took[1] < most * took[0], took
+
+
+def _fixed_block(data, last):
+    """Bits of a block of literals in the fixed codes, first bit first."""
+    bits = [last, 1, 0]
+    for x in data:
+        code, n = (0x30 + x, 8) if x < 144 else (0x190 + x - 144, 9)
+        bits += [code >> (n - 1 - k) & 1 for k in range(n)]
+    return bits + [0] * 7
+
+
+def test_edges_of_segments_strips_and_rounds(ctx):
+    """Members that end around a thread's 66 bytes of the CRC, around strips of
+    3968 bytes and around the 992 * 224 bits that the threads read at once;
+    copies and runs across a strip's edge."""
+    import zlib
+
+    text = random_fastq(14, 400)
+    cases = []
+
+    def add(data, level=9):
+        c = zlib.compressobj(level, zlib.DEFLATED, -15)
+        cases.append((c.compress(data) + c.flush(), data))
+
+    for n in (65, 66, 67, 131, 132, 133, 3967, 3968, 3969, 7935, 7936, 7937, 65279):
+        add(text[:n])
+    for at in (3900, 3960, 3965, 3967, 3968, 3969):
+        for run in (b"F" * 300, b"ACG" * 120, text[:257], text[at - 5:at] * 60):
+            add(text[:at] + run + text[:50])
+    # 27776 codes of 8 bits fill the 992 segments: the end-of-block code before,
+    # up to and past their end, then another block
+    for a, b in ((27775, 0), (27774, 1), (27773, 2), (27776, 0), (27770, 4), (27777, 0)):
+        data = bytes([65 + k % 50 for k in range(a)]) + bytes([200] * b)
+        bits = _fixed_block(data, 0) + _fixed_block(text[:100], 1)
+        cases.append((np.packbits(np.array(bits, np.uint8), bitorder="little").tobytes(), data + text[:100]))
+    for p, d in cases:
+        assert zlib.decompress(p, -15) == d
+    for lead in (0, 1):
+        status, got, _, _ = _inflate_raw(ctx, [(p, len(d), zlib.crc32(d)) for p, d in cases], lead)
+        for i, ((_, d), s, g) in enumerate(zip(cases, status, got)):
+            assert s == 0 and g == d, i
