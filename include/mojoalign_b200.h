@@ -318,7 +318,9 @@ int ma_last_launch_count(const ma_ctx* ctx);
  *   wave_loci_per_read    wavefront locus list capacity per read of the
  *                         batch (1..64, default 4; at least 1024 entries);
  *                         reads whose loci do not fit a round wait for the
- *                         next one, and for the stage-2 warps after the last.
+ *                         next one, or go to the stage-2 warps (after the last
+ *                         one, and when the round's loci exceed the list by
+ *                         more than half).
  *   wave_max_rounds       wavefront rounds before the reads still active
  *                         go to the stage-2 warps (0 = as many as the
  *                         longest read needs, default).

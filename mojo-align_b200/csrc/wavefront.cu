@@ -18,8 +18,9 @@
 // in the reference's order, so pruning against that best and taking the
 // minimum key over the round gives the reference's hit.  A read whose loci
 // do not fit the list is left out of its round (its memo and best roll
-// back) and starts the next one from the same endpoint; reads still active
-// after the last round are finished by the stage-2 warp kernel.
+// back) and starts the next one from the same endpoint, or where the list is
+// far too short goes to the stage-2 warp kernel, which also finishes the reads
+// still active after the last round.
 #include <cuda_runtime.h>
 
 #include "ma_device.cuh"
@@ -573,6 +574,14 @@ __global__ void __launch_bounds__(256, 4) wf_finalize_kernel(DevIndex ix, DevRea
     const uint32_t n_act = w.counters[C_ACTIVE];
     const int lane = threadIdx.x & 31;
     const uint32_t stride = gridDim.x * blockDim.x;
+    // Reads that the list had no room for wait for the next round when it held
+    // two thirds of what the round asked for.  With less room most reads would
+    // wait, and their searches run again round after round: 400 k pairs 2x150 with
+    // 1, 2 or (rounds of 32 endpoints) 4 entries per read 9.3, 6.6 and 5.3 ms,
+    // 18.4, 11.9 and 6.8 when all wait.  With nearly enough stage 2 takes longer:
+    // 3.3 and 3.7 ms with 3 entries and with 4 (2 endpoints in the first round),
+    // 3.5 and 5.4 when none waits.
+    const bool wait = !last_round && 2 * *loci_count(w) <= 3 * w.locus_cap;
     if constexpr (S) {
         if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&w.counters[C_ROUNDS], n_act);
     }
@@ -588,10 +597,10 @@ __global__ void __launch_bounds__(256, 4) wf_finalize_kernel(DevIndex ix, DevRea
             const int n_end = endpoint_count(P, qlen);
             if (w.overflow[r]) {
                 // left out of this round: roll back; the next round takes the
-                // same endpoints up again, stage 2 after the last one
+                // same endpoints up again, or stage 2 does
                 w.overflow[r] = 0;
                 w.memo_next[r] = w.memo_n[r];
-                if (last_round) to_stage2 = true;
+                if (!wait) to_stage2 = true;
                 else to_next = true;
             } else {
                 const uint32_t mn = w.memo_next[r];

@@ -71,3 +71,30 @@ def test_young_repeats_parameter_sweep(ctx, young_repeat_ref, params):
     fa, prefix = young_repeat_ref
     rb = _reads(fa, 3000, True, 250, 14, len_fixed=250, conv_non_cpg=0.97, sub_rate=0.01)
     compare(prefix, ctx, rb.bases, rb.lens, rb.n1, True, 250, params, k=12, k3=19)
+
+
+@pytest.mark.parametrize("n1,max_len", [(20000, 150), (6000, 250)])
+def test_a_list_far_too_short_repeats_few_searches(ctx, repeat_ref, n1, max_len):
+    """Rounds that ask for several times what the locus list holds hand the
+    reads left out to stage 2: their searches are not run again round after
+    round (1.5 times the Occ lines of a list with room, 3 when all wait)."""
+    from mojoalign_b200 import map_batch
+    from test_gpu_parity import gpu_index
+
+    fa, prefix = repeat_ref
+    rb = _reads(fa, n1, True, max_len, 3, len_fixed=max_len, conv_non_cpg=0.97)
+    short, room = (2, 1, 0, 2, 1, 1, 32, 1, 0, 0), (2, 1, 0, 2, 1, 1, 32, 64, 0, 0)
+    if n1 < 10000:
+        compare(prefix, ctx, rb.bases, rb.lens, n1, True, max_len, BENCH_PARAMS, k=12, k3=19, tunings=[short, room])
+    gi = gpu_index(ctx, prefix, 12, 19)
+    occ_lines = []
+    for tuning in (short, room):
+        ctx.set_tuning(*tuning)
+        ctx.set_profiling(2)
+        try:
+            map_batch(ctx, gi, rb.bases, rb.lens, n1, True, max_len, "C2T", "G2A", BENCH_PARAMS)
+            occ_lines.append(ctx.traffic()[0])
+        finally:
+            ctx.set_profiling(0)
+            ctx.set_tuning()
+    assert occ_lines[0] < 2.2 * occ_lines[1], occ_lines
