@@ -295,8 +295,7 @@ int ma_last_launch_count(const ma_ctx* ctx);
  *                         selection), stage1_endpoints endpoints per read in
  *                         the first round and wave_endpoints in each later
  *                         one; reads left over go to the stage-2 warps.  The
- *                         three were different forms of the passes once and
- *                         run the same kernels (2 is the default).
+ *                         three run the same kernels (2 is the default).
  *   stage1_endpoints      endpoints stage 1 (or the first round) covers
  *                         (default 1).
  *   stage2_blocks_per_sm  persistent blocks per SM for stage 2 (0 = the
@@ -329,10 +328,12 @@ int ma_last_launch_count(const ma_ctx* ctx);
  *                         fuller rounds for the reads that stay active
  *                         longest; default); 0: every later round covers
  *                         wave_endpoints.
- * With stage1_endpoints and all wave_* fields at their defaults ma_map_batch
- * and ma_map_batch_device fit the rounds to the call: batches too small to
- * fill the GPU take one round, or two to three wide ones, and the locus list
- * is longer (up to 256 entries per read within 64 MB, 8 within 512 MB).
+ * With stage1_endpoints and all wave_* fields at their defaults (set or left)
+ * ma_map_batch and ma_map_batch_device fit the rounds to the call: batches too
+ * small to fill the GPU take one round, or two to three wide ones, and the
+ * locus list is longer (up to 256 entries per read within 64 MB, 8 within 512
+ * MB).  A server's groups run the rounds as they are set: a longer list would
+ * leave less of its memory budget for reads.
  */
 typedef struct ma_tuning {
     int32_t seed_kernel;

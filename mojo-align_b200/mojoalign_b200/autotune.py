@@ -11,7 +11,13 @@ search threads, so the round width is the warps-per-read choice: 4, 8 and
 16 endpoints pack 8, 4 and 2 reads per warp (64, 32, 16 reads per 256-thread
 CTA), 32, 64 and 128 endpoints give each read 1, 2 and 4 warps (8, 4 and 2
 reads per CTA).  The stage-2 warps take one read each.  seed_kernels 2, 3 and 4 name
-the same wavefront passes.
+the same wavefront passes, so one of them is swept.
+
+A wavefront tuning whose first round, round width, list length, round limit and
+growth are the defaults (1, 8, 4, 0, 1) is fitted to the size of each call: such
+a candidate is timed with the rounds that fit the sample, and a call of another
+size runs the rounds that fit that one.  The result says so (TuneResult.fitted);
+a sample as large as the calls to come times what they will run.
 
 The seed stride is not swept: it decides which right endpoints are tried
 (linear_gpu_fm.mojo:1828) and so changes results.
@@ -28,7 +34,7 @@ from .params import FmParams
 DEFAULT_CANDIDATES = [
     (0, 1, 0, 1, 16, 32, 32),
     (1, 1, 0, 2, 1, 1, 32),
-    (2, 1, 0, 0, 1, 1, 8, 4, 0, 1),
+    (2, 1, 0, 0, 1, 1, 8, 4, 0, 1),    # fitted to the call
     (2, 1, 0, 1, 1, 1, 8, 4, 0, 1),
     (2, 1, 0, 2, 1, 1, 8, 4, 0, 1),
     (2, 1, 0, 0, 1, 1, 16, 4, 0, 0),
@@ -40,21 +46,12 @@ DEFAULT_CANDIDATES = [
     (2, 1, 0, 1, 1, 1, 8, 16, 0, 1),
     (2, 2, 0, 1, 1, 1, 8, 16, 0, 1),
     (2, 1, 0, 2, 1, 1, 8, 16, 0, 1),
+    (2, 2, 0, 2, 1, 1, 8, 16, 0, 1),
+    (2, 2, 0, 1, 1, 1, 8, 32, 0, 1),
     (2, 1, 0, 1, 1, 1, 32, 4, 0, 0),   # one warp per read and round
+    (2, 1, 0, 1, 1, 1, 32, 16, 0, 0),
     (2, 1, 0, 1, 1, 1, 64, 4, 0, 0),   # two warps per read
     (2, 1, 0, 1, 1, 1, 128, 4, 0, 0),  # four warps per read
-    (3, 1, 0, 1, 1, 1, 8, 4, 0, 1),
-    (3, 1, 0, 2, 1, 1, 8, 4, 0, 1),
-    (3, 1, 0, 1, 1, 1, 8, 16, 0, 1),
-    (3, 2, 0, 1, 1, 1, 8, 16, 0, 1),
-    (3, 1, 0, 2, 1, 1, 8, 16, 0, 1),
-    (3, 1, 0, 1, 1, 1, 32, 16, 0, 0),
-    (4, 1, 0, 1, 1, 1, 8, 4, 0, 1),
-    (4, 1, 0, 1, 1, 1, 8, 16, 0, 1),
-    (4, 2, 0, 1, 1, 1, 8, 16, 0, 1),
-    (4, 2, 0, 2, 1, 1, 8, 16, 0, 1),
-    (2, 2, 0, 1, 1, 1, 8, 32, 0, 1),   # locus lists of 32 per read
-    (4, 2, 0, 1, 1, 1, 8, 32, 0, 1),
 ]
 FIELDS = ("seed_kernel", "stage1_endpoints", "stage2_blocks_per_sm", "reg_level", "stage1_max_rows",
           "stage2_first_wave", "wave_endpoints", "wave_loci_per_read", "wave_max_rounds", "wave_growth")
@@ -63,11 +60,18 @@ FIELDS = ("seed_kernel", "stage1_endpoints", "stage2_blocks_per_sm", "reg_level"
 DEFAULTS = (2, 1, 0, 2, 1, 1, 8, 4, 0, 1)
 
 
+def fitted(candidate) -> bool:
+    """Whether the rounds of a candidate are fitted to the size of each call."""
+    c = tuple(candidate) + DEFAULTS[len(candidate):]
+    return c[0] >= 2 and c[1] == DEFAULTS[1] and c[6:] == DEFAULTS[6:]
+
+
 @dataclass
 class TuneResult:
     tuning: dict
     seed_ms: float
     all_ms: list
+    fitted: bool = False  # seed_ms is that of rounds fitted to the sample's size
 
 
 def autotune(ctx: GpuContext, index: GpuIndex, bases: np.ndarray, lens: np.ndarray, n1: int, paired: bool,
@@ -106,4 +110,5 @@ def autotune(ctx: GpuContext, index: GpuIndex, bases: np.ndarray, lens: np.ndarr
     ctx.set_tuning(*best)
     best = tuple(best) + tuple(DEFAULTS[len(best):])
     return TuneResult(dict(zip(FIELDS, best)), best_ms,
-                      [{"tuning": dict(zip(FIELDS, c)), "seed_ms": round(t, 3)} for t, c in timings])
+                      [{"tuning": dict(zip(FIELDS, c)), "seed_ms": round(t, 3), "fitted": fitted(c)}
+                       for t, c in timings], fitted(best))
