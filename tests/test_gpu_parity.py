@@ -393,3 +393,59 @@ def test_host_batch_with_some_outputs_page_locked(ctx, small_ref, pinned, n1, pa
         ctx.set_pipeline()
     for f in MapResult.FIELDS:
         assert np.array_equal(getattr(got, f), o[f]), f
+
+
+@pytest.mark.parametrize("n1,max_len", [(131_072, 40), (131_073, 40), (262_145, 40), (466_033, 40), (466_034, 40),
+                                        (1_100_000, 36)])
+def test_default_rounds_of_large_batches(ctx, small_ref, n1, max_len):
+    """Either side of the read counts at which the fitted rounds change: one
+    more round above 131072 reads, lists of 8 entries per read above 262144 and
+    the unchanged 1, 8, 16 .. rounds from 466034 on."""
+    fa, prefix = small_ref
+    rb = sim(fa, n1, False, max_len=max_len, seed=n1, len_fixed=max_len, len_min=max_len)
+    ctx.set_pipeline(n1, 0, n1, 1)  # the batch in one piece
+    try:
+        compare(prefix, ctx, rb.bases, rb.lens, n1, False, max_len, BENCH_PARAMS, tunings=[()])
+    finally:
+        ctx.set_pipeline()
+
+
+@pytest.mark.parametrize("n1", [131_072, 140_000])
+@pytest.mark.parametrize("length,waits", [(4_500, True), (20_000, False)])
+def test_default_rounds_with_a_full_locus_list(ctx, tmp_path, length, waits, n1):
+    """Reads of an element in 12 copies, all of them candidates of every seed,
+    in 18 % or 80 % of the text: the wide round asks for somewhat more rows than
+    its list holds (the reads left out run it again, or go to stage 2 where it
+    is the last) or for five times as many (they go to stage 2)."""
+    from mojoalign_b200 import build_index
+
+    rng = np.random.default_rng(1)
+    element = rng.integers(0, 4, length)
+    parts = [p for _ in range(12) for p in (rng.integers(0, 4, 25_000 - length), element)]
+    fa = tmp_path / "ref.fa"
+    fa.write_bytes(b">chr1\n" + np.frombuffer(b"ACGT", np.uint8)[np.concatenate(parts)].tobytes() + b"\n")
+    prefix = str(fa) + ".bwameth.c2t"
+    build_index(fa, prefix, bwameth_c2t=True, sa_intv=32, device=-1)
+    rb = sim(fa, n1, False, max_len=60, seed=n1, len_fixed=60, len_min=60, sub_rate=0.02)
+    # the same rounds with room for every row, and the default's list
+    room = (2, 2, 0, 2, 1, 1, 29, 64, 0, 1)
+    work = []
+    for tuning in (room, ()):
+        ctx.set_pipeline(n1, 0, n1, 1)  # the batch in one piece
+        try:
+            compare(prefix, ctx, rb.bases, rb.lens, n1, False, 60, BENCH_PARAMS, tunings=[tuning])
+            ctx.set_tuning(*tuning)
+            ctx.set_profiling(2)
+            map_batch(ctx, gpu_index(ctx, prefix, 12, 12), rb.bases, rb.lens, n1, False, 60, 1, 2, BENCH_PARAMS)
+            t, s2 = ctx.traffic(), ctx.traffic_stage2()
+            work.append((t[5] - s2[5], s2[9]))  # endpoints searched in the rounds, reads in stage 2
+        finally:
+            ctx.set_profiling(0)
+            ctx.set_tuning()
+            ctx.set_pipeline()
+    _INDEX_CACHE.pop((prefix, 12, 12)).close()
+    assert work[0][1] == 0
+    if waits and n1 > 131_072:
+        assert work[1][0] > work[0][0] and work[1][1] == 0, work
+    else:
+        assert work[1][1] > 0, work
