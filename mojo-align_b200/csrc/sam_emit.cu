@@ -372,10 +372,10 @@ __device__ __forceinline__ void put_int(uint8_t* o, int64_t v, uint32_t k) {
     if (v < 0) o[0] = '-';
 }
 
-// Where in a line's formatted fields its contig names belong when they are
-// left out of them.
+// Where in a line's formatted fields its contig names begin, or belong when
+// they are left out of them, and the fields' end.
 struct Cuts {
-    uint32_t rname, rnext;
+    uint32_t rname, rnext, end;
 };
 
 // \t FLAG \t RNAME \t POS \t MAPQ \t CIGAR \t RNEXT \t PNEXT \t TLEN \t at o (one
@@ -418,6 +418,7 @@ __device__ __forceinline__ Cuts put_fields(uint8_t* o, const SamDev& d, const Li
     *o++ = '\t';
     num(h.pnext, '\t');
     num(h.tlen, '\t');
+    cuts.end = static_cast<uint32_t>(o - first);
     return cuts;
 }
 
@@ -441,12 +442,13 @@ __device__ __forceinline__ uint8_t tail_byte(const SamDev& d, uint32_t j) {
 struct __align__(16) LinePlan {
     const uint8_t *name, *seq, *qual;
     uint32_t n_nm, n_sq, n_ql;
-    uint32_t fields;  // bytes of the formatted fields in the line's slot
+    uint32_t fields;  // bytes of the formatted fields in the line's slot, 0: put_head
     uint32_t rc;
-    uint8_t widen;             // the name holds bytes >= 0x80
-    uint8_t apart;             // the contig names are not in the slot
-    uint8_t at_rname, at_rnext;  // and belong here
+    // put_head's: the name holds bytes >= 0x80, bytes in the slot, and where
+    // the contig names that are not in it belong (NONE: they are)
+    uint8_t widen, slot, at_rname, at_rnext;
 };
+constexpr uint32_t NONE = 255;
 static_assert(sizeof(LinePlan) == 48, "line plan layout");
 
 // A lane's share of a line's source bytes: two name bytes, eight bases and
@@ -492,19 +494,26 @@ __device__ __forceinline__ void put_rest(uint8_t* o, const SamDev& d, const Line
         for (uint32_t j = 32 + lane; j < n_tail; j += 32) ot[j] = tail_byte(d, j);
 }
 
-// A name with bytes >= 0x80, each of which becomes U+FFFD; returns its bytes.
-__device__ __noinline__ uint64_t wide_name(uint8_t* o, const uint8_t* nm, uint32_t n_nm, uint32_t lane) {
+// The name and fields of a line whose name has bytes >= 0x80 (each becomes
+// U+FFFD) or whose contig names are not in its slot; returns their bytes.
+__device__ __noinline__ uint64_t put_head(uint8_t* o, const SamDev& d, const LinePlan& q, const LineRec& h,
+                                          const uint8_t* slot, uint32_t lane) {
+    const uint32_t n_nm = q.n_nm;
     uint64_t w = 0;
     for (uint32_t b = 0; b < n_nm; b += 32) {
         const uint32_t i = b + lane;
-        const uint8_t c = i < n_nm ? nm[i] : 0;
+        const uint8_t c = i < n_nm ? q.name[i] : 0;
         const uint32_t wd = i < n_nm ? (c >= 0x80 ? 3u : 1u) : 0u;
-        uint32_t incl = wd;
-        for (int s = 1; s < 32; s <<= 1) {
-            const uint32_t v = __shfl_up_sync(FULL, incl, s);
-            if (lane >= s) incl += v;
+        uint32_t ex = lane, all = min(32u, n_nm - b);
+        if (q.widen) {
+            uint32_t incl = wd;
+            for (int s = 1; s < 32; s <<= 1) {
+                const uint32_t v = __shfl_up_sync(FULL, incl, s);
+                if (lane >= s) incl += v;
+            }
+            ex = incl - wd;
+            all = __shfl_sync(FULL, incl, 31);
         }
-        const uint32_t ex = incl - wd;
         if (wd == 1) {
             o[w + ex] = c;
         } else if (wd == 3) {
@@ -512,22 +521,17 @@ __device__ __noinline__ uint64_t wide_name(uint8_t* o, const uint8_t* nm, uint32
             o[w + ex + 1] = 0xbf;
             o[w + ex + 2] = 0xbd;
         }
-        w += __shfl_sync(FULL, incl, 31);
+        w += all;
     }
-    return w;
-}
-
-// The slot of a line whose contig names are left out of it, with the names in
-// their places; returns the bytes.
-__device__ __forceinline__ uint64_t put_apart(uint8_t* o, const SamDev& d, const LinePlan& q, const LineRec& h,
-                                              const uint8_t* slot, uint32_t lane) {
-    const uint32_t a = q.at_rname, b = q.at_rnext, n = q.fields;
-    const uint32_t n1 = h.contig_kind == K_NAME ? h.contig_len : 0, n2 = h.rnext_kind == K_NAME ? h.rnext_len : 0;
+    o += w;
+    const uint32_t a = q.at_rname, b = q.at_rnext, n = q.slot;
+    const uint32_t n1 = a != NONE && h.contig_kind == K_NAME ? h.contig_len : 0;
+    const uint32_t n2 = b != NONE && h.rnext_kind == K_NAME ? h.rnext_len : 0;
     const uint8_t *name1 = d.names + h.contig_off, *name2 = d.names + h.rnext_off;
     for (uint32_t i = lane; i < n; i += 32) o[i + (i >= a ? n1 : 0) + (i >= b ? n2 : 0)] = slot[i];
     for (uint32_t i = lane; i < n1; i += 32) o[a + i] = __ldg(name1 + i);
     for (uint32_t i = lane; i < n2; i += 32) o[b + n1 + i] = __ldg(name2 + i);
-    return static_cast<uint64_t>(n) + n1 + n2;
+    return w + n + n1 + n2;
 }
 
 // A warp takes `per` consecutive lines.  One lane per line formats its
@@ -535,12 +539,13 @@ __device__ __forceinline__ uint64_t put_apart(uint8_t* o, const SamDev& d, const
 // the lines together one after the other in its stage and stores it in
 // 16-byte blocks when the next line does not fit.  Contig names that do not
 // fit the slot are left out of it and put in their places by the warp: 200 k
-// lines with names of 80 bytes take 0.20 ms, 0.75 with the lane copying them
-// byte by byte (0.17 with names of 20).
-// Bound by instruction issue: 1 M lines of 388 B take 0.47 ms; with each
-// line's fields formatted by its warp, eight lanes busy, and byte-wise copies
-// it was 2.04 ms.
-__global__ void __launch_bounds__(WRITE_WARPS * 32) sam_write_kernel(SamDev d, uint64_t n_lines, const uint64_t* ends,
+// lines with names of 80 bytes take 0.28 ms, 0.75 with the lane copying them
+// byte by byte (0.18 with names of 20).
+// Bound by instruction issue: 1 M lines of 388 B take 0.43 ms with 64 registers
+// (eight blocks an SM), 0.49 with the 80 that the compiler would take; with each
+// line's fields formatted by its warp, eight lanes busy, and byte-wise copies it
+// was 2.04 ms.
+__global__ void __launch_bounds__(WRITE_WARPS * 32, 8) sam_write_kernel(SamDev d, uint64_t n_lines, const uint64_t* ends,
                                                                     const LineRec* recs, uint32_t per) {
     __shared__ __align__(16) uint8_t s_stage[WRITE_WARPS][STAGE + 16];
     __shared__ LinePlan s_plan[WRITE_WARPS][32];
@@ -578,14 +583,13 @@ __global__ void __launch_bounds__(WRITE_WARPS * 32) sam_write_kernel(SamDev d, u
             q.n_ql = d.qual_len[r];
             q.rc = h.mapped && (h.flag & 16);
             const uint64_t f = fields_len(h);
+            const bool names = f <= SLOT;  // the contig names fit the slot too
+            const Cuts cuts = put_fields(slot[lane], d, h, names);
+            q.fields = names && !h.widen ? static_cast<uint32_t>(f) : 0;
             q.widen = h.widen;
-            q.apart = f > SLOT;
-            const uint64_t named = (h.contig_kind == K_NAME ? h.contig_len : 0ull) +
-                                   (h.rnext_kind == K_NAME ? h.rnext_len : 0ull);
-            q.fields = static_cast<uint32_t>(q.apart ? f - named : f);
-            const Cuts cuts = put_fields(slot[lane], d, h, !q.apart);
-            q.at_rname = static_cast<uint8_t>(cuts.rname);
-            q.at_rnext = static_cast<uint8_t>(cuts.rnext);
+            q.slot = static_cast<uint8_t>(cuts.end);
+            q.at_rname = static_cast<uint8_t>(names ? NONE : cuts.rname);
+            q.at_rnext = static_cast<uint8_t>(names ? NONE : cuts.rnext);
             plan[lane] = q;
         }
         __syncwarp();
@@ -598,18 +602,14 @@ __global__ void __launch_bounds__(WRITE_WARPS * 32) sam_write_kernel(SamDev d, u
                                     const LinePlan& q = plan[k];
                                     if (k + 1 < count) load_raw(next, plan[k + 1], lane);
                                     const uint32_t n_nm = q.n_nm, fields = q.fields;
-                                    if (q.widen) {
-                                        o += wide_name(o, q.name, n_nm, lane);
+                                    if (!fields) {
+                                        o += put_head(o, d, q, recs[base + k], slot[k], lane);
                                     } else {
                                         if (lane < n_nm) o[lane] = static_cast<uint8_t>(x.n0);
                                         if (lane + 32 < n_nm) o[lane + 32] = static_cast<uint8_t>(x.n1);
                                         if (n_nm > 64)
                                             for (uint32_t i = 64 + lane; i < n_nm; i += 32) o[i] = __ldg(q.name + i);
                                         o += n_nm;
-                                    }
-                                    if (q.apart) {
-                                        o += put_apart(o, d, q, recs[base + k], slot[k], lane);
-                                    } else {
                                         for (uint32_t i = lane; i < fields; i += 32) o[i] = slot[k][i];
                                         o += fields;
                                     }

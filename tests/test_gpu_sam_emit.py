@@ -239,7 +239,7 @@ def test_lines_at_the_edges_of_the_lanes_the_slots_and_the_stage(ctx, rg, paired
 
 def test_long_contig_names_cost_little(ctx):
     """Names of 150 bytes, most pairs on two contigs: the warp copies the names,
-    so a call takes little more than with short ones (1.3 times; 6 times when
+    so a call takes little more than with short ones (1.6 times; 6 times when
     the lane that formats a line's fields copied them)."""
     import torch
 
