@@ -52,10 +52,9 @@ METRIC = "reads/s seed+extend"
 # step of the default genome workload (3100 Mbp, 50 M uneven single-end
 # reads), from a one-pass ncu capture of that step with the tuning below;
 # roofline.traffic reports it for runs of that workload and tuning, and null
-# otherwise.  None: the capture (24660) is of the search and eval kernels
-# before they ran from lists per warp.
-GENOME_SEED_DRAM_BYTES_PER_READ = None
-GENOME_SEED_DRAM_TUNING = (4, 2, 0, 1, 1, 1, 8, 32, 0, 1)
+# otherwise.
+GENOME_SEED_DRAM_BYTES_PER_READ = 28431
+GENOME_SEED_DRAM_TUNING = (2, 2, 0, 1, 1, 1, 8, 32, 0, 1)
 GENOME_SEED_DRAM_AT_K = 28  # the capture's A/T window table (0: none)
 # The workload parameters: the reference defaults with seed_len 19 and
 # max_occ 500 (mojoalign_b200.params.BENCH_PARAMS holds the same values; the
