@@ -753,7 +753,7 @@ def run_fq2bam_stage(args, ctx, gi, rb, local, params):
                            "phases_s": gz_phases, "input_bytes": gz_bytes,
                            "e2e": {"h2d_bytes_per_step": int(gz_phases.get("fastq_h2d_bytes", gz_bytes)),
                                    "d2h_bytes_per_step": out_gz.stat().st_size},
-                           "inflate": "BGZF members copied to the device and inflated there (one CTA per member)",
+                           "inflate": "BGZF members copied to the device and inflated there (a CTA or a warp per member)",
                            "parity": {"bam_content_equals_plain_input": bool(gz_same)}},
         }
     finally:
