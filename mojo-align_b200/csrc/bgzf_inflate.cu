@@ -29,7 +29,7 @@
 // leaves: members that this form does not hold (more than 0xff00 bytes, as some
 // writers fill them, or many blocks), members with anything invalid in them (it
 // gives their status), and those that many warps finish sooner than the CTAs
-// (cta_takes, Rounds).
+// (Cost, Rounds).
 // Every code's reads stay in the staged input and every cell in the member:
 // sizes are checked before they are used.
 // Bound by latency: per member of 65280 bytes of FASTQ the sync rounds take
@@ -218,6 +218,7 @@ struct __align__(16) Smem {
     uint32_t first_flag;
     uint32_t mine[CTA_THREADS / 32];  // which of the CTA's next members it takes
     uint32_t stopped;                 // it takes no more of them
+    unsigned long long cta_ns, warp_ns;  // of those that warps are faster at: in the CTA all, in a warp the slowest
 };
 
 // Barriers of the THREADS that work on a member (the header warp takes none).
@@ -560,26 +561,37 @@ __device__ __forceinline__ bool member_spans(const bgzf_inflate::Job& j, uint32_
     return !(so > j.in_bytes || sl > j.in_bytes - so || dof > j.out_bytes || isz > j.out_bytes - dof);
 }
 
-// Whether a CTA takes member m of a call of j.n; its spans are checked.  A CTA
-// decodes a large member up to 40 times as fast as a warp, but 148 members are in
-// CTAs at a time and 9472 in warps, and a small member's time is the CTA's own.
-// So: the CTAs' turns at members like this one against one member's time in a
-// warp, and an SM's time for a member either way, in nanoseconds by the kind of
-// its first block (fitted to members of 512 .. 65280 bytes: FASTQ at level 6,
-// zeros, base-64 text, fixed codes, whose segments fall into step late, and stored
-// noise).  16000 members of 512 bytes of FASTQ: 1.5 ms in warps, 5.3 in CTAs;
-// 2368 of 4096 bytes 0.82 and 0.95, of 16384 bytes 2.5 and 1.15.  8000 members of
-// 65280 bytes of zeros 2.1 and 6.8 ms, of stored noise 2.2 and 3.5, 2000 of
-// FASTQ in fixed codes 9.8 and 18.3.
-__device__ __forceinline__ bool cta_takes(const bgzf_inflate::Job& j, uint32_t m) {
+// What a member takes, in nanoseconds by the kind of its first block (fitted to
+// members of 512 .. 65280 bytes: FASTQ at level 6, zeros, base-64 text, fixed
+// codes, whose segments fall into step late, and stored noise).
+struct Cost {
+    uint64_t cta;   // a CTA, which has the SM to itself
+    uint64_t warp;  // a warp, alone
+    uint64_t sm;    // one more on an SM whose 64 warps are at work
+};
+
+__device__ __forceinline__ Cost member_cost(const bgzf_inflate::Job& j, uint32_t m) {
     const uint64_t isz = j.isize[m], src = j.src_len[m];
-    if (isz < 4 || isz > MAX_BYTES || src < 1 || src > (1u << 26)) return false;
     const uint32_t type = j.in[j.src_off[m]] >> 1 & 3;
-    const uint64_t cta = type == 0 ? 17000 + isz * 3 / 4 : type == 1 ? 45000 + src * 45 : 50000 + isz * 9 / 10;  // a turn
-    const uint64_t warp = type == 0 ? 10000 + isz * 8 : 130000 + src * 260 + isz * 6;  // the first members in warps
-    const uint64_t sm = type == 0 ? 4000 + isz * 9 / 16 : 9000 + src * 17 + isz / 2;   // one more, all warps at work
-    return j.n * cta <= gridDim.x * warp || cta <= sm;
+    if (type == 0) return Cost{17000 + isz * 3 / 4, 10000 + isz * 8, 4000 + isz * 9 / 16};
+    return Cost{type == 1 ? 45000 + src * 45 : 50000 + isz * 9 / 10, 130000 + src * 260 + isz * 6, 9000 + src * 17 + isz / 2};
 }
+
+// Whether a CTA can take member m; its spans are checked.
+__device__ __forceinline__ bool cta_holds(const bgzf_inflate::Job& j, uint32_t m) {
+    return j.isize[m] >= 4 && j.isize[m] <= MAX_BYTES && j.src_len[m] >= 1 && j.src_len[m] <= (1u << 26);
+}
+
+// A CTA decodes a large member up to 40 times as fast as a warp, but 148 members
+// are in CTAs at a time and 9472 in warps, and a small member's time is the CTA's
+// own.  So a CTA leaves those of its members that an SM's warps are faster at
+// (Cost), when they would take the CTAs longer than the slowest of them takes a
+// warp, and the second kernel's start.  16000 members of 512 bytes of FASTQ: 1.5 ms in
+// warps, 5.3 in CTAs; 2368 of 4096 bytes 0.82 and 0.95, of 16384 bytes 2.5 and
+// 1.15.  8000 members of 65280 bytes of zeros 2.1 and 6.8 ms, of stored noise 2.2
+// and 3.5, 2000 of FASTQ in fixed codes 9.8 and 18.3.  One member of 600 bytes
+// among 1960 of 65280 stays with its CTA: in a warp it would add 0.2 ms to 1.4.
+constexpr uint64_t LEFT_START = 15000;
 
 // Codes that fall into step late, beyond four turns of the CTAs: there a member
 // whose literal codes are all but an eighth of one length (base-64, hexadecimal
@@ -792,13 +804,26 @@ __global__ void __launch_bounds__(CTA_THREADS, 1) bgzf_inflate_kernel(bgzf_infla
     // CTA_THREADS it takes is looked up for all of them at once
     for (uint64_t base = 0; blockIdx.x + base * gridDim.x < j.n; base += CTA_THREADS) {
         auto member = [&](int i) { return static_cast<uint32_t>(blockIdx.x + (base + i) * gridDim.x); };
-        bool take = false;
-        if (blockIdx.x + (base + t) * gridDim.x < j.n) {
-            const uint32_t m = member(static_cast<int>(t));
-            const bool spans = member_spans(j, m);
-            take = spans && cta_takes(j, m);
-            if (!take) j.status[m] = spans ? S_LEFT : bgzf_inflate::S_SPAN;
+        const bool any = blockIdx.x + (base + t) * gridDim.x < j.n;
+        const uint64_t turns = (j.n + gridDim.x - 1) / gridDim.x, here = (j.n - blockIdx.x + gridDim.x - 1) / gridDim.x;
+        const uint32_t m0 = member(static_cast<int>(t));
+        const bool spans = any && member_spans(j, m0), holds = spans && cta_holds(j, m0);
+        bool slower = false;
+        if (t == 0) S.cta_ns = S.warp_ns = 0;
+        __syncthreads();
+        if (holds) {
+            const Cost c = member_cost(j, m0);
+            slower = c.cta > c.sm;
+            if (slower) {
+                atomicAdd(&S.cta_ns, static_cast<unsigned long long>(c.cta));
+                atomicMax(&S.warp_ns, static_cast<unsigned long long>(c.warp));
+            }
         }
+        __syncthreads();
+        // CTAs of one member more or less than others are to decide alike
+        const bool leave = S.cta_ns * turns > (S.warp_ns + LEFT_START) * here;
+        const bool take = holds && !(slower && leave);
+        if (any && !take) j.status[m0] = spans ? S_LEFT : bgzf_inflate::S_SPAN;
         const uint32_t word = __ballot_sync(0xffffffffu, take);
         if ((t & 31) == 0) S.mine[t >> 5] = word;
         __syncthreads();

@@ -313,3 +313,50 @@ def test_edges_of_segments_strips_and_rounds(ctx):
         status, got, _, _ = _inflate_raw(ctx, [(p, len(d), zlib.crc32(d)) for p, d in cases], lead)
         for i, ((_, d), s, g) in enumerate(zip(cases, status, got)):
             assert s == 0 and g == d, i
+
+
+@pytest.mark.parametrize("last", [300, 600, 1500])
+def test_a_small_last_member_costs_nothing(ctx, last):
+    """The member that ends a file is decoded beside the others of its CTA, not
+    by a warp after all of them (0.2 to 0.4 ms on top of 2.3)."""
+    import torch
+    import zlib
+
+    text = random_fastq(13, 6000)
+    pieces = [text[a * 65280:(a + 1) * 65280] for a in range(8)] + [text[:last]]
+    src, so, sl = bytearray(), [], []
+    for p in pieces:
+        c = zlib.compressobj(6, zlib.DEFLATED, -15)
+        d = c.compress(p) + c.flush()
+        so.append(len(src))
+        sl.append(len(d))
+        src += d
+    crc = np.array([zlib.crc32(p) for p in pieces], np.uint32).view(np.int32)
+    d_in = torch.frombuffer(src, dtype=torch.uint8).cuda()
+    took = []
+    for n in (1036, 1037):
+        i = np.arange(n) % 8
+        i[1036:] = 8
+        size = np.array([len(p) for p in pieces])[i]
+        put = lambda v, t: torch.from_numpy(np.asarray(v).astype(t)).cuda()  # noqa: E731
+        cols = [put(np.array(so)[i], np.int64), put(np.array(sl)[i], np.int32), put(np.cumsum(size) - size, np.int64),
+                put(size, np.int32), put(crc[i], np.int32)]
+        d_out = torch.zeros(int(size.sum()), dtype=torch.uint8, device="cuda")
+        status = torch.full((n,), 77, dtype=torch.int32, device="cuda")
+        stream = torch.cuda.Stream()
+        torch.cuda.synchronize()
+        times = []
+        for _ in range(13):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record(stream)
+            _lib.check(_lib.lib.ma_bgzf_inflate_device(ctx.handle, d_in.data_ptr(), len(src),
+                                                       *[c.data_ptr() for c in cols], n, d_out.data_ptr(),
+                                                       d_out.numel(), status.data_ptr(), stream.cuda_stream),
+                       ctx.handle)
+            b.record(stream)
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+        took.append(float(np.median(times[3:])))
+        assert not status.any()
+        assert d_out[-last if n > 1036 else -65280:].cpu().numpy().tobytes() == pieces[i[-1]]
+    assert took[1] < 1.05 * took[0], took
