@@ -805,7 +805,7 @@ __global__ void __launch_bounds__(CTA_THREADS, 1) bgzf_inflate_kernel(bgzf_infla
     for (uint64_t base = 0; blockIdx.x + base * gridDim.x < j.n; base += CTA_THREADS) {
         auto member = [&](int i) { return static_cast<uint32_t>(blockIdx.x + (base + i) * gridDim.x); };
         const bool any = blockIdx.x + (base + t) * gridDim.x < j.n;
-        const uint64_t turns = (j.n + gridDim.x - 1) / gridDim.x, here = (j.n - blockIdx.x + gridDim.x - 1) / gridDim.x;
+        const uint64_t n = j.n, turns = (n + gridDim.x - 1) / gridDim.x, here = (n - blockIdx.x + gridDim.x - 1) / gridDim.x;
         const uint32_t m0 = member(static_cast<int>(t));
         const bool spans = any && member_spans(j, m0), holds = spans && cta_holds(j, m0);
         bool slower = false;
